@@ -170,10 +170,11 @@ struct Ranges {
 };
 
 // launch shapes: traversal blocks per SM, narrow-phase blocks per SM (one is resident at
-// a time; more blocks split the work finer), the traversal's schedule (0: one query per
-// thread, k_traverse_q; 1: 32 queries per warp walking together, k_traverse_w) and, for
-// k_traverse_q, the tree levels below the root each block copies into shared memory (0-2),
-// and the narrow phase's batch (1: 256 sub-tests, 2: 512)
+// a time; more blocks split the work finer), the traversal's schedule (0: each warp shares out
+// the node visits of its queries, k_traverse_walk; 1: 32 queries per warp walking together,
+// k_traverse_w) and, under schedule 0, the tree levels below the root that each block copies
+// into shared memory (1-2: one query per thread, k_traverse_q; 0: k_traverse_walk), and the
+// narrow phase's batch (1: 256 sub-tests, 2: 512)
 struct Shape {
     int trav, narrow, warp, stage, batch;
 };
@@ -290,8 +291,12 @@ template <class T> int traverse(ccc_engine* e, const Tables& t, const int* flags
         CCC_LAUNCH("k_traverse", s, k_traverse_w<<<g, TRAV_THREADS, 0, s>>>(
             e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
+    else if (SHAPES[e->shape].stage == 0 && vid)
+        CCC_LAUNCH("k_traverse", s, k_traverse_walk<true><<<g, WALK_THREADS, 0, s>>>(
+            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+            (int)e->L.cand_cap, e->hdr(), flags, vid));
     else if (SHAPES[e->shape].stage == 0)
-        CCC_LAUNCH("k_traverse", s, k_traverse_q<0><<<g, TRAV_THREADS, 0, s>>>(
+        CCC_LAUNCH("k_traverse", s, k_traverse_walk<false><<<g, WALK_THREADS, 0, s>>>(
             e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     else if (SHAPES[e->shape].stage == 1)

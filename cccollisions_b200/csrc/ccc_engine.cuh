@@ -21,6 +21,7 @@
 #pragma once
 
 #include "ccc_kernels.cuh"
+#include "ccc_walk.cuh"
 
 namespace ccc {
 
@@ -351,19 +352,9 @@ static __global__ void k_karras_build(Forest F, const unsigned long long* __rest
 }
 
 // ---------------------------------------------------------------------------------------
-// Four-wide nodes.  Every even-depth internal node b of the binary tree (the root has depth
-// 0) heads a QNode whose 2 to 4 slots are b's children, where a child that is itself an
-// internal node (odd depth) is replaced by its two children.  A slot holds a child box
-// (fp32, rounded outward), a reference (>= 0: the QNode of an even-depth internal node;
-// ~pos: the leaf at sorted position pos) and an aux word (the rightmost leaf position below
-// an internal slot, the triangle id of a leaf slot).  Unused slots hold an empty box.
-// QNodes are indexed by their binary node.  One QNode visit covers two binary levels, so a
-// tree walk needs half as many dependent node fetches.
-struct __align__(16) QNode {
-    float4 lox, loy, loz, hix, hiy, hiz;
-    int4 ref, aux;
-};
-static constexpr int Q_EMPTY = 0x7fffffff;
+// Four-wide nodes (QNode).  Every even-depth internal node b of the binary tree (the root has
+// depth 0) heads a QNode whose 2 to 4 slots are b's children, where a child that is itself an
+// internal node (odd depth) is replaced by its two children.  Unused slots hold an empty box.
 // qcode of an internal node: (QNode << 2) | slot for an even-depth node below the root;
 // QCODE_ROOT for the root; for an odd-depth node, which has no slot of its own,
 // QCODE_ODD - ((QNode << 2) | first slot) locates the two adjacent slots of its children
@@ -934,24 +925,65 @@ static __global__ void k_engine_refit_front(Forest F, const int* __restrict__ np
     }
 }
 
-// Continuous-collision candidates of resident trees: one query leaf per thread walks the
-// QNodes with an explicit per-thread stack (local memory), tests the 4 slot boxes of a node at once
-// (fp32; the query box is the leaf's own outward-rounded slot box), keeps the reference's
-// order rule (a slot is skipped when its rightmost leaf position is not after the query's,
-// so each unordered pair is found once) and emits (min id, max id) in data slots.  Candidates
-// are the pairs whose fp32 boxes overlap, a superset of the exact ones; the continuous
-// narrow phase re-tests every pair's swept sub-boxes exactly.  With the corner classes
-// (vid, the collision step), pairs whose triangles share a vertex, which the narrow phase
-// drops, are not emitted.
-//
-// SD > 0: the top SD + 1 levels of the mesh of a block's first query (at most 1 + 4 + 16
-// QNodes) are copied into shared memory at every step of the block's loop, breadth first,
-// and every reference from one copied node to another is rewritten to TRAV_STAGED | its
-// index among the copies; the block's queries of that mesh start at the copied root and read
-// those nodes from shared memory.  The other queries (a block spanning two meshes) walk
-// the global nodes.
+// Continuous-collision candidates of resident trees (walk_forest).  The query box is the
+// leaf's own outward-rounded slot box, so the candidates are the pairs whose fp32 boxes
+// overlap, a superset of the exact ones; the continuous narrow phase re-tests every pair's
+// swept sub-boxes exactly.  With the corner classes (vid, the collision step), pairs whose
+// triangles share a vertex, which the narrow phase drops, are not emitted.
+template <bool CLASSES> struct EngineWalk {
+    const QNode* qnodes;
+    const int* qleaf;
+    const int* leaf_tri;
+    const int* mflags;      // null, or the meshes with MF_DONE are skipped
+    const int4* vid;
+    static constexpr bool ORDERED = true;
+    __device__ __forceinline__ bool query(const Forest& F, int M, int v, WsHeader* hdr, WalkQuery& q) const {
+        const int m = find_mesh(F.voff, M, v, 0);
+        const int vo = __ldg(F.voff + m);
+        q.base = __ldg(F.poff + m);
+        q.n = __ldg(F.voff + m + 1) - vo;
+        q.pos = v - vo;
+        if (q.n < 2 || (mflags && (__ldg(mflags + __ldg(F.sid + m)) & MF_DONE))) return false;
+        q.id = __ldg(leaf_tri + q.base + q.pos);
+        const int lq = __ldg(qleaf + q.base + q.pos);
+        if (q.id < 0 || q.id >= q.n || lq < 0 || (lq >> 2) >= q.n - 1) {
+            atomicOr(&hdr->status, ST_MALFORMED_TREE);
+            return false;
+        }
+        const float* f = reinterpret_cast<const float*>(qnodes + (q.base + (lq >> 2))) + (lq & 3);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            q.lo[c] = __ldg(f + 4 * c);
+            q.hi[c] = __ldg(f + 12 + 4 * c);
+        }
+        return true;
+    }
+    __device__ __forceinline__ int rightmost(int, int, int aux) const { return aux; }
+    __device__ __forceinline__ bool keep(int base, int n, int, int id, int, int cid) const {
+        if (!CLASSES) return true;
+        return !classes_meet(__ldg(vid + base + id), __ldg(vid + base + cid));
+    }
+};
+
+template <bool CLASSES>
+static __global__ void __launch_bounds__(WALK_THREADS, 8)
+k_traverse_walk(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, const int* __restrict__ leaf_tri,
+                Forest F, int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const int* __restrict__ mflags,
+                const int4* __restrict__ vid) {
+    __shared__ WalkWarp S[WALK_WARPS];
+    const EngineWalk<CLASSES> pol{qnodes, qleaf, leaf_tri, mflags, vid};
+    walk_forest(pol, qnodes, F, cand, cand_cap, hdr, S[threadIdx.x >> 5]);
+}
+
+// The walk with one query leaf per thread (autotuner candidates): an explicit per-thread stack
+// in local memory, the same candidates as k_traverse_walk.  The top SD + 1 levels (SD 1 or 2)
+// of the mesh of a block's first query (at most 1 + 4 + 16 QNodes) are copied into shared
+// memory at every step of the block's loop, breadth first, and every reference from one
+// copied node to another is rewritten to TRAV_STAGED | its index among the copies; the
+// block's queries of that mesh start at the copied root and read those nodes from shared
+// memory.  The other queries (a block spanning two meshes) walk the global nodes.
 static constexpr int TRAV_STAGED = 1 << 30;
-__device__ __forceinline__ int trav_stage_count(int sd) { return sd == 0 ? 0 : (sd == 1 ? 5 : 21); }
+__host__ __device__ constexpr int trav_stage_count(int sd) { return sd == 1 ? 5 : 21; }
 
 template <int SD>
 static __global__ void __launch_bounds__(TRAV_THREADS)
@@ -960,58 +992,56 @@ k_traverse_q(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, co
              const int4* __restrict__ vid) {
     int stack[STACK_DEPTH];          // per-thread, in local memory (L1): shared memory holds the buffer
     __shared__ int2 cbuf[TRAV_BUF][TRAV_THREADS];     // candidate buffer (see flush_candidates)
-    __shared__ QNode top[SD > 0 ? (SD == 1 ? 5 : 21) : 1];
-    __shared__ int top_src[SD > 0 ? (SD == 1 ? 5 : 21) : 1];    // global index of each copy
+    __shared__ QNode top[trav_stage_count(SD)];
+    __shared__ int top_src[trav_stage_count(SD)];    // global index of each copy
     __shared__ int top_n, top_mesh;
     int nbuf = 0;
     const int tid = threadIdx.x;
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
-        if (SD > 0) {
-            // copy the top levels of the first query's mesh (block-uniform steps)
-            __syncthreads();       // the previous step's walks are done with the copies
-            if (tid == 0) {
-                const int m0 = find_mesh(F.voff, M, base, 0);
-                const int n0 = __ldg(F.voff + m0 + 1) - __ldg(F.voff + m0);
-                const bool ok = n0 >= 2 && !(mflags && (__ldg(mflags + __ldg(F.sid + m0)) & MF_DONE));
-                top_mesh = ok ? m0 : -1;
-                top_n = ok ? 1 : 0;
-                top_src[0] = 0;
+        // copy the top levels of the first query's mesh (block-uniform steps)
+        __syncthreads();       // the previous step's walks are done with the copies
+        if (tid == 0) {
+            const int m0 = find_mesh(F.voff, M, base, 0);
+            const int n0 = __ldg(F.voff + m0 + 1) - __ldg(F.voff + m0);
+            const bool ok = n0 >= 2 && !(mflags && (__ldg(mflags + __ldg(F.sid + m0)) & MF_DONE));
+            top_mesh = ok ? m0 : -1;
+            top_n = ok ? 1 : 0;
+            top_src[0] = 0;
+        }
+        __syncthreads();
+        const int m0 = top_mesh;
+        const QNode* qn0 = qnodes + (m0 >= 0 ? __ldg(F.poff + m0) : 0);
+        const int n0 = m0 >= 0 ? __ldg(F.voff + m0 + 1) - __ldg(F.voff + m0) : 0;
+        int lo = 0;                                 // first copy of the current level
+#pragma unroll 1
+        for (int lev = 0; lev <= SD && m0 >= 0; ++lev) {
+            const int hi = top_n;                   // copies [lo, hi) are this level's
+            // copy the level's nodes, 8 threads a node (16 bytes each)
+            for (int w = tid; w < (hi - lo) * 8; w += blockDim.x) {
+                const int i = lo + w / 8, part = w % 8;
+                reinterpret_cast<int4*>(top + i)[part] =
+                    __ldg(reinterpret_cast<const int4*>(qn0 + top_src[i]) + part);
             }
             __syncthreads();
-            const int m0 = top_mesh;
-            const QNode* qn0 = qnodes + (m0 >= 0 ? __ldg(F.poff + m0) : 0);
-            const int n0 = m0 >= 0 ? __ldg(F.voff + m0 + 1) - __ldg(F.voff + m0) : 0;
-            int lo = 0;                                 // first copy of the current level
-#pragma unroll 1
-            for (int lev = 0; lev <= SD && m0 >= 0; ++lev) {
-                const int hi = top_n;                   // copies [lo, hi) are this level's
-                // copy the level's nodes, 8 threads a node (16 bytes each)
-                for (int w = tid; w < (hi - lo) * 8; w += blockDim.x) {
-                    const int i = lo + w / 8, part = w % 8;
-                    reinterpret_cast<int4*>(top + i)[part] =
-                        __ldg(reinterpret_cast<const int4*>(qn0 + top_src[i]) + part);
-                }
-                __syncthreads();
-                if (lev < SD && tid == 0) {
-                    // the next level: the copies' internal children, rewritten to their copies
-                    int cnt = hi;
-                    for (int i = lo; i < hi; ++i) {
-                        int* rr = reinterpret_cast<int*>(&top[i].ref);
-                        for (int sl = 0; sl < 4; ++sl) {
-                            const int r = rr[sl];
-                            if (r == Q_EMPTY || r < 0 || r >= n0 - 1) continue;    // leaf, empty or bad
-                            top_src[cnt] = r;
-                            rr[sl] = TRAV_STAGED | cnt;
-                            ++cnt;
-                        }
+            if (lev < SD && tid == 0) {
+                // the next level: the copies' internal children, rewritten to their copies
+                int cnt = hi;
+                for (int i = lo; i < hi; ++i) {
+                    int* rr = reinterpret_cast<int*>(&top[i].ref);
+                    for (int sl = 0; sl < 4; ++sl) {
+                        const int r = rr[sl];
+                        if (r == Q_EMPTY || r < 0 || r >= n0 - 1) continue;    // leaf, empty or bad
+                        top_src[cnt] = r;
+                        rr[sl] = TRAV_STAGED | cnt;
+                        ++cnt;
                     }
-                    top_n = cnt;
                 }
-                __syncthreads();
-                lo = hi;
+                top_n = cnt;
             }
+            __syncthreads();
+            lo = hi;
         }
         const int v = base + tid;
         if (v < total) {
@@ -1042,7 +1072,7 @@ k_traverse_q(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, co
                     qhi[2] = __ldg(f + 20 + sl);
                 }
                 int sp = 0;
-                int node = (SD > 0 && m == top_mesh) ? TRAV_STAGED : 0;
+                int node = m == top_mesh ? TRAV_STAGED : 0;
                 const int limit = 2 * n + 64;
                 for (int it = 0;; ++it) {
                     if (it > limit) {
@@ -1051,7 +1081,7 @@ k_traverse_q(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, co
                     }
                     float4 LX, LY, LZ, HX, HY, HZ;
                     int4 R, A;
-                    if (SD > 0 && (node & TRAV_STAGED)) {
+                    if (node & TRAV_STAGED) {
                         const QNode& t = top[node & 0xff];
                         LX = t.lox; LY = t.loy; LZ = t.loz; HX = t.hix; HY = t.hiy; HZ = t.hiz; R = t.ref; A = t.aux;
                     } else {
@@ -1071,7 +1101,7 @@ k_traverse_q(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, co
                     for (int s = 0; s < 4; ++s) {
                         const int ref = rr[s];
                         if (ref == Q_EMPTY) continue;
-                        const bool staged = SD > 0 && ref >= 0 && (ref & TRAV_STAGED);
+                        const bool staged = ref >= 0 && (ref & TRAV_STAGED);
                         if (!staged && (ref >= n - 1 || (ref < 0 && ~ref >= n))) { bad = true; continue; }
                         bool hit = (qlo[0] <= hx[s]) && (qhi[0] >= lx[s]) && (qlo[1] <= hy[s]) && (qhi[1] >= ly[s]) &&
                                    (qlo[2] <= hz[s]) && (qhi[2] >= lz[s]);

@@ -187,10 +187,10 @@ class Engine:
     @staticmethod
     def schedules() -> list[dict]:
         """The autotuner's candidate schedules: traversal blocks per SM, narrow-phase blocks
-        per SM (in units of the resident count), the traversal form (0 one query per
-        thread, 1 32 queries per warp), the tree levels below the root that each traversal
-        block keeps in shared memory (0-2, one query per thread) and the narrow phase's
-        batch in units of 256 sub-tests (1 or 2)."""
+        per SM (in units of the resident count), the traversal form (0 a warp shares out its
+        queries' node visits, 1 32 queries per warp walk together), the tree levels below the
+        root that each traversal block keeps in shared memory (0-2; with 1 or 2, form 0 walks
+        one query per thread) and the narrow phase's batch in units of 256 sub-tests (1 or 2)."""
         out = []
         for i in range(N.lib().ccc_engine_schedule_count()):
             a = (ctypes.c_int32 * 5)()

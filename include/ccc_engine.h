@@ -113,9 +113,10 @@ int ccc_engine_autotune(ccc_engine* e, void* stream, int32_t* choice);
 
 /* The autotuner's candidate schedules (no counterpart in the reference): their number;
  * the parameters of one in out[5] (out[0] traversal blocks per SM, out[1] narrow-phase
- * blocks per SM in units of the resident count, out[2] traversal form: 0 one query per
- * thread, 1 32 queries per warp walking the tree together, out[3] tree levels below the
- * root that each block of the one-query-per-thread form copies into shared memory, 0-2,
+ * blocks per SM in units of the resident count, out[2] traversal form: 0 a warp shares
+ * out the node visits of its queries, 1 32 queries per warp walk the tree together, out[3]
+ * tree levels below the root that each block copies into shared memory, 0-2 (with 1 or 2,
+ * form 0 walks one query per thread),
  * out[4] the narrow phase's batch in units of 256 sub-tests, 1 or 2); and fixing the
  * engine to one of them. */
 int ccc_engine_schedule_count(void);
