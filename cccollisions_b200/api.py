@@ -112,14 +112,14 @@ def bvh_motion(triangles, triangles_next):
 def _bvh(triangles, triangles_next):
     B, F = triangles.size(0), triangles.size(1)
     dev = triangles.device
-    bboxes = -1 * torch.ones((B, 2 * F - 1, 6), dtype=triangles.dtype, device=dev)
-    tree = -1 * torch.ones((B, 2 * F - 1, 4), dtype=torch.int64, device=dev)
+    # (the build writes every element, and nothing in it can fail on the device: no status)
+    bboxes = torch.empty((B, 2 * F - 1, 6), dtype=triangles.dtype, device=dev)
+    tree = torch.empty((B, 2 * F - 1, 4), dtype=torch.int64, device=dev)
     with _with_device(triangles):
         ws = _workspace(N.OP_BVH, B, F, 0, dev)
         rc = N.lib().ccc_bvh(_dtype_code(triangles), _ptr(triangles), _ptr(triangles_next), B, F, _ptr(bboxes),
                              _ptr(tree), _ptr(ws), ws.numel(), _stream(dev))
         N.check(rc, "bvh")
-        _report(ws, dev, B, "bvh")
     return [bboxes, tree]
 
 

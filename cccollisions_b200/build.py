@@ -25,7 +25,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libccc_b200.so")
 SOURCES = ["ccc_capi.cu", "ccc_engine.cu"]
 NARROW_SOURCE = "ccc_narrow.cu"
-HEADERS = ["ccc_kernels.cuh", "ccc_walk.cuh", "ccc_engine.cuh", "ccc_runtime.cuh", "ccc_geom.cuh", "ccc_libm.h", "ccc_ddmul.h"]
+HEADERS = ["ccc_kernels.cuh", "ccc_walk.cuh", "ccc_tree.cuh", "ccc_engine.cuh", "ccc_runtime.cuh", "ccc_geom.cuh", "ccc_libm.h", "ccc_ddmul.h"]
 ROOT = os.path.dirname(HERE)
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -111,108 +111,6 @@ static __global__ void k_uniform_offsets(int* nm, int* voff, int* poff, int* sid
 }
 
 // ---------------------------------------------------------------------------------------
-// Build (reference order): leaf boxes, Karras topology, bottom-up box refit.
-// The reference's scene box is reduced from AABB() = (-MAX, +MAX) (aabb.cu:25-34,
-// build_bvh.cu:243-244), which makes every Morton code 0; with all keys equal the stable
-// sort keeps the input order, so leaf position p holds triangle p and the Karras prefix
-// delta(i, j) reduces to 32 + clz(i ^ j).
-
-// leaf rows: box of triangle p (swept over t0/t1 for motion), tree row (parent set later,
-// -1, -1, p)
-template <class T>
-__global__ void k_leaf_rows(const T* __restrict__ x0, const T* __restrict__ x1, const int* __restrict__ moff, int M,
-                            int total, T* __restrict__ bboxes, long long* __restrict__ tree) {
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int m = find_mesh(moff, M, g, 0);
-    int F = moff[m + 1] - moff[m];
-    int p = g - moff[m];
-    long long row = 2LL * moff[m] - m + (F - 1) + p;
-    Box<T> b = tri_box(load_tri(x0, g));
-    if (x1) b = merge(b, tri_box(load_tri(x1, g)));      // MergeTriBoundingBoxes (452-460)
-    store_box(bboxes + row * 6, b);
-    tree[row * 4 + 1] = -1;
-    tree[row * 4 + 2] = -1;
-    tree[row * 4 + 3] = p;
-}
-
-// delta for all-equal keys and identity ids (LongestCommonPrefix, bvh.cu:65-89)
-__device__ __forceinline__ int delta_id(int i, int j, int n) {
-    if (j < 0 || j > n - 1) return -1;
-    return 32 + __clz(i ^ j);
-}
-
-// BuildRadixTree (build_bvh.cu:74-143) for identity order.  The split search is the
-// standard Karras one (steps ceil(l/2), ceil(l/4), ..., 1), which reaches the same split
-// as the reference's loop.
-static __global__ void k_karras_identity(const int* __restrict__ moff, int M, int total_internal, long long* __restrict__ tree) {
-    int gi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gi >= total_internal) return;
-    int m = find_mesh(moff, M, gi, 1);
-    int n = moff[m + 1] - moff[m];
-    int i = gi - (moff[m] - m);
-    long long base = 2LL * moff[m] - m;
-    int dnext = delta_id(i, i + 1, n), dlast = delta_id(i, i - 1, n);
-    int d = (dnext - dlast >= 0) ? 1 : -1;
-    int dmin = delta_id(i, i - d, n);
-    int lmax = 2;
-    while (delta_id(i, i + lmax * d, n) > dmin) lmax *= 2;
-    int l = 0;
-    for (int t = lmax / 2; t >= 1; t /= 2)
-        if (delta_id(i, i + (l + t) * d, n) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = delta_id(i, j, n);
-    int s = 0;
-    for (int div = 2;; div *= 2) {
-        int t = (l + div - 1) / div;
-        if (delta_id(i, i + (s + t) * d, n) > dnode) s += t;
-        if (t <= 1) break;
-    }
-    int split = i + s * d + min(d, 0);
-    long long lc = (min(i, j) == split) ? (long long)(n - 1 + split) : (long long)split;
-    long long rc = (max(i, j) == split + 1) ? (long long)(n - 1 + split + 1) : (long long)(split + 1);
-    tree[(base + i) * 4 + 1] = lc;
-    tree[(base + i) * 4 + 2] = rc;
-    tree[(base + i) * 4 + 3] = -1;
-    tree[(base + lc) * 4 + 0] = i;
-    tree[(base + rc) * 4 + 0] = i;
-    if (i == 0) tree[base * 4 + 0] = -1;
-}
-
-// CreateHierarchy (build_bvh.cu:145-209): each leaf climbs; the second thread to reach a
-// node writes the union of its children's boxes and continues.
-template <class T>
-__global__ void k_refit(const int* __restrict__ moff, int M, int total, T* bboxes, const long long* __restrict__ tree,
-                        int* __restrict__ visits, int* status) {
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    int m = find_mesh(moff, M, g, 0);
-    int n = moff[m + 1] - moff[m];
-    if (n < 2) return;
-    int p = g - moff[m];
-    long long base = 2LL * moff[m] - m;
-    int* vis = visits + (moff[m] - m);
-    long long node = tree[(base + n - 1 + p) * 4 + 0];
-    for (int guard = 0; guard < n; ++guard) {
-        if (node < 0 || node >= n - 1) { atomicOr(status, ST_MALFORMED_TREE); return; }
-        __threadfence();
-        if (atomicAdd(vis + node, 1) == 0) return;
-        long long lc = tree[(base + node) * 4 + 1], rc = tree[(base + node) * 4 + 2];
-        const T* lb = bboxes + (base + lc) * 6;
-        const T* rb = bboxes + (base + rc) * 6;
-        Box<T> L, R;
-        L.lo = mk<T>(__ldcg(lb + 0), __ldcg(lb + 1), __ldcg(lb + 2));
-        L.hi = mk<T>(__ldcg(lb + 3), __ldcg(lb + 4), __ldcg(lb + 5));
-        R.lo = mk<T>(__ldcg(rb + 0), __ldcg(rb + 1), __ldcg(rb + 2));
-        R.hi = mk<T>(__ldcg(rb + 3), __ldcg(rb + 4), __ldcg(rb + 5));
-        store_box(bboxes + (base + node) * 6, merge(L, R));
-        if (node == 0) return;
-        node = tree[(base + node) * 4 + 0];
-    }
-    atomicOr(status, ST_MALFORMED_TREE);
-}
-
-// ---------------------------------------------------------------------------------------
 // Import of exported tensors into traversal nodes (build_bvh_from_array_tree 667-705 and
 // set_rightmost_nodes 707-743).
 
@@ -1522,7 +1420,7 @@ template <class T, int LIB>
 __global__ void __launch_bounds__(NARROW_THREADS)
 k_impulses_from_rows(const long long* __restrict__ rows, const T* __restrict__ roots, int B, long long N, int F,
                      const T* __restrict__ x0, const T* __restrict__ x1, const T* __restrict__ masses,
-                     T* __restrict__ dv_out, T* __restrict__ dx_out, int* __restrict__ cnt_out, WsHeader* hdr) {
+                     T* __restrict__ dv_out, T* __restrict__ dx_out, int* __restrict__ cnt_out) {
     long long total = (long long)B * N;
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < total;
          r += (long long)gridDim.x * blockDim.x) {
