@@ -7,7 +7,9 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "../../include/ccc_b200.h"
 #include "ccc_kernels.cuh"
@@ -72,27 +74,34 @@ void timing_after(int slot, cudaStream_t s) {
 namespace {
 
 // Workspace layout (every section 256-byte aligned):
-//   [header 64 B][mesh counters M][visit counters total-M]   <- zeroed per call
+//   [header 64 B][mesh counters M]   <- zeroed per call
+//   [visit counters total-M]
 //   [mesh table: count, offsets M+1, data offsets M, slot ids M][rightmost total-M]
-//   [nodes total x 64 B (mesh m's F-1 nodes from slot m*F)][candidates cap x 8 B]
+//   [nodes total x 128 B (QNode; mesh m's F-1 nodes from slot m*F)][candidates cap x 8 B]
+// A workspace too small for the four-wide nodes (ccc_find_collisions_continuous_static's fixed
+// array with more than some 250,000 triangles at 16 candidates) holds binary nodes of 64 B
+// instead, in the same order.
 struct Layout {
     int64_t hdr, mesh_cnt, visits, zero_end, moff, table, rmk, nodes, cand, end;
     int64_t cand_cap;
+    bool wide;
 };
 
-Layout layout(int64_t B, int64_t F, int64_t maxc, bool need_nodes) {
+Layout layout(int64_t B, int64_t F, int64_t maxc, bool need_nodes, bool wide = true) {
     Layout L;
     int64_t total = B * F;
     int64_t internal = total - B;
+    L.wide = wide;
     L.hdr = 0;
     L.mesh_cnt = align_up(L.hdr + (int64_t)sizeof(WsHeader), 256);
     L.visits = align_up(L.mesh_cnt + B * 4, 256);
-    L.zero_end = align_up(L.visits + internal * 4, 256);
-    L.moff = L.zero_end;
+    // (the import of the four-wide nodes clears the visit counters itself)
+    L.moff = align_up(L.visits + internal * 4, 256);
+    L.zero_end = wide ? L.mesh_cnt + B * 4 : L.moff;
     L.table = align_up(L.moff + (B + 1) * 4, 256);
     L.rmk = align_up(L.table + (3 * B + 4) * 4, 256);
     L.nodes = need_nodes ? align_up(L.rmk + internal * 4, 256) : L.rmk;
-    L.cand = need_nodes ? align_up(L.nodes + total * (int64_t)sizeof(TNode), 256) : L.nodes;
+    L.cand = need_nodes ? align_up(L.nodes + total * (int64_t)(wide ? sizeof(QNode) : sizeof(TNode)), 256) : L.nodes;
     L.cand_cap = need_nodes ? total * maxc : 0;
     L.end = align_up(L.cand + L.cand_cap * 8, 256);
     return L;
@@ -128,15 +137,15 @@ struct Prepared {
     int* visits;
     int* moff;
     int* rmk;
-    TNode* nodes;
+    char* nodes;
     int2* cand;
     int* table;
     Forest forest;
 };
 
-int prepare(void* ws, int64_t ws_bytes, int64_t B, int64_t F, int64_t maxc, bool need_nodes, cudaStream_t s,
-            Prepared& P) {
-    P.L = layout(B, F, maxc, need_nodes);
+int prepare(void* ws, int64_t ws_bytes, int64_t B, int64_t F, int64_t maxc, cudaStream_t s, Prepared& P) {
+    P.L = layout(B, F, maxc, true);
+    if (ws_bytes < P.L.end) P.L = layout(B, F, maxc, true, false);
     if (ws == nullptr || ws_bytes < P.L.end) return CCC_ERR_WORKSPACE;
     P.base = (char*)ws;
     P.hdr = (WsHeader*)(P.base + P.L.hdr);
@@ -144,7 +153,7 @@ int prepare(void* ws, int64_t ws_bytes, int64_t B, int64_t F, int64_t maxc, bool
     P.visits = (int*)(P.base + P.L.visits);
     P.moff = (int*)(P.base + P.L.moff);
     P.rmk = (int*)(P.base + P.L.rmk);
-    P.nodes = (TNode*)(P.base + P.L.nodes);
+    P.nodes = P.base + P.L.nodes;
     P.cand = (int2*)(P.base + P.L.cand);
     P.table = (int*)(P.base + P.L.table);
     // the packed table is stored twice over: moff (= voff) feeds the tensor-layout kernels
@@ -153,10 +162,18 @@ int prepare(void* ws, int64_t ws_bytes, int64_t B, int64_t F, int64_t maxc, bool
     P.forest.poff = P.table + 4;
     P.forest.sid = P.table + 4 + B;
     if (cudaMemsetAsync(P.base, 0, (size_t)P.L.zero_end, s) != cudaSuccess) return CCC_ERR_CUDA;
-    CCC_LAUNCH("k_uniform_offsets", s, k_uniform_offsets<<<grid_for(B + 1, 256), 256, 0, s>>>(
-        P.table, P.moff, P.table + 4, P.table + 4 + B, (int)B, (int)F));
-    CCC_LAUNCH_CHECK();
     return CCC_OK;
+}
+
+// the two traversal kernels' compile-time choices
+template <class T, class Fn> void with_walk(bool masked, bool exact_f32, Fn&& fn) {
+    if (masked) {
+        if (exact_f32) fn(std::true_type{}, std::true_type{});
+        else fn(std::true_type{}, std::false_type{});
+    } else {
+        if (exact_f32) fn(std::false_type{}, std::true_type{});
+        else fn(std::false_type{}, std::false_type{});
+    }
 }
 
 // import + traversal shared by every query operation; candidates land in P.cand
@@ -168,29 +185,38 @@ int run_broad_phase(const void* bboxes, const int64_t* tree, const uint8_t* mask
     int M = (int)B;
     int total = (int)(B * F);
     int internal = total - M;
-    CCC_LAUNCH("k_import_nodes", s, k_import_nodes<T><<<grid_for(internal, 256), 256, 0, s>>>(P.moff, M, internal, bb, tr, P.nodes, &P.hdr->status));
-    CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_import_rightmost", s, k_import_rightmost<<<grid_for(total, 256), 256, 0, s>>>(P.moff, M, total, tr, P.nodes, P.visits, P.rmk,
-                                                            &P.hdr->status));
-    CCC_LAUNCH_CHECK();
-    int g = grid_for(total, TRAV_THREADS);
     int cap = (int)P.L.cand_cap;
-    TensorLeaves<T> lv{bb, tr};
-    if (mask) {
-        if (exact_f32)
-            CCC_LAUNCH("k_traverse", s, k_traverse<T, true, true><<<g, TRAV_THREADS, 0, s>>>(P.nodes, lv, P.forest, mask, th,
-                                                                                             P.cand, cap, P.hdr, nullptr));
-        else
-            CCC_LAUNCH("k_traverse", s, k_traverse<T, true, false><<<g, TRAV_THREADS, 0, s>>>(P.nodes, lv, P.forest, mask, th,
-                                                                                              P.cand, cap, P.hdr, nullptr));
-    } else {
-        if (exact_f32)
-            CCC_LAUNCH("k_traverse", s, k_traverse<T, false, true><<<g, TRAV_THREADS, 0, s>>>(P.nodes, lv, P.forest, mask, th,
-                                                                                              P.cand, cap, P.hdr, nullptr));
-        else
-            CCC_LAUNCH("k_traverse", s, k_traverse<T, false, false><<<g, TRAV_THREADS, 0, s>>>(P.nodes, lv, P.forest, mask,
-                                                                                               th, P.cand, cap, P.hdr, nullptr));
+    if (P.L.wide) {
+        QNode* nodes = (QNode*)P.nodes;
+        CCC_LAUNCH("k_import_nodes", s, k_import_wide<T><<<grid_for(internal, 128), 128, 0, s>>>(
+            (int)F, M, bb, tr, nodes, P.visits, P.rmk, P.table, P.moff, P.hdr));
+        CCC_LAUNCH_CHECK();
+        CCC_LAUNCH("k_import_rightmost", s, k_import_rightmost_wide<<<grid_for(total, 256), 256, 0, s>>>(
+            (int)F, total, tr, P.visits, P.rmk, P.hdr));
+        CCC_LAUNCH_CHECK();
+        const int g = std::min(grid_for(total, WALK_WARPS), num_sms() * 8);
+        with_walk<T>(mask != nullptr, exact_f32, [&](auto masked, auto exact) {
+            CCC_LAUNCH("k_traverse", s, k_walk_tensors<T, masked.value, exact.value><<<g, WALK_THREADS, 0, s>>>(
+                nodes, bb, tr, mask, P.rmk, (int)F, P.forest, th, P.cand, cap, P.hdr));
+        });
+        CCC_LAUNCH_CHECK();
+        return CCC_OK;
     }
+    TNode* nodes = (TNode*)P.nodes;
+    CCC_LAUNCH("k_uniform_offsets", s, k_uniform_offsets<<<grid_for(B + 1, 256), 256, 0, s>>>(
+        P.table, P.moff, P.table + 4, P.table + 4 + B, M, (int)F));
+    CCC_LAUNCH_CHECK();
+    CCC_LAUNCH("k_import_nodes", s, k_import_nodes<T><<<grid_for(internal, 256), 256, 0, s>>>(
+        P.moff, M, internal, bb, tr, nodes, &P.hdr->status));
+    CCC_LAUNCH_CHECK();
+    CCC_LAUNCH("k_import_rightmost", s, k_import_rightmost<<<grid_for(total, 256), 256, 0, s>>>(
+        P.moff, M, total, tr, nodes, P.visits, P.rmk, &P.hdr->status));
+    CCC_LAUNCH_CHECK();
+    const TensorLeaves<T> lv{bb, tr};
+    with_walk<T>(mask != nullptr, exact_f32, [&](auto masked, auto exact) {
+        CCC_LAUNCH("k_traverse", s, k_traverse<T, masked.value, exact.value><<<grid_for(total, TRAV_THREADS), TRAV_THREADS, 0, s>>>(
+            nodes, lv, P.forest, mask, th, P.cand, cap, P.hdr, nullptr));
+    });
     CCC_LAUNCH_CHECK();
     return CCC_OK;
 }
@@ -238,7 +264,7 @@ template <class T>
 int static_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_t B, int64_t F, double threshold,
                 int64_t max_collisions, int64_t* out, void* ws, int64_t ws_bytes, cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, max_collisions, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, max_collisions, s, P);
     if (rc) return rc;
     // the reference passes a float threshold into T-typed kernels
     T th = (T)(float)threshold;
@@ -254,7 +280,7 @@ template <class T, int OP>
 int te_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_t B, int64_t F, int64_t max_collisions,
             int64_t* rows, void* coefs, int32_t* masks, void* ws, int64_t ws_bytes, cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, max_collisions, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, max_collisions, s, P);
     if (rc) return rc;
     // the reference's triangle-edge queries traverse and intersect with threshold 0
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, (T)0, is_f32<T>(), P, s);
@@ -294,7 +320,7 @@ int ccd_impl(const void* bboxes, const int64_t* tree, const void* x0, const void
              int64_t F, int64_t maxc, int64_t maxcol, int64_t* rows, void* times, void* ws, int64_t ws_bytes,
              cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, maxc, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, maxc, s, P);
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, mask, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
@@ -311,7 +337,7 @@ template <class T>
 int mincol_impl(const void* bboxes, const int64_t* tree, const void* x0, const void* x1, int64_t B, int64_t F,
                 int64_t maxc, int64_t* rows, void* ws, int64_t ws_bytes, cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, maxc, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, maxc, s, P);
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
@@ -328,7 +354,7 @@ template <class T>
 int prox_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_t B, int64_t F, double threshold,
               int64_t maxc, int64_t* rows, void* ws, int64_t ws_bytes, cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, maxc, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, maxc, s, P);
     if (rc) return rc;
     T th = (T)(float)threshold;
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, th, is_f32<T>() && th == 0, P, s);
@@ -344,7 +370,7 @@ int impulses_impl(const void* bboxes, const int64_t* tree, const void* x0, const
                   const uint8_t* mask, int64_t B, int64_t F, int64_t maxc, void* dv, void* dx, int32_t* cnt, void* ws,
                   int64_t ws_bytes, cudaStream_t s) {
     Prepared P;
-    int rc = prepare(ws, ws_bytes, B, F, maxc, true, s, P);
+    int rc = prepare(ws, ws_bytes, B, F, maxc, s, P);
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, mask, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
@@ -642,7 +668,7 @@ int ccc_find_collisions_continuous_static(int dtype, const void* bboxes, const i
     int rc = check_common(dtype, B, F);
     if (rc) return rc;
     if (!rows_fit(B, F, maxc) || !rows_fit(B, F, maxcol)) return CCC_ERR_INVALID_ARG;
-    int64_t need = layout(B, F, maxc, true).end;
+    int64_t need = layout(B, F, maxc, true, false).end;
     if (need > CCC_STATIC_SCRATCH_BYTES) return CCC_ERR_TOO_LARGE;
     void* base = static_scratch_base();
     if (base == nullptr) return CCC_ERR_CUDA;

@@ -46,7 +46,8 @@ struct WsHeader {
     int live_count;    // engine staging: pairs with sub-tests to solve (Weld.live)
     int pending_count; // engine staging: pairs left with vertex-face sub-tests to place
     int expand_count;  // engine narrow phase: records for k_ccd_expand (Weld.expand)
-    int pad[6];
+    int general;       // imported tree: not the radix tree of the positions
+    int pad[5];
 };
 
 struct __align__(16) TNode {

@@ -149,4 +149,217 @@ k_bvh_levels(const T* __restrict__ x0, const T* __restrict__ x1, int n, int chun
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// Import of caller tensors for the walk (build_bvh_from_array_tree, build_bvh.cu:667-705, and
+// set_rightmost_nodes, 707-743): every internal node's QNode, its children with the internal
+// ones replaced by their own children.  A replaced child is not visited itself, so each of
+// its two slots holds the intersection of its box with the child's: the query meets both, as
+// it would have to one level at a time, and for boxes that contain their children's (every
+// tree built from them) the intersection is the slot's own box.
+//
+// The rightmost leaf position below a node, which the order rule needs, is known without a
+// climb when the children are those of the radix tree of the positions (bvh and bvh_motion,
+// the reference's too); a tree with any other child raises hdr->general, and
+// k_import_rightmost_wide then climbs for all of them.  Measured for a bvh_motion tree of 52,738
+// triangles (fp64): binary nodes and climbs 34 us, four-wide nodes and no climb 10 us.
+template <class T> __device__ __forceinline__ void box_outward(const T* p, float lo[3], float hi[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if (sizeof(T) == 4) {
+            lo[c] = (float)__ldg(p + c);
+            hi[c] = (float)__ldg(p + 3 + c);
+        } else {
+            lo[c] = __double2float_rd((double)__ldg(p + c));
+            hi[c] = __double2float_ru((double)__ldg(p + 3 + c));
+        }
+    }
+}
+
+// the larger (smaller) of a and b, NaN when either is: a NaN box meets nothing
+__device__ __forceinline__ float max_nan(float a, float b) { return a != a || a > b ? a : b; }
+__device__ __forceinline__ float min_nan(float a, float b) { return a != a || a < b ? a : b; }
+
+template <class T>
+__global__ void k_import_wide(int n, int meshes, const T* __restrict__ bboxes, const long long* __restrict__ tree,
+                              QNode* __restrict__ qnodes, int* __restrict__ visits, int* __restrict__ rmk,
+                              int* __restrict__ table, int* __restrict__ moff, WsHeader* hdr) {
+    const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+    const int internal = meshes * (n - 1);
+    // the packed mesh table (Forest): count, offsets, data offsets, slot ids
+    for (int i = gi; i <= meshes; i += gridDim.x * blockDim.x) {
+        moff[i] = i * n;
+        if (i < meshes) {
+            table[4 + i] = i * n;
+            table[4 + meshes + i] = i;
+        }
+        if (i == 0) table[0] = meshes;
+    }
+    if (gi >= internal) return;
+    const int m = gi / (n - 1), k = gi - m * (n - 1);
+    const long long base = (long long)m * (2LL * n - 1);
+    const long long* tr = tree + base * 4;
+    const T* bb = bboxes + base * 6;
+    visits[gi] = 0;
+    rmk[gi] = -1;
+    const int2 r = radix_range(k, n);
+    const int2 regular = radix_children(r, 31 - __clz(r.x ^ r.y), n);
+    bool bad = false;
+    auto child = [&](int node, int side) {
+        long long c = __ldg(tr + node * 4LL + 1 + side);
+        if (c <= 0 || c >= 2LL * n - 1) {
+            bad = true;
+            c = 2LL * n - 2;                 // keep the record pointing at a valid leaf
+        }
+        return (int)c;
+    };
+    const float inf = __int_as_float(0x7f800000);
+    float lo[3][4], hi[3][4];
+    int ref[4], aux[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        ref[s] = Q_EMPTY;
+        aux[s] = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lo[c][s] = inf;
+            hi[c][s] = -inf;
+        }
+    }
+    // slot s (a constant) from row c, within the box above it when there is one
+    auto slot = [&](int s, int c, bool within, const float* alo, const float* ahi) {
+        float l[3], h[3];
+        box_outward<T>(bb + c * 6LL, l, h);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d][s] = within ? max_nan(l[d], alo[d]) : l[d];
+            hi[d][s] = within ? min_nan(h[d], ahi[d]) : h[d];
+        }
+        if (c >= n - 1) {
+            const long long id = __ldg(tr + c * 4LL + 3);
+            if (id < 0 || id >= n) bad = true;
+            ref[s] = ~(c - (n - 1));
+            aux[s] = id < 0 || id >= n ? 0 : (int)id;
+        } else {
+            ref[s] = c;
+            aux[s] = radix_range(c, n).y;    // (of a regular tree)
+        }
+    };
+    const int c0 = child(k, 0), c1 = child(k, 1);
+    if (c0 != regular.x || c1 != regular.y) hdr->general = 1;
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const int c = side ? c1 : c0;
+        if (c >= n - 1) {
+            slot(2 * side, c, false, nullptr, nullptr);
+        } else {
+            float alo[3], ahi[3];
+            box_outward<T>(bb + c * 6LL, alo, ahi);
+            slot(2 * side, child(c, 0), true, alo, ahi);
+            slot(2 * side + 1, child(c, 1), true, alo, ahi);
+        }
+    }
+    if (bad) atomicOr(&hdr->status, ST_MALFORMED_TREE);
+    QNode q;
+    q.lox = make_float4(lo[0][0], lo[0][1], lo[0][2], lo[0][3]);
+    q.loy = make_float4(lo[1][0], lo[1][1], lo[1][2], lo[1][3]);
+    q.loz = make_float4(lo[2][0], lo[2][1], lo[2][2], lo[2][3]);
+    q.hix = make_float4(hi[0][0], hi[0][1], hi[0][2], hi[0][3]);
+    q.hiy = make_float4(hi[1][0], hi[1][1], hi[1][2], hi[1][3]);
+    q.hiz = make_float4(hi[2][0], hi[2][1], hi[2][2], hi[2][3]);
+    q.ref = make_int4(ref[0], ref[1], ref[2], ref[3]);
+    q.aux = make_int4(aux[0], aux[1], aux[2], aux[3]);
+    qnodes[(long long)m * n + k] = q;        // mesh m's nodes start at its first triangle slot
+}
+
+// the rightmost leaf position below every internal node of a general tree, by climbs
+static __global__ void k_import_rightmost_wide(int n, int total, const long long* __restrict__ tree,
+                                               int* __restrict__ visits, int* __restrict__ rmk, WsHeader* hdr) {
+    if (!*(volatile int*)&hdr->general) return;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= total) return;
+    const int m = g / n, ioff = m * (n - 1);
+    const long long* tr = tree + (long long)m * (2LL * n - 1) * 4;
+    long long node = tr[(n - 1LL + (g - (long long)m * n)) * 4];
+    for (int guard = 0; guard < n; ++guard) {
+        if (node < 0 || node >= n - 1) { atomicOr(&hdr->status, ST_MALFORMED_TREE); return; }
+        __threadfence();
+        if (atomicAdd(visits + ioff + node, 1) == 0) return;
+        int r = 0;
+        for (int side = 0; side < 2; ++side) {
+            long long c = tr[node * 4 + 1 + side];
+            if (c <= 0 || c >= 2LL * n - 1) c = 2LL * n - 2;
+            r = max(r, c >= n - 1 ? (int)(c - (n - 1)) : __ldcg(rmk + ioff + c));
+        }
+        rmk[ioff + node] = r;
+        if (node == 0) return;
+        node = tr[node * 4];
+    }
+    atomicOr(&hdr->status, ST_MALFORMED_TREE);
+}
+
+// The walk over imported trees (traverseBVH, collisions_static.cu:10-103; traverseBVHPartial,
+// collisions_continuous.cu:127-230): fp32 boxes with outward rounding in the nodes, then the
+// exact reference-precision test of every leaf hit (EXACT_F32: the fp32 boxes are exact and
+// the threshold is 0, so there is nothing to test again).  MASKED: only the marked leaves
+// query, against every leaf, and of two marked triangles the smaller reports the pair.
+// Measured against one query a thread on binary nodes (which a workspace too small for the
+// four-wide ones still takes): 968 triangles 49 -> 10 us, 7,938 (fp32) 41 -> 17 us, 52,738
+// 124 -> 48 us, 130,050 260 -> 112 us, 40,800 (fp32) with 30 % marked 280 -> 42 us.
+template <class T, bool MASKED, bool EXACT_F32> struct TensorWalk {
+    const T* bboxes;
+    const long long* tree;
+    const uint8_t* mask;
+    const int* rmk;          // of a general tree
+    T th;
+    int n, general;
+    static constexpr bool ORDERED = !MASKED;
+    __device__ __forceinline__ long long row(int base, int pos) const {
+        return 2LL * base - base / n + (n - 1) + pos;     // mesh m's rows start at m (2 n - 1)
+    }
+    __device__ __forceinline__ bool query(const Forest&, int, int v, WsHeader* hdr, WalkQuery& q) const {
+        const int m = v / n;
+        q.base = m * n;
+        q.n = n;
+        q.pos = v - q.base;
+        if (MASKED && !mask[v]) return false;
+        const long long at = row(q.base, q.pos);
+        const long long id = __ldg(tree + at * 4 + 3);
+        if (id < 0 || id >= n) {
+            atomicOr(&hdr->status, ST_MALFORMED_TREE);
+            return false;
+        }
+        q.id = (int)id;
+        const T* b = bboxes + at * 6;
+        // conservative fp32 query box: threshold folded in, rounded outward, nudged one more ulp
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (EXACT_F32) {
+                q.lo[c] = (float)__ldg(b + c);
+                q.hi[c] = (float)__ldg(b + 3 + c);
+            } else {
+                q.lo[c] = nudge_down(__double2float_rd((double)__ldg(b + c) - (double)th));
+                q.hi[c] = nudge_up(__double2float_ru((double)__ldg(b + 3 + c) + (double)th));
+            }
+        }
+        return true;
+    }
+    __device__ __forceinline__ int rightmost(int base, int ref, int aux) const {
+        return general ? __ldg(rmk + (base - base / n) + ref) : aux;
+    }
+    __device__ __forceinline__ bool keep(int base, int, int pos, int id, int cpos, int cid) const {
+        if (MASKED && mask[base + cid] && !(id < cid)) return false;
+        return EXACT_F32 || overlap(load_box(bboxes + row(base, pos) * 6), load_box(bboxes + row(base, cpos) * 6), th);
+    }
+};
+
+template <class T, bool MASKED, bool EXACT_F32>
+__global__ void __launch_bounds__(WALK_THREADS, 8)
+k_walk_tensors(const QNode* __restrict__ qnodes, const T* __restrict__ bboxes, const long long* __restrict__ tree,
+               const uint8_t* __restrict__ mask, const int* __restrict__ rmk, int n, Forest F, T th,
+               int2* __restrict__ cand, int cand_cap, WsHeader* hdr) {
+    __shared__ WalkWarp S[WALK_WARPS];
+    const TensorWalk<T, MASKED, EXACT_F32> pol{bboxes, tree, mask, rmk, th, n, *(volatile int*)&hdr->general};
+    walk_forest(pol, qnodes, F, cand, cand_cap, hdr, S[threadIdx.x >> 5]);
+}
+
 }  // namespace ccc

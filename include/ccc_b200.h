@@ -96,7 +96,8 @@ int ccc_debug_stage(int op, int lib, const double* in, int in_stride, double* ou
 int ccc_debug_math(int op, const double* in, double* out, int64_t n, void* stream);
 
 /* Bytes of device scratch an operation needs for B meshes of F triangles with the given
- * per-triangle candidate capacity (ignored by CCC_OP_BVH). */
+ * per-triangle candidate capacity (ignored by CCC_OP_BVH).  The queries also run in about
+ * 64 bytes less per triangle (B * F), with tree nodes of half the width and a slower traversal. */
 int64_t ccc_workspace_size(int op, int64_t B, int64_t F, int64_t max_candidates_per_triangle);
 
 /* Copies the status word, the candidate count and up to n_mesh per-mesh row counts from
@@ -203,7 +204,8 @@ int ccc_compute_impulses_from_collisions(int dtype, const int64_t* collisions, c
  * forbids allocations): the same computation and outputs as ccc_find_collisions_continuous,
  * with its scratch in a fixed device array of ccc_static_scratch_bytes() bytes (64 MiB)
  * that every GPU loading this library holds until exit.  Problems whose scratch
- * (ccc_workspace_size(CCC_OP_CONTINUOUS, B, F, max_candidates_per_triangle)) exceeds it
+ * (ccc_workspace_size(CCC_OP_CONTINUOUS, B, F, max_candidates_per_triangle), less the 64 or
+ * so bytes per triangle that it can do without) exceeds it
  * return CCC_ERR_TOO_LARGE before any device work.  Every call looks up the array's device
  * address on the current device (cudaGetSymbolAddress, a host-side lookup, so a
  * cudaDeviceReset in between is harmless); the first call on a device also loads the
