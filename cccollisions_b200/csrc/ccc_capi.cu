@@ -77,14 +77,16 @@ namespace {
 //   [header 64 B][mesh counters M]   <- zeroed per call
 //   [visit counters total-M]
 //   [mesh table: count, offsets M+1, data offsets M, slot ids M][rightmost total-M]
-//   [nodes total x 128 B (QNode; mesh m's F-1 nodes from slot m*F)][candidates cap x 8 B]
+//   [nodes total x 128 B (QNode; mesh m's F-1 nodes from slot m*F; after the traversal, the
+//   records of the roots that passed the filter)][candidates cap x 8 B]
+//   [sub-test masks cap x 2 B, from 2^24 triangles]
 // A workspace too small for the four-wide nodes (ccc_find_collisions_continuous_static's fixed
 // array with more than some 250,000 triangles at 16 candidates) holds binary nodes of 64 B
 // instead, in the same order.
 struct Layout {
-    int64_t hdr, mesh_cnt, visits, zero_end, moff, table, rmk, nodes, cand, end;
+    int64_t hdr, mesh_cnt, visits, zero_end, moff, table, rmk, nodes, cand, masks, end;
     int64_t cand_cap;
-    bool wide;
+    bool wide, pack;
 };
 
 Layout layout(int64_t B, int64_t F, int64_t maxc, bool need_nodes, bool wide = true) {
@@ -103,7 +105,10 @@ Layout layout(int64_t B, int64_t F, int64_t maxc, bool need_nodes, bool wide = t
     L.nodes = need_nodes ? align_up(L.rmk + internal * 4, 256) : L.rmk;
     L.cand = need_nodes ? align_up(L.nodes + total * (int64_t)(wide ? sizeof(QNode) : sizeof(TNode)), 256) : L.nodes;
     L.cand_cap = need_nodes ? total * maxc : 0;
-    L.end = align_up(L.cand + L.cand_cap * 8, 256);
+    // (sub-test masks join their pairs in the candidate buffer while the slots leave room)
+    L.pack = total <= ((int64_t)1 << PACK_BITS);
+    L.masks = align_up(L.cand + L.cand_cap * 8, 256);
+    L.end = L.pack ? L.masks : align_up(L.masks + L.cand_cap * 2, 256);
     return L;
 }
 
@@ -315,6 +320,38 @@ int te_entry(int dtype, const void* bboxes, const int64_t* tree, const void* tri
                                             ws_bytes, s);
 }
 
+// one wave of resident blocks for the kernels that loop over their work, at most one block
+// for each `per` of the most items there can be
+inline int wave(int64_t items, int per, int blocks_per_sm) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>((items + per - 1) / per, (int64_t)num_sms() * blocks_per_sm));
+}
+
+template <class T> CcdArgs<T> ccd_args(const Prepared& P, const void* x0, const void* x1) {
+    CcdArgs<T> A{};
+    A.cand = P.cand;
+    A.masks = P.L.pack ? nullptr : (const unsigned short*)(P.base + P.L.masks);
+    A.cand_cap = (int)P.L.cand_cap;
+    A.hdr = P.hdr;
+    A.x0 = (const T*)x0;
+    A.x1 = (const T*)x1;
+    A.F = P.forest;
+    A.mesh_counters = P.mesh_cnt;
+    // (the nodes are not read after the traversal)
+    A.W.expand = (int4*)P.nodes;
+    A.W.expand_cap = (int)std::min<int64_t>((P.L.cand - P.L.nodes) / (int64_t)sizeof(int4), (int64_t)1 << 30);
+    return A;
+}
+
+// the sub-test masks of the candidates, into the candidate buffer (MASK_PACK) or as rows
+template <class T, int USE>
+int run_masks(const Prepared& P, const CcdArgs<T>& A, long long* rows, int max_per_tri, cudaStream_t s) {
+    CCC_LAUNCH("k_ccd_mask", s, k_ccd_mask<T, USE><<<wave(P.L.cand_cap, STAGE_THREADS, 3), STAGE_THREADS, 0, s>>>(
+        P.cand, A.cand_cap, P.hdr, A.x0, A.x1, const_cast<unsigned short*>(A.masks), nullptr, P.forest, rows,
+        max_per_tri, P.mesh_cnt));
+    CCC_LAUNCH_CHECK();
+    return CCC_OK;
+}
+
 template <class T>
 int ccd_impl(const void* bboxes, const int64_t* tree, const void* x0, const void* x1, const uint8_t* mask, int64_t B,
              int64_t F, int64_t maxc, int64_t maxcol, int64_t* rows, void* times, void* ws, int64_t ws_bytes,
@@ -324,10 +361,15 @@ int ccd_impl(const void* bboxes, const int64_t* tree, const void* x0, const void
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, mask, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
+    CcdArgs<T> A = ccd_args<T>(P, x0, x1);
+    A.rows = (long long*)rows;
+    A.times = (T*)times;
+    A.max_per_tri = (int)maxcol;
+    rc = run_masks<T, MASK_PACK>(P, A, nullptr, 0, s);
+    if (rc) return rc;
     cudaError_t le = cudaSuccess;
-    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIBV, SRC_CANDIDATES>(
-        num_sms() * CCD_MIN_BLOCKS, s, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)x0, (const T*)x1, P.forest, (long long*)rows,
-        (T*)times, (int)maxcol, P.mesh_cnt, Weld{}, CornerSink<T>{})));
+    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIBV, SRC_PACKED>(
+        wave(P.L.cand_cap, CCD_BLOCK, ccd_min_blocks(1)), s, A, CornerSink<T>{})));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -341,13 +383,7 @@ int mincol_impl(const void* bboxes, const int64_t* tree, const void* x0, const v
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
-    cudaError_t le = cudaSuccess;
-    CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_MINCOL, CornerSink<T>, LIB_PORTABLE, SRC_CANDIDATES>(
-        num_sms() * CCD_MIN_BLOCKS, s, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)x0, (const T*)x1, P.forest, (long long*)rows,
-        nullptr, (int)(maxc * 15), P.mesh_cnt, Weld{}, CornerSink<T>{}));
-    if (le != cudaSuccess) return CCC_ERR_CUDA;
-    CCC_LAUNCH_CHECK();
-    return CCC_OK;
+    return run_masks<T, MASK_ROWS>(P, ccd_args<T>(P, x0, x1), (long long*)rows, (int)(maxc * 15), s);
 }
 
 template <class T>
@@ -374,10 +410,17 @@ int impulses_impl(const void* bboxes, const int64_t* tree, const void* x0, const
     if (rc) return rc;
     rc = run_broad_phase<T>(bboxes, tree, mask, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
+    const CcdArgs<T> A = ccd_args<T>(P, x0, x1);
+    rc = run_masks<T, MASK_PACK>(P, A, nullptr, 0, s);
+    if (rc) return rc;
+    const CornerSink<T> sink{(const T*)masses, (T*)dv, (T*)dx, (int*)cnt};
     cudaError_t le = cudaSuccess;
-    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_IMPULSES, CornerSink<T>, LIBV, SRC_CANDIDATES>(
-        num_sms() * CCD_MIN_BLOCKS, s, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)x0, (const T*)x1, P.forest, nullptr, nullptr, 0,
-        P.mesh_cnt, Weld{}, CornerSink<T>{(const T*)masses, (T*)dv, (T*)dx, (int*)cnt})));
+    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_IMPULSES, CornerSink<T>, LIBV, SRC_PACKED>(
+        wave(P.L.cand_cap, CCD_BLOCK, ccd_min_blocks(1)), s, A, sink)));
+    if (le != cudaSuccess) return CCC_ERR_CUDA;
+    CCC_LAUNCH_CHECK();
+    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_contacts", s, le = launch_ccd_contacts<T, CornerSink<T>, LIBV>(
+        wave(P.L.cand_cap, 128, 8), s, A, sink)));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
     return CCC_OK;

@@ -197,9 +197,53 @@ CCC_HD double ccc_certmul2_hi(double x0, double x1, double y) {
     return ccc_certmul(x0, x1, 2, y).hi;
 }
 
-// Leading terms the solver uses: x^2 (as a 2-term expansion) and x^3 = (x^2) * x.
+// x^2 as a 2-term expansion, certifiedMul<1,1,2>(x, x).
 CCC_HD ccc_dd ccc_sq_dd(double x) { return ccc_certmul1(x, x); }
-CCC_HD double ccc_cube_hi(double x) {
-    ccc_dd s = ccc_sq_dd(x);
-    return ccc_certmul2_hi(s.hi, s.lo, x);
+
+// x^2 (2 terms) and the leading term of x^3 = certifiedMul<2,1,2>(x^2, x), as the solver uses
+// them for its coefficients.
+struct ccc_powers {
+    double sq, sq_lo, cube;
+};
+CCC_HD_CALL ccc_powers ccc_powers_any(double x) {
+    const ccc_dd s = ccc_sq_dd(x);
+    ccc_powers r;
+    r.sq = s.hi;
+    r.sq_lo = s.lo;
+    r.cube = ccc_certmul2_hi(s.hi, s.lo, x);
+    return r;
 }
+
+// Whether r, the exact rest of a product rounded to c, is clear of half an ulp of c by 2^-25
+// of it, and c no power of two.  For the products below, half an ulp of c is 2^25 or 2^26 times
+// the 2^(e0-80) that the short paths ask for, so this implies their test, in a few operations
+// on c's high word.
+CCC_HD bool ccc_clear_of_tie(double c, double r) {
+    const uint32_t h = (uint32_t)(ccc_dbits(c) >> 32);
+    // (2^-53 of c's binade) (1 - 2^-25)
+    const double lim = ccc_dfrombits(((uint64_t)((h & 0x7ff00000u) - (53u << 20) - 1u) << 32) | 0xf0000000u);
+    return (h & 0x000fffffu) != 0 && fabs(r) < lim;
+}
+
+// The short paths of both products under one range test: with x between 2^-150 and 2^150
+// every exponent in them is in their range, and the square's rest is at most half its ulp.
+// About 30 instructions against some 100 of the two short paths one after the other; the
+// ones that fail a test (a few in 10^7, and zeros) take those.
+CCC_HD ccc_powers ccc_square_and_cube(double x) {
+    const uint32_t h = (uint32_t)(ccc_dbits(x) >> 32) & 0x7fffffffu;
+    const double p = ccc_mul(x, x);
+    const double e = ccc_fma(x, x, -p);
+    const double q = ccc_mul(p, x);
+    const double rest = ccc_add(ccc_fma(p, x, -q), ccc_mul(e, x));
+    const double c = ccc_add(q, rest);
+    const double res = ccc_add(ccc_sub(q, c), rest);
+    if (h - (873u << 20) < (300u << 20) && ccc_clear_of_tie(p, e) && ccc_clear_of_tie(c, res)) {
+        ccc_powers r;
+        r.sq = p;
+        r.sq_lo = e;
+        r.cube = c;
+        return r;
+    }
+    return ccc_powers_any(x);
+}
+CCC_HD double ccc_cube_hi(double x) { return ccc_square_and_cube(x).cube; }

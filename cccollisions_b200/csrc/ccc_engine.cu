@@ -362,6 +362,18 @@ template <class T> int stage(ccc_engine* e, cudaStream_t s) {
     return CCC_OK;
 }
 
+template <class T> CcdArgs<T> engine_args(ccc_engine* e, const Forest& f, const Weld& W) {
+    CcdArgs<T> A{};
+    A.cand_cap = (int)e->L.cand_cap;
+    A.hdr = e->hdr();
+    A.x0 = e->at<T>(e->L.x0);
+    A.x1 = e->at<T>(e->L.x1);
+    A.F = f;
+    A.mesh_counters = e->at<int>(e->L.mesh_cnt);
+    A.W = W;
+    return A;
+}
+
 template <class T> int ccd_step(ccc_engine* e, cudaStream_t s) {
     if (cudaMemsetAsync(e->base, 0, e->L.zero_bytes, s) != cudaSuccess) return CCC_ERR_CUDA;
     Tables t = e->active();
@@ -383,18 +395,19 @@ template <class T> int ccd_step(ccc_engine* e, cudaStream_t s) {
     if (rc) return rc;
     rc = stage<T>(e, s);
     if (rc) return rc;
-    int g = num_sms() * ccd_min_blocks(SRC_STAGED, SHAPES[e->shape].batch) * SHAPES[e->shape].narrow;
+    const int batch = SHAPES[e->shape].batch;
+    const int g = num_sms() * ccd_min_blocks(batch) * SHAPES[e->shape].narrow;
+    CcdArgs<T> A = engine_args<T>(e, t.f, engine_weld(e));
+    A.rows = e->at<long long>(e->L.rows);
+    A.times = e->at<T>(e->L.times);
+    A.max_per_tri = (int)e->maxcol;
     cudaError_t le = cudaSuccess;
-    if (SHAPES[e->shape].batch == 2)
+    if (batch == 2)
         CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIBV, SRC_STAGED, 2>(
-            g, s, e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), e->at<T>(e->L.x0), e->at<T>(e->L.x1), t.f,
-            e->at<long long>(e->L.rows), e->at<T>(e->L.times), (int)e->maxcol, e->at<int>(e->L.mesh_cnt),
-            engine_weld(e), CornerSink<T>{})));
+            g, s, A, CornerSink<T>{})));
     else
         CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIBV, SRC_STAGED>(
-            g, s, e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), e->at<T>(e->L.x0), e->at<T>(e->L.x1), t.f,
-            e->at<long long>(e->L.rows), e->at<T>(e->L.times), (int)e->maxcol, e->at<int>(e->L.mesh_cnt),
-            engine_weld(e), CornerSink<T>{})));
+            g, s, A, CornerSink<T>{})));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
     CCC_LAUNCH("k_ccd_expand", s, k_ccd_expand<T><<<num_sms() * 8, EXPAND_THREADS, 0, s>>>(
@@ -416,13 +429,24 @@ template <class T> int loop_step(ccc_engine* e, int max_iter, cudaStream_t s) {
     if (rc) return rc;
     rc = traverse<T>(e, t, flags, nullptr, s);
     if (rc) return rc;
-    int g = num_sms() * CCD_MIN_BLOCKS * SHAPES[e->shape].narrow;
-    const Weld W{};
+    Weld W{};
+    W.live = e->at<int4>(e->L.live);
+    W.expand = e->at<int4>(e->L.pending);
+    W.expand_cap = (int)e->L.cand_cap;
+    const CcdArgs<T> A = engine_args<T>(e, t.f, W);
+    CCC_LAUNCH("k_ccd_mask", s, k_ccd_mask<T, MASK_LIST><<<num_sms() * 3, STAGE_THREADS, 0, s>>>(
+        e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), A.x0, A.x1, nullptr, e->at<int4>(e->L.live), t.f,
+        nullptr, 0, A.mesh_counters));
+    CCC_LAUNCH_CHECK();
     LoopSink<T> sink{e->at<T>(e->L.masses), e->at<int>(e->L.faces), t.vt, e->at<long long>(e->L.acc), contacts};
+    const int g = num_sms() * ccd_min_blocks(1) * SHAPES[e->shape].narrow;
     cudaError_t le = cudaSuccess;
-    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIBV, SRC_EXACT>(
-        g, s, e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), e->at<T>(e->L.x0), e->at<T>(e->L.x1), t.f,
-        nullptr, nullptr, 0, e->at<int>(e->L.mesh_cnt), W, sink)));
+    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_narrow", s, le = launch_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIBV, SRC_STAGED>(
+        g, s, A, sink)));
+    if (le != cudaSuccess) return CCC_ERR_CUDA;
+    CCC_LAUNCH_CHECK();
+    CCC_WITH_LIB(CCC_LAUNCH("k_ccd_contacts", s, le = launch_ccd_contacts<T, LoopSink<T>, LIBV>(
+        num_sms() * 8, s, A, sink)));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
     CCC_LAUNCH("k_loop_update", s, k_loop_update<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(
@@ -518,8 +542,8 @@ bool active_built(const ccc_engine* e) {
 template <class T> bool prepare_kernels() {
     return prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_PORTABLE, SRC_STAGED>() == cudaSuccess &&
-           prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_REFERENCE, SRC_EXACT>() == cudaSuccess &&
-           prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_PORTABLE, SRC_EXACT>() == cudaSuccess &&
+           prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
+           prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_PORTABLE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_REFERENCE, SRC_STAGED, 2>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_PORTABLE, SRC_STAGED, 2>() == cudaSuccess;
 }

@@ -478,12 +478,14 @@ k_te_narrow(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T*
     }
 }
 
-enum CcdMode { CCD_ROWS = 0, CCD_IMPULSES = 1, CCD_MINCOL = 2 };
-// where the continuous narrow phase takes its pairs from: the candidate buffer (the
-// reference-format operations), the candidate buffer with the pairs' exact leaf boxes
-// tested as well (the engine's impulse loop, whose candidates come from fp32 boxes rounded
-// outward), or the engine's staged list (shared sub-tests)
-enum CcdSource { SRC_CANDIDATES = 0, SRC_EXACT = 1, SRC_STAGED = 2 };
+// what becomes of a root that passes the filter: a row of find_collisions_continuous, or a
+// contact whose impulses go to a sink
+enum CcdMode { CCD_ROWS = 0, CCD_IMPULSES = 1 };
+// where the continuous narrow phase takes its pairs and their sub-tests from: the candidate
+// buffer with the masks that k_ccd_mask left in it (reference-format operations), or the
+// engine's list of pairs with work (the collision step's shared sub-tests, k_ccd_stage_*, or
+// the impulse loop's, k_ccd_mask)
+enum CcdSource { SRC_PACKED = 0, SRC_STAGED = 1 };
 
 // Receiver of the impulses of CCD_IMPULSES: per-corner sums and counters (F, 3, 3) / (F, 3)
 // of the reference's compute_impulses.  Per-corner masses (F, 3) feed the contact.
@@ -499,64 +501,62 @@ template <class T> struct CornerSink {
 };
 
 // Continuous narrow phase (collisions_continuous.cu:14-765, collisions_impulses.cu:24-1067),
-// block-synchronous.  Blocks of CCD_BLOCK threads loop over chunks of CCD_BLOCK candidate
-// pairs.  Every thread runs the shared-vertex test and the 15 swept sub-box tests of its
-// pair, and the surviving (pair, type) sub-tests are appended to a ring queue in shared
-// memory.  Whenever a full batch of CCD_BATCH sub-tests is queued (and once more at the end
-// for the remainder), the block solves it in three phases separated by barriers, so that
-// every warp of the block runs the same phase's code at the same time:
-//   (1) cubic coefficients and the solver prefix of every sub-test, which classifies it;
-//   (2) the roots, with the sub-tests ordered by solver branch;
-//   (3) the root filter and the output of every root in [0, 1], edge-edge roots first and
-//       vertex-face roots after them, so that a warp runs one of the two filters.
+// block-synchronous: blocks of CCD_BLOCK threads take CCD_BLOCK pairs at a time and queue
+// their sub-tests, and each stage of the solve runs on a full block of its own queue's
+// entries, so that every warp of the block runs the same stage's code at the same time:
+//   (1) the cubic's coefficients; sub-tests without a root in [0, 1] for certain end here
+//       (cubic_misses), the others are queued with their coefficients;
+//   (2) the solver prefix, which classifies them, and the roots, ordered by solver branch; the
+//       roots in [0, 1] are queued, edge-edge ones from the front of their array and
+//       vertex-face ones from its back;
+//   (3) the root filter, a warp at a time of one kind of root; the roots that pass leave a
+//       record (or, for the reference's rows, a row).
 // Sub-tests take different branches and have 0 to 3 roots: solved in arrival order they
-// leave most lanes idle, and a kernel whose warps are in different phases needs all of its
-// code in the instruction cache at once.  Queued batches are always full, so no phase runs
-// with a partly empty round of threads.
-#ifndef CCC_CCD_BLOCK
-#define CCC_CCD_BLOCK 256
-#endif
-#ifndef CCC_CCD_MIN_BLOCKS
-#define CCC_CCD_MIN_BLOCKS 3
-#endif
-#ifndef CCC_CCD_BATCH_MULT
-#define CCC_CCD_BATCH_MULT 1
-#endif
-static constexpr int CCD_BLOCK = CCC_CCD_BLOCK;
-static constexpr int CCD_MIN_BLOCKS = CCC_CCD_MIN_BLOCKS;      // resident blocks per SM
-// the engine's staged kernel with batches of 256 needs no more than 64 registers, so four
-// of its blocks fit an SM
-static constexpr int CCD_MIN_BLOCKS_STAGED = 4;
-constexpr int ccd_min_blocks(int src, int bm) {
-    return src == SRC_STAGED && bm == 1 ? CCD_MIN_BLOCKS_STAGED : CCD_MIN_BLOCKS;
-}
-static constexpr int CCD_BATCH = CCC_CCD_BATCH_MULT * CCD_BLOCK;
-static_assert(CCD_BLOCK % 32 == 0 && CCD_BLOCK <= 1024 && 3 * CCD_BATCH <= 65536, "CCD_BLOCK");
+// leave most lanes idle, and a kernel whose warps are in different stages needs all of its
+// code in the instruction cache at once.  A stage that took only what the stage before it
+// left of its batch would run with most of its threads idle between two barriers: on the
+// 256 x 256 fold, three sub-tests in four have no root in [0, 1].
+// Measured against one kernel that staged, solved and applied a batch from end to end (fp64):
+// the fold's impulses 1,698 -> 109 (masks) + 752 + 82 us (contacts), ten served folds 931 ->
+// 94 + 445 + 39 us an iteration, the cloth over the sphere 214 -> 21 + 161 us, 968 triangles
+// 45 -> 5 + 15 + 6 us; the 64-mesh step, whose masks were apart already, 5,336 -> 4,950 us.
+// What bounds it: instruction issue (52-57 % of the slots at 26-28 of 32 lanes; some 2,100
+// instructions per 32 sub-tests, a quarter of them in the FP64 pipe), with waits for fixed
+// latencies 2.6, barriers 2.0 and memory 1.6-2.6 warps an issue.  Blocks of 128 threads: 5,219
+// against 5,168 us on the 64 meshes, 801 against 759 us on the fold.
+static constexpr int CCD_BLOCK = 256;
+// resident blocks per SM (64 registers a thread, 54 KB of shared memory a block)
+constexpr int ccd_min_blocks(int bm) { return bm == 1 ? 4 : 2; }
+static_assert(CCD_BLOCK % 32 == 0 && CCD_BLOCK <= 1024, "CCD_BLOCK");
 
 constexpr size_t align16(size_t x) { return (x + 15) / 16 * 16; }
 
 // dynamic shared memory of one block (byte offsets) for batches of NB sub-tests
-template <class T, int NB = CCD_BATCH> struct CcdLayout {
-    static constexpr int QUEUE = NB + 15 * CCD_BLOCK;     // a partial batch plus a chunk's worst case
-    static constexpr size_t rec = 0;                                                   // double [6][NB]
-    static constexpr size_t root_val = rec + 6 * NB * sizeof(double);                  // T [3 NB]
-    static constexpr size_t items = align16(root_val + 3 * NB * sizeof(T));            // int2 [QUEUE]
-    static constexpr size_t clist = items + QUEUE * sizeof(int2);                      // u16 [NB]
-    static constexpr size_t root_rec = clist + NB * 2;                                 // u16 [3 NB]
-    static constexpr size_t rec_cls = root_rec + 3 * NB * 2;                           // u8 [NB]
-    static constexpr size_t rec_pos = align16(rec_cls + NB);                           // u16 [NB]
-    static constexpr size_t spairs = align16(rec_pos + NB * 2);                        // int2 [BLOCK]
-    static constexpr size_t pbuf = spairs + CCD_BLOCK * sizeof(int2);                   // u16 [BLOCK / 32][64]
-    static constexpr size_t ints = align16(pbuf + (CCD_BLOCK / 32) * 64 * 2);          // int [64]
+template <class T, int NB> struct CcdLayout {
+    static constexpr int ITEMS = NB + 3 * CCD_BLOCK;      // less than a batch, and an intake
+    static constexpr int SURV = 2 * NB;                   // less than a batch, and a batch
+    // less than a round of warps and two partial ones, and three roots of a batch
+    static constexpr int ROOTS = 3 * NB + CCD_BLOCK + 32;
+    static constexpr int OUT = CCD_BLOCK;
+    static constexpr size_t coef = 0;                                                  // double [4][SURV]
+    static constexpr size_t gh = coef + 4 * SURV * sizeof(double);                     // double [2][NB]
+    static constexpr size_t out = gh + 2 * NB * sizeof(double);                        // int4 [OUT]
+    static constexpr size_t root_val = out + OUT * sizeof(int4);                       // T [ROOTS]
+    static constexpr size_t root_item = align16(root_val + ROOTS * sizeof(T));         // int2 [ROOTS]
+    static constexpr size_t items = root_item + ROOTS * sizeof(int2);                  // int2 [ITEMS]
+    static constexpr size_t surv = items + ITEMS * sizeof(int2);                       // int2 [SURV]
+    static constexpr size_t clist = surv + SURV * sizeof(int2);                        // u16 [NB]
+    static constexpr size_t pos = clist + NB * 2;                                      // u16 [NB]
+    static constexpr size_t cls = pos + NB * 2;                                        // u8 [NB]
+    static constexpr size_t ints = align16(cls + NB);                                  // int [64]
     static constexpr size_t bytes = ints + 64 * sizeof(int);
-    static_assert(3 * NB <= 65536, "batch indices are 16-bit");
+    static_assert(NB <= 65536, "batch indices are 16-bit");
 };
 
-// slots of the small int area
-// (class counts and root counts come in two sets, used by alternate batches; each set of
-// root counts holds the edge-edge and the vertex-face count)
-// (the live-pair counter of a chunk also comes in two, used by alternate chunks)
-enum CcdInts { CI_WARP = 0, CI_TOTAL = 32, CI_COUNT = 33, CI_ROOTS = 41, CI_LIVE = 45 };
+// slots of the small int area: the intake's warp counts and total; the survivors queued since
+// the kernel began; the solver classes' counts (two sets, used by alternate batches); the
+// queued roots of each kind; the buffered records and where they go
+enum CcdInts { CI_WARP = 0, CI_TOTAL = 32, CI_SURV = 33, CI_COUNT = 34, CI_EE = 42, CI_VF = 43, CI_OUT = 44, CI_BASE = 45 };
 
 // a queued sub-test: triangle slots i and j, type k in the top bits of j (slots < 2^28),
 // bit 28 of i set when the sub-test stands for all its repeats (see Weld)
@@ -607,10 +607,10 @@ struct Weld {
     const int4* live;      // the pairs with sub-tests to solve (hdr->live_count of them, from
                            // k_ccd_stage_*): slots i, j and the sub-tests it solves (bits
                            // 0..14) with those that stand for their repeats (bits 15..29)
-    int4* expand;          // the roots that passed the filter, for k_ccd_expand
-                           // (hdr->expand_count, at most expand_cap): slots i | shared << 28,
-                           // j | type << 28, the root as a double (low, high words); null:
-                           // k_ccd_narrow writes the rows itself
+    int4* expand;          // the roots that passed the filter, for k_ccd_expand or
+                           // k_ccd_contacts (hdr->expand_count, at most expand_cap): slots
+                           // i | shared << 28, j | type << 28, the root as a double (low, high
+                           // words)
     int expand_cap;
 };
 
@@ -973,340 +973,475 @@ k_ccd_stage_pending(int cand_cap, WsHeader* hdr, Weld W, const int4* __restrict_
     }
 }
 
+// The sub-tests of every candidate pair of the operations without corner classes: pairs whose
+// triangles share a vertex (equal coordinates) have none; the others queue per warp in shared
+// memory and are taken 32 at a time for the swept sub-box tests, as in k_ccd_stage_mask (about
+// half of the pairs are mesh neighbours, and gathering the rest keeps the warps full).
+//  * MASK_PACK: the mask joins its pair in the candidate buffer: bits 0..7 above the first slot,
+//    8..14 above the second (slots below 2^24), or in `masks` when that is given;
+//  * MASK_LIST: the pairs with sub-tests go to the list `live` (the engine's impulse loop,
+//    whose candidates come from fp32 boxes rounded outward: with the exact leaf-box test);
+//  * MASK_ROWS: a row (i, j, type) per sub-test (find_mincol_cand).
+enum MaskUse { MASK_PACK = 0, MASK_LIST = 1, MASK_ROWS = 2 };
+constexpr int PACK_BITS = 24;
+constexpr int PACK_MASK = (1 << PACK_BITS) - 1;
+
+template <class T, int USE>
+__global__ void __launch_bounds__(STAGE_THREADS, 3)
+k_ccd_mask(int2* cand, int cand_cap, WsHeader* hdr, const T* __restrict__ x0, const T* __restrict__ x1,
+           unsigned short* __restrict__ masks, int4* __restrict__ live, Forest F, long long* __restrict__ rows,
+           int max_per_tri, int* __restrict__ mesh_counters) {
+    __shared__ int2 q_pr[STAGE_WARPS][64];
+    __shared__ int q_at[STAGE_WARPS][64];
+    const int n = min(*(volatile int*)&hdr->cand_count, cand_cap);
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int warps = gridDim.x * STAGE_WARPS;
+    int masked = 0, qn = 0;             // qn: queued pairs of this warp (warp-uniform)
+    for (long long base = (blockIdx.x * STAGE_WARPS + wq) * 32LL;; base += warps * 32LL) {
+        const bool more = base < n;
+        if (!more && qn == 0) break;
+        if (more) {
+            const long long c = base + lane;
+            int2 pr = make_int2(0, 0);
+            bool lv = false;
+            if (c < n) {
+                pr = cand[c];
+                lv = !ccd_pair_shares_vertex<T>(x0, pr.x, pr.y);
+                if (USE == MASK_PACK && masks && !lv) masks[c] = 0;
+            }
+            const unsigned m = __ballot_sync(FULL, lv);
+            if (lv) {
+                const int at = qn + __popc(m & lt);
+                q_pr[wq][at] = pr;
+                q_at[wq][at] = (int)c;
+            }
+            qn += __popc(m);
+            __syncwarp();
+        }
+        while (qn >= 32 || (!more && qn > 0)) {
+            const bool valid = lane < qn;
+            int2 pr = make_int2(0, 0);
+            unsigned bits = 0u;
+            if (valid) {
+                pr = q_pr[wq][lane];
+                bits = ccd_pair_subbox_mask<T, USE != MASK_ROWS, USE == MASK_LIST>(x0, x1, pr.x, pr.y);
+                masked += __popc(bits);
+                if (USE == MASK_PACK) {
+                    const int at = q_at[wq][lane];
+                    if (masks) masks[at] = (unsigned short)bits;
+                    else if (bits)
+                        cand[at] = make_int2(pr.x | (int)((bits & 0xffu) << PACK_BITS),
+                                             pr.y | (int)((bits >> 8) << PACK_BITS));
+                }
+            }
+            if (USE == MASK_LIST) {
+                // (at most one record per candidate)
+                const unsigned ml = __ballot_sync(FULL, bits != 0u);
+                int b0 = 0;
+                if (lane == 0 && ml) b0 = atomicAdd(&hdr->live_count, __popc(ml));
+                b0 = __shfl_sync(FULL, b0, 0) + __popc(ml & lt);
+                if (bits) live[b0] = make_int4(pr.x, pr.y, (int)bits, 0);
+            }
+            if (USE == MASK_ROWS) {
+                while (bits) {
+                    const int k = __ffs(bits) - 1;
+                    bits &= bits - 1;
+                    const OutRegion R = out_region(F, forest_size(F), pr.x, max_per_tri);
+                    const long long r = append_row(mesh_counters, F, R.m, R.cap, &hdr->status);
+                    if (r >= 0) {
+                        const long long o = (long long)R.po * max_per_tri + r;
+                        rows[o * 3 + 0] = pr.x - R.po;
+                        rows[o * 3 + 1] = pr.y - R.po;
+                        rows[o * 3 + 2] = k;
+                    }
+                }
+            }
+            // the queue's second half moves to the front
+            __syncwarp();
+            if (lane + 32 < qn) {
+                q_pr[wq][lane] = q_pr[wq][lane + 32];
+                q_at[wq][lane] = q_at[wq][lane + 32];
+            }
+            qn = qn > 32 ? qn - 32 : 0;
+            __syncwarp();
+        }
+    }
+    if (USE != MASK_ROWS) {
+        masked = __reduce_add_sync(FULL, masked);
+        if (lane == 0 && masked) atomicAdd(&hdr->subtests, masked);
+    }
+}
+
+// What k_ccd_narrow and k_ccd_contacts work on.
+template <class T> struct CcdArgs {
+    const int2* cand;               // SRC_PACKED: the pairs with their masks
+    const unsigned short* masks;    // ... null: packed into the pairs
+    int cand_cap;
+    WsHeader* hdr;
+    const T* x0;
+    const T* x1;
+    Forest F;
+    long long* rows;                // CCD_ROWS
+    T* times;
+    int max_per_tri;
+    int* mesh_counters;
+    Weld W;                         // live (SRC_STAGED), expand, and the classes when sub-tests are shared
+};
+
 // The continuous narrow phase is compiled in one translation unit only, ccc_narrow.cu, with
 // nvcc's default multiply-add contraction as the reference is compiled (CUDA's pow, which the
 // solver calls, computes slightly different results on rare arguments under -fmad=false);
 // every operation of this library's own in it is contraction-proof (mulrn / addrn / subrn,
-// fmaT).  The other units see only the launcher's declaration; ccc_narrow.cu instantiates
+// fmaT).  The other units see only the launchers' declarations; ccc_narrow.cu instantiates
 // the (type, mode, sink, math library) combinations the library launches.
 template <class T, int MODE, class Sink, int LIB, int SRC, int BM = 1>
-cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const int2* cand, int cand_cap, WsHeader* hdr, const T* x0,
-                              const T* x1, Forest F, long long* rows, T* times, int max_per_tri, int* mesh_counters,
-                              Weld W, Sink sink);
+cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink);
 template <class T, int MODE, class Sink, int LIB, int SRC, int BM = 1> cudaError_t prepare_ccd_narrow();
+// the contacts of the records that launch_ccd_narrow<CCD_IMPULSES> left
+template <class T, class Sink, int LIB>
+cudaError_t launch_ccd_contacts(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink);
 
 #ifdef CCC_NARROW_TU
+// the contact of one root (i, j, type, time) and its impulses
+template <class T, class Sink, int LIB>
+__device__ __forceinline__ void contact_of_root(const CcdArgs<T>& A, const Sink& sink, int i, int j, int k, T root) {
+    const MTet<T> tet = load_tet(A.x0, A.x1, i, j, k);
+    T mq[4];
+#pragma unroll
+    for (int pt = 0; pt < 4; ++pt)
+        mq[pt] = sink.masses[(long long)(tet_side(k, pt) ? j : i) * 3 + tet_corner(k, pt)];
+    const Contact<T> ct = contact<T, LIB>(tet, k, root, mq);
+    sink.add(tet, i, j, k, root, ct, A.F, forest_size(A.F), &A.hdr->status);
+}
+
+// The consequences of one record in place, for the records that do not fit their list (which
+// has room for several a triangle): every row of the root, or its contact.
+template <class T, int MODE, class Sink, int LIB>
+__device__ __noinline__ void record_in_place(const CcdArgs<T>* A, const Sink* sink, int4 rec) {
+    const int qx = rec.x & SLOT_MASK, qy = rec.y & SLOT_MASK, k = (rec.y >> 28) & 15;
+    const T root = (T)__hiloint2double(rec.w, rec.z);
+    if (MODE == CCD_ROWS) {
+        const OutRegion R = out_region(A->F, forest_size(A->F), qx, A->max_per_tri);
+        auto row = [&](int a, int b, int kk) {
+            const long long r = append_row(A->mesh_counters, A->F, R.m, R.cap, &A->hdr->status);
+            if (r >= 0) {
+                const long long o = (long long)R.po * A->max_per_tri + r;
+                A->rows[o * 3 + 0] = a - R.po;
+                A->rows[o * 3 + 1] = b - R.po;
+                A->rows[o * 3 + 2] = kk;
+                A->times[o] = root;
+            }
+        };
+        const bool shared = (rec.x >> 28) & 1;
+        if (!(shared && weld_members(A->W, qx, qy, k, __ldg(A->W.vid + qx), __ldg(A->W.vid + qy), row))) row(qx, qy, k);
+    } else {
+        contact_of_root<T, Sink, LIB>(*A, *sink, qx, qy, k, root);
+    }
+}
+
 template <class T, int MODE, class Sink, int LIB, int SRC, int BM>
-__global__ void __launch_bounds__(CCD_BLOCK, ccd_min_blocks(SRC, BM))
-k_ccd_narrow(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T* __restrict__ x0,
-             const T* __restrict__ x1, Forest F, long long* __restrict__ rows, T* __restrict__ times, int max_per_tri,
-             int* __restrict__ mesh_counters, Weld W, Sink sink) {
+__global__ void __launch_bounds__(CCD_BLOCK, ccd_min_blocks(BM))
+k_ccd_narrow(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink sink) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using L = CcdLayout<T, BM * CCD_BLOCK>;
-    constexpr bool STAGED = SRC == SRC_STAGED;
-    double* rec = reinterpret_cast<double*>(smem + L::rec);
-    T* root_val = reinterpret_cast<T*>(smem + L::root_val);
-    int2* items = reinterpret_cast<int2*>(smem + L::items);
-    unsigned short* clist = reinterpret_cast<unsigned short*>(smem + L::clist);
-    unsigned short* root_rec = reinterpret_cast<unsigned short*>(smem + L::root_rec);
-    unsigned char* rec_cls = smem + L::rec_cls;
-    unsigned short* rec_pos = reinterpret_cast<unsigned short*>(smem + L::rec_pos);
-    int2* spairs = reinterpret_cast<int2*>(smem + L::spairs);
-    unsigned short* pbuf = reinterpret_cast<unsigned short*>(smem + L::pbuf);
-    int* ints = reinterpret_cast<int*>(smem + L::ints);
-    constexpr int NW = CCD_BLOCK / 32;
     constexpr int NB = BM * CCD_BLOCK;
-    constexpr int Q = L::QUEUE;
-    const int M = forest_size(F);
+    constexpr int NW = CCD_BLOCK / 32;
+    using L = CcdLayout<T, NB>;
+    double* coef = reinterpret_cast<double*>(smem + L::coef);
+    double* gh = reinterpret_cast<double*>(smem + L::gh);
+    int4* out = reinterpret_cast<int4*>(smem + L::out);
+    T* root_val = reinterpret_cast<T*>(smem + L::root_val);
+    int2* root_item = reinterpret_cast<int2*>(smem + L::root_item);
+    int2* items = reinterpret_cast<int2*>(smem + L::items);
+    int2* surv = reinterpret_cast<int2*>(smem + L::surv);
+    unsigned short* clist = reinterpret_cast<unsigned short*>(smem + L::clist);
+    unsigned short* cpos = reinterpret_cast<unsigned short*>(smem + L::pos);
+    unsigned char* ccls = smem + L::cls;
+    int* ints = reinterpret_cast<int*>(smem + L::ints);
+    WsHeader* hdr = A.hdr;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned FULL = 0xffffffffu;
     const unsigned lt = (1u << lane) - 1u;
-    const int n = min(*(volatile int*)(STAGED ? &hdr->live_count : &hdr->cand_count), cand_cap);
-    int head = 0, queued = 0;           // ring queue of sub-tests (block-uniform)
-    int masked = 0;                     // this thread's sub-tests before repeats are shared
-    // class counts and root count of a batch, two sets used by alternate batches: a batch
-    // clears the other set at its end, when every read of that set is two barriers back
-    // (the staging barriers order the initial clearing before the first batch)
-    int par = 0, cpar = 0;
-    if (tid < 8) ints[CI_COUNT + tid] = 0;
-    if (tid < 4) ints[CI_ROOTS + tid] = 0;
-    if (tid < 2) ints[CI_LIVE + tid] = 0;
-    __syncthreads();
-    for (long long base = (long long)blockIdx.x * CCD_BLOCK;; base += (long long)gridDim.x * CCD_BLOCK) {
-        const bool more = base < n;
-        if (!more && queued == 0) break;
-        if (more) {
-            int2 pr = make_int2(0, 0);
-            uint32_t bits = 0;
-            unsigned shared_bits = 0;
-            if constexpr (STAGED) {
-                // the resident engine's pairs come staged by k_ccd_stage_*: the pairs with
-                // sub-tests to solve, which ones, and which of them stand for their repeats
-                const long long c = base + tid;
-                if (c < n) {
-                    const int4 rec = W.live[c];
-                    pr = make_int2(rec.x, rec.y);
-                    bits = (unsigned)rec.z & 0x7fffu;
-                    shared_bits = ((unsigned)rec.z >> 15) & 0x7fffu;
-                }
-            } else {
-                // about half of the candidate pairs are mesh neighbours that share a vertex:
-                // the chunk's other pairs are gathered first (block-wide), so that the 15
-                // swept sub-box tests run on full warps
-                long long c = base + tid;
-                bool live = false;
-                if (c < n) {
-                    pr = cand[c];
-                    live = !ccd_pair_shares_vertex<T>(x0, pr.x, pr.y) &&
-                           (SRC != SRC_EXACT || ccd_pair_leaf_overlap<T>(x0, x1, pr.x, pr.y));
-                }
-                const unsigned lb = __ballot_sync(FULL, live);
-                int lbase = 0;
-                if (lane == 0 && lb) lbase = atomicAdd(&ints[CI_LIVE + cpar], __popc(lb));
-                lbase = __shfl_sync(FULL, lbase, 0);
-                if (live) spairs[lbase + __popc(lb & lt)] = pr;
-                __syncthreads();
-                const int nlive = ints[CI_LIVE + cpar];
-                // the other chunk parity's counter was last read before the barrier above
-                if (tid == 0) ints[CI_LIVE + (cpar ^ 1)] = 0;
-                cpar ^= 1;
-                pr = make_int2(0, 0);
-                if (tid < nlive) {
-                    pr = spairs[tid];
-                    bits = ccd_pair_subbox_mask<T, MODE != CCD_MINCOL>(x0, x1, pr.x, pr.y);
-                }
-                if (MODE != CCD_MINCOL) masked += __popc(bits);
-                if (MODE == CCD_MINCOL) {
-                    while (bits) {
-                        int k = __ffs(bits) - 1;
-                        bits &= bits - 1;
-                        OutRegion R = out_region(F, M, pr.x, max_per_tri);
-                        long long r = append_row(mesh_counters, F, R.m, R.cap, &hdr->status);
-                        if (r >= 0) {
-                            long long o = (long long)R.po * max_per_tri + r;
-                            rows[o * 3 + 0] = pr.x - R.po;
-                            rows[o * 3 + 1] = pr.y - R.po;
-                            rows[o * 3 + 2] = k;
-                        }
-                    }
-                    // the next chunk reuses spairs and the other live counter
-                    __syncthreads();
-                    continue;
+    const int n = min(*(volatile int*)(SRC == SRC_STAGED ? &hdr->live_count : &hdr->cand_count), A.cand_cap);
+    // queue fills and positions (block-uniform)
+    int ihead = 0, iq = 0;              // sub-tests: ring of ITEMS
+    unsigned staken = 0;                // survivors: ring of SURV, taken so far (queued: ints[CI_SURV])
+    int sq = 0;
+    int nee = 0, nvf = 0;               // roots: edge-edge at [0, nee), vertex-face at [ROOTS - nvf, ROOTS)
+    int par = 0;                        // the class counts' set
+    int solved = 0, filtered = 0;       // totals of this block
+    bool pend = false;                  // sub-tests of the current pairs that found no room yet
+    int2 pr = make_int2(0, 0);
+    unsigned bits = 0u, shared_bits = 0u;
+    if (tid < 64) ints[tid] = 0;
+    // pairs of an intake: a whole block's, or fewer when the grid would not have work for every
+    // block (a small call's blocks then end after one batch)
+    const int per = min(CCD_BLOCK, max(16, (int)((n + (long long)gridDim.x - 1) / gridDim.x)));
+    long long base = (long long)blockIdx.x * per;
+
+    // a record of a passing root, past the block's buffer: to the list, or in place
+    auto put = [&](int4 rec, int at) {
+        if (at < A.W.expand_cap) A.W.expand[at] = rec;
+        else record_in_place<T, MODE, Sink, LIB>(&A, &sink, rec);
+    };
+    // the buffered records (block-wide; between barriers)
+    auto flush = [&]() {
+        const int cnt = min(ints[CI_OUT], L::OUT);
+        if (MODE == CCD_ROWS && SRC == SRC_PACKED) {
+            // the rows themselves, one a record
+            for (int i = tid; i < cnt; i += CCD_BLOCK) {
+                const int4 rec = out[i];
+                const int qx = rec.x & SLOT_MASK, qy = rec.y & SLOT_MASK;
+                const OutRegion R = out_region(A.F, forest_size(A.F), qx, A.max_per_tri);
+                const long long r = append_row(A.mesh_counters, A.F, R.m, R.cap, &hdr->status);
+                if (r >= 0) {
+                    const long long o = (long long)R.po * A.max_per_tri + r;
+                    A.rows[o * 3 + 0] = qx - R.po;
+                    A.rows[o * 3 + 1] = qy - R.po;
+                    A.rows[o * 3 + 2] = (rec.y >> 28) & 15;
+                    A.times[o] = (T)__hiloint2double(rec.w, rec.z);
                 }
             }
-            // append the chunk's sub-tests (block-wide exclusive scan of the counts)
+        } else {
+            if (tid == 0) ints[CI_BASE] = atomicAdd(&hdr->expand_count, cnt);
+            __syncthreads();
+            const int b0 = ints[CI_BASE];
+            for (int i = tid; i < cnt; i += CCD_BLOCK) put(out[i], b0 + i);
+        }
+        __syncthreads();
+        if (tid == 0) ints[CI_OUT] = 0;
+    };
+
+    __syncthreads();
+    while (true) {
+        // ---- sub-tests of the next pairs, until there is a batch of them
+        while (iq < NB && (pend || base < n)) {
+            if (!pend) {
+                const long long c = base + tid;
+                base += (long long)gridDim.x * per;
+                bits = shared_bits = 0u;
+                if (tid < per && c < n) {
+                    if (SRC == SRC_STAGED) {
+                        const int4 rec = A.W.live[c];
+                        pr = make_int2(rec.x, rec.y);
+                        bits = (unsigned)rec.z & 0x7fffu;
+                        shared_bits = ((unsigned)rec.z >> 15) & 0x7fffu;
+                    } else {
+                        pr = A.cand[c];
+                        if (A.masks) {
+                            bits = A.masks[c];
+                        } else {
+                            bits = ((unsigned)pr.x >> PACK_BITS) | (((unsigned)pr.y >> PACK_BITS) << 8);
+                            pr.x &= PACK_MASK;
+                            pr.y &= PACK_MASK;
+                        }
+                    }
+                }
+            }
+            // (block-wide exclusive scan of the counts)
             const int cnt = __popc(bits);
             const int incl = warp_inclusive_scan(cnt, lane);
             if (lane == 31) ints[CI_WARP + warp] = incl;
             __syncthreads();
             if (warp == 0) {
-                int v = lane < NW ? ints[CI_WARP + lane] : 0;
-                int sc = warp_inclusive_scan(v, lane);
+                const int v = lane < NW ? ints[CI_WARP + lane] : 0;
+                const int sc = warp_inclusive_scan(v, lane);
                 if (lane < NW) ints[CI_WARP + lane] = sc - v;
                 if (lane == 31) ints[CI_TOTAL] = sc;
             }
             __syncthreads();
-            int pos = head + queued + ints[CI_WARP + warp] + incl - cnt;
-            const int total = ints[CI_TOTAL];
-            while (bits) {
-                int k = __ffs(bits) - 1;
+            const int room = L::ITEMS - iq, total = ints[CI_TOTAL];
+            int at = ints[CI_WARP + warp] + incl - cnt;
+            while (bits && at < room) {
+                const int k = __ffs(bits) - 1;
                 bits &= bits - 1;
-                items[pos % Q] = pack_subtest(pr.x, pr.y, k, (shared_bits >> k) & 1u);
-                ++pos;
+                items[(ihead + iq + at) % L::ITEMS] = pack_subtest(pr.x, pr.y, k, (shared_bits >> k) & 1u);
+                ++at;
             }
-            if (tid == 0 && total) atomicAdd(&hdr->solved, total);
-            queued += total;
+            pend = total > room;
+            iq += min(total, room);
             __syncthreads();
         }
-        // solve full batches (and, after the last chunk, the remainder)
-        while (queued >= NB || (!more && queued > 0)) {
-            const int nb = min(NB, queued);
-            // (1) coefficients and solver prefix; each sub-test takes its place in its class
-            for (int ri = tid; ri < nb; ri += CCD_BLOCK) {
-                int2 it = items[(head + ri) % Q];
-                int k = (it.y >> 28) & 15;
-                MTet<T> tet = load_tet(x0, x1, it.x & SLOT_MASK, it.y & SLOT_MASK, k);
-                T cf[4];
-                cubic_coeffs(tet, cf);
-                rec[0 * NB + ri] = (double)cf[0];
-                rec[1 * NB + ri] = (double)cf[1];
-                rec[2 * NB + ri] = (double)cf[2];
-                rec[3 * NB + ri] = (double)cf[3];
-                double g, h;
-                int cls = cubic_prefix<LIB>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3], g, h);
-                rec[4 * NB + ri] = g;
-                rec[5 * NB + ri] = h;
-                rec_cls[ri] = (unsigned char)cls;
-                if (cls != CUBIC_NONE) rec_pos[ri] = (unsigned short)atomicAdd(&ints[CI_COUNT + 4 * par + cls - 1], 1);
+        const bool drained = !pend && base >= n;         // (block-uniform: base is)
+        // ---- (1) coefficients
+        if (iq > 0) {
+            const int nb = min(NB, iq);
+            for (int r0 = 0; r0 < nb; r0 += CCD_BLOCK) {
+                const int ri = r0 + tid;
+                bool go = false;
+                int2 it = make_int2(0, 0);
+                T cf[4] = {T(0), T(0), T(0), T(0)};
+                if (ri < nb) {
+                    it = items[(ihead + ri) % L::ITEMS];
+                    const MTet<T> tet = load_tet(A.x0, A.x1, it.x & SLOT_MASK, it.y & SLOT_MASK, (it.y >> 28) & 15);
+                    cubic_coeffs(tet, cf);
+                    go = !(cf[0] == 0 && cf[1] == 0) &&          // (the linear case has no root that is kept)
+                         !cubic_misses<T>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]);
+                }
+                const unsigned m = __ballot_sync(FULL, go);
+                unsigned b0 = 0;
+                if (lane == 0 && m) b0 = (unsigned)atomicAdd(&ints[CI_SURV], __popc(m));
+                b0 = __shfl_sync(FULL, b0, 0) + __popc(m & lt);
+                if (go) {
+                    const unsigned slot = b0 % L::SURV;
+                    surv[slot] = it;
+                    coef[0 * L::SURV + slot] = (double)cf[0];
+                    coef[1 * L::SURV + slot] = (double)cf[1];
+                    coef[2 * L::SURV + slot] = (double)cf[2];
+                    coef[3 * L::SURV + slot] = (double)cf[3];
+                }
+            }
+            solved += nb;
+            ihead = (ihead + nb) % L::ITEMS;
+            iq -= nb;
+            __syncthreads();
+            sq = (int)((unsigned)ints[CI_SURV] - staken);
+        }
+        // ---- (2) solver prefix and roots
+        if (sq >= NB || (drained && iq == 0 && sq > 0)) {
+            const int nb = min(NB, sq);
+            for (int r0 = 0; r0 < nb; r0 += CCD_BLOCK) {
+                const int ri = r0 + tid;
+                int cls = CUBIC_NONE;
+                if (ri < nb) {
+                    const unsigned slot = (staken + ri) % L::SURV;
+                    double g, h;
+                    cls = cubic_prefix<LIB>(coef[0 * L::SURV + slot], coef[1 * L::SURV + slot],
+                                            coef[2 * L::SURV + slot], coef[3 * L::SURV + slot], g, h);
+                    gh[ri] = g;
+                    gh[NB + ri] = h;
+                    ccls[ri] = (unsigned char)cls;
+                }
+                // its place in its class, one atomic a warp and class
+#pragma unroll
+                for (int c = CUBIC_QUAD; c <= CUBIC_ONE; ++c) {
+                    const unsigned m = __ballot_sync(FULL, cls == c);
+                    if (!m) continue;
+                    int b0 = 0;
+                    if (lane == 0) b0 = atomicAdd(&ints[CI_COUNT + 4 * par + c - 1], __popc(m));
+                    b0 = __shfl_sync(FULL, b0, 0) + __popc(m & lt);
+                    if (cls == c) cpos[ri] = (unsigned short)b0;
+                }
             }
             __syncthreads();
-            // sub-tests ordered by class (every thread forms the class offsets itself)
+            // ordered by class (every thread forms the class offsets itself)
             const int* counts = ints + CI_COUNT + 4 * par;
             const int o1 = counts[0];
             const int o2 = o1 + counts[1];
             const int o3 = o2 + counts[2];
             const int nsolve = o3 + counts[3];
             for (int ri = tid; ri < nb; ri += CCD_BLOCK) {
-                int cls = rec_cls[ri];
+                const int cls = ccls[ri];
                 if (cls != CUBIC_NONE) {
-                    int off = cls == 1 ? 0 : (cls == 2 ? o1 : (cls == 3 ? o2 : o3));
-                    clist[off + rec_pos[ri]] = (unsigned short)ri;
-                }
-            }
-            __syncthreads();
-            // (2) roots; the ones in [0, 1] go to the root list, edge-edge roots from its
-            // front and vertex-face roots from its back
-            for (int j0 = 0; j0 < nsolve; j0 += CCD_BLOCK) {
-                const int j = j0 + tid;
-                T rr[3] = {(T)-1, (T)-1, (T)-1};
-                int ri = 0;
-                bool ee = false;
-                if (j < nsolve) {
-                    ri = clist[j];
-                    ee = ((items[(head + ri) % Q].y >> 28) & 15) < 9;
-                    int cc = (j >= o1) + (j >= o2) + (j >= o3);
-                    class_roots<T, LIB>(cc + 1, rec[0 * NB + ri], rec[1 * NB + ri], rec[2 * NB + ri],
-                                        rec[3 * NB + ri], rec[4 * NB + ri], rec[5 * NB + ri], rr);
-                }
-#pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    bool keep = j < nsolve && (rr[s] >= 0 && rr[s] <= 1);
-                    unsigned me = __ballot_sync(FULL, keep && ee);
-                    unsigned mf = __ballot_sync(FULL, keep && !ee);
-                    int ae = 0, af = 0;
-                    if (lane == 0 && me) ae = atomicAdd(&ints[CI_ROOTS + 2 * par], __popc(me));
-                    if (lane == 0 && mf) af = atomicAdd(&ints[CI_ROOTS + 2 * par + 1], __popc(mf));
-                    ae = __shfl_sync(FULL, ae, 0) + __popc(me & lt);
-                    af = __shfl_sync(FULL, af, 0) + __popc(mf & lt);
-                    if (keep) {
-                        const int at = ee ? ae : 3 * NB - 1 - af;
-                        root_rec[at] = (unsigned short)ri;
-                        root_val[at] = rr[s];
-                    }
-                }
-            }
-            __syncthreads();
-            const int nee = ints[CI_ROOTS + 2 * par];
-            const int nroots = nee + ints[CI_ROOTS + 2 * par + 1];
-            if (tid == 0 && nroots) atomicAdd(&hdr->roots, nroots);
-            // (3) filter and output
-            if (MODE == CCD_ROWS) {
-                // about one root in twelve passes the filter: those are buffered per warp and
-                // their rows written 32 at a time, so that the mesh lookup and the row append
-                // run on full warps rather than on the few lanes that passed
-                unsigned short* pb = pbuf + warp * 64;
-                int np = 0;                        // buffered roots of this warp (warp-uniform)
-                // (mask: the lanes that call it together)
-                auto emit = [&](int j, unsigned mask) {
-                    const int2 it = items[(head + root_rec[j]) % Q];
-                    const int qx = it.x & SLOT_MASK, qy = it.y & SLOT_MASK, k = (it.y >> 28) & 15;
-                    const T tv = root_val[j];
-                    // every pair of a shared sub-test is in the mesh of (qx, qy)
-                    const OutRegion R = out_region(F, M, qx, max_per_tri);
-                    auto row = [&](int a, int b, int kk) {
-                        long long r = append_row(mesh_counters, F, R.m, R.cap, &hdr->status);
-                        if (r >= 0) {
-                            long long o = (long long)R.po * max_per_tri + r;
-                            rows[o * 3 + 0] = a - R.po;
-                            rows[o * 3 + 1] = b - R.po;
-                            rows[o * 3 + 2] = kk;
-                            times[o] = tv;
-                        }
-                    };
-                    if constexpr (STAGED) {
-                        // each passing root leaves a record for k_ccd_expand, which writes its
-                        // rows (every pair's, for a shared sub-test); the roots that do not
-                        // fit in the record list are written here
-                        unsigned rest = mask;
-                        if (W.expand) {
-                            const int leader = __ffs(mask) - 1;
-                            int b0 = 0;
-                            if (lane == leader) b0 = atomicAdd(&hdr->expand_count, __popc(mask));
-                            b0 = __shfl_sync(mask, b0, leader) + __popc(mask & lt);
-                            const bool fits = b0 < W.expand_cap;
-                            rest = __ballot_sync(mask, !fits);
-                            if (fits) {
-                                const double tw = (double)tv;
-                                W.expand[b0] = make_int4(it.x, it.y, __double2loint(tw), __double2hiint(tw));
-                                return;
-                            }
-                        }
-                        int ma[WELD_FANCAP], mb[WELD_FANCAP], mk[WELD_FANCAP];
-                        const int nm = weld_list(W, qx, qy, k, (it.x >> 28) & 1, ma, mb, mk);
-                        // the rows of all the lanes in one mesh are reserved with one atomic
-                        const int base = reserve_rows(mesh_counters, F, R.m, nm, rest);
-                        for (int i = 0; i < nm; ++i) {
-                            const long long r = (long long)base + i;
-                            if (r >= R.cap) {
-                                atomicOr(&hdr->status, ST_OUT_OVERFLOW);
-                                break;
-                            }
-                            const long long o = (long long)R.po * max_per_tri + r;
-                            rows[o * 3 + 0] = ma[i] - R.po;
-                            rows[o * 3 + 1] = mb[i] - R.po;
-                            rows[o * 3 + 2] = mk[i];
-                            times[o] = tv;
-                        }
-                    } else {
-                        row(qx, qy, k);
-                    }
-                };
-                for (int b0 = warp * 32; b0 < nroots; b0 += CCD_BLOCK) {
-                    const int jj = b0 + lane;
-                    int j = 0;
-                    bool pass = false;
-                    if (jj < nroots) {
-                        j = jj < nee ? jj : 3 * NB - 1 - (jj - nee);
-                        const int2 it = items[(head + root_rec[j]) % Q];
-                        const int k = (it.y >> 28) & 15;
-                        MTet<T> tet = load_tet(x0, x1, it.x & SLOT_MASK, it.y & SLOT_MASK, k);
-                        pass = ccd_filter(tet, k, root_val[j]);
-                    }
-                    const unsigned pm = __ballot_sync(FULL, pass);
-                    if (pass) pb[np + __popc(pm & lt)] = (unsigned short)j;
-                    np += __popc(pm);
-                    if (np >= 32) {
-                        __syncwarp();
-                        emit(pb[lane], FULL);
-                        __syncwarp();
-                        if (lane < np - 32) pb[lane] = pb[32 + lane];
-                        __syncwarp();
-                        np -= 32;
-                    }
-                }
-                __syncwarp();
-                if (lane < np) emit(pb[lane], (1u << np) - 1u);     // (np < 32 here)
-            } else {
-                for (int jj = tid; jj < nroots; jj += CCD_BLOCK) {
-                    const int j = jj < nee ? jj : 3 * NB - 1 - (jj - nee);
-                    int2 it = items[(head + root_rec[j]) % Q];
-                    int k = (it.y >> 28) & 15;
-                    int2 q = make_int2(it.x & SLOT_MASK, it.y & SLOT_MASK);
-                    T root = root_val[j];
-                    MTet<T> tet = load_tet(x0, x1, q.x, q.y, k);
-                    if (!ccd_filter(tet, k, root)) continue;
-                    // the contact of every pair with this sub-test (its own corner masses)
-                    int ma[STAGED ? WELD_FANCAP : 1], mb[STAGED ? WELD_FANCAP : 1], mk[STAGED ? WELD_FANCAP : 1];
-                    int nm = 1;
-                    if constexpr (STAGED) nm = weld_list(W, q.x, q.y, k, (it.x >> 28) & 1, ma, mb, mk);
-                    else {
-                        ma[0] = q.x;
-                        mb[0] = q.y;
-                        mk[0] = k;
-                    }
-                    for (int i = 0; i < nm; ++i) {
-                        const int a = ma[i], b = mb[i], kk = mk[i];
-                        T mq[4];
-#pragma unroll
-                        for (int pt = 0; pt < 4; ++pt)
-                            mq[pt] = sink.masses[(long long)(tet_side(kk, pt) ? b : a) * 3 + tet_corner(kk, pt)];
-                        Contact<T> ct = contact<T, LIB>(tet, kk, root, mq);
-                        sink.add(tet, a, b, kk, root, ct, F, M, &hdr->status);
-                    }
+                    const int off = cls == 1 ? 0 : (cls == 2 ? o1 : (cls == 3 ? o2 : o3));
+                    clist[off + cpos[ri]] = (unsigned short)ri;
                 }
             }
             if (tid < 4) ints[CI_COUNT + 4 * (par ^ 1) + tid] = 0;
-            if (tid >= 4 && tid < 6) ints[CI_ROOTS + 2 * (par ^ 1) + tid - 4] = 0;
-            par ^= 1;
-            head = (head + nb) % Q;
-            queued -= nb;
             __syncthreads();
+            for (int j0 = 0; j0 < nsolve; j0 += CCD_BLOCK) {
+                const int j = j0 + tid;
+                T rr[3] = {(T)-1, (T)-1, (T)-1};
+                int2 it = make_int2(0, 0);
+                if (j < nsolve) {
+                    const int ri = clist[j];
+                    const unsigned slot = (staken + ri) % L::SURV;
+                    it = surv[slot];
+                    const int cc = (j >= o1) + (j >= o2) + (j >= o3);
+                    class_roots<T, LIB>(cc + 1, coef[0 * L::SURV + slot], coef[1 * L::SURV + slot],
+                                        coef[2 * L::SURV + slot], coef[3 * L::SURV + slot], gh[ri], gh[NB + ri], rr);
+                }
+                // (places of the three roots of every lane: one atomic a warp and kind)
+                const bool ee = ((it.y >> 28) & 15) < 9;
+                const unsigned mee = __ballot_sync(FULL, ee);
+                unsigned keep[3];
+#pragma unroll
+                for (int s = 0; s < 3; ++s)
+                    keep[s] = __ballot_sync(FULL, j < nsolve && (rr[s] >= 0 && rr[s] <= 1));
+                int ae = 0, af = 0;
+                const int ce = __popc(keep[0] & mee) + __popc(keep[1] & mee) + __popc(keep[2] & mee);
+                const int ca = __popc(keep[0]) + __popc(keep[1]) + __popc(keep[2]);
+                if (lane == 0 && ce) ae = atomicAdd(&ints[CI_EE], ce);
+                if (lane == 0 && ca > ce) af = atomicAdd(&ints[CI_VF], ca - ce);
+                ae = __shfl_sync(FULL, ae, 0);
+                af = __shfl_sync(FULL, af, 0);
+#pragma unroll
+                for (int s = 0; s < 3; ++s) {
+                    const unsigned mine = keep[s] & (ee ? mee : ~mee);
+                    if ((keep[s] >> lane) & 1u) {
+                        const int before = __popc(mine & lt);
+                        const int at = ee ? ae + before : L::ROOTS - 1 - af - before;
+                        root_item[at] = it;
+                        root_val[at] = rr[s];
+                    }
+                    ae += __popc(keep[s] & mee);
+                    af += __popc(keep[s] & ~mee);
+                }
+            }
+            par ^= 1;
+            staken += nb;
+            sq -= nb;
+            __syncthreads();
+            nee = ints[CI_EE];
+            nvf = ints[CI_VF];
         }
+        // ---- (3) filter: whole rounds of full warps, or all that is left at the end
+        const bool last = drained && iq == 0 && sq == 0;
+        int we = nee >> 5, wv = nvf >> 5;
+        if (last) {
+            we = (nee + 31) >> 5;
+            wv = (nvf + 31) >> 5;
+        } else {
+            const int w8 = (we + wv) / NW * NW;
+            we = min(we, w8);
+            wv = w8 - we;
+        }
+        if (we + wv > 0) {
+            // (units are taken from the ends of the lists, so nothing moves)
+            for (int u = warp; u < we + wv; u += NW) {
+                const bool ee = u < we;
+                const int at = ee ? nee - 1 - 32 * u - lane : L::ROOTS - nvf + 32 * (u - we) + lane;
+                const bool valid = ee ? at >= 0 : at < L::ROOTS;
+                bool pass = false;
+                int4 rec = make_int4(0, 0, 0, 0);
+                if (valid) {
+                    const int2 it = root_item[at];
+                    const T root = root_val[at];
+                    const int k = (it.y >> 28) & 15;
+                    const MTet<T> tet = load_tet(A.x0, A.x1, it.x & SLOT_MASK, it.y & SLOT_MASK, k);
+                    pass = ccd_filter(tet, k, root);
+                    const double tw = (double)root;
+                    rec = make_int4(it.x, it.y, __double2loint(tw), __double2hiint(tw));
+                }
+                const unsigned pm = __ballot_sync(FULL, pass);
+                int b0 = 0;
+                if (lane == 0 && pm) b0 = atomicAdd(&ints[CI_OUT], __popc(pm));
+                b0 = __shfl_sync(FULL, b0, 0) + __popc(pm & lt);
+                if (pass) {
+                    if (b0 < L::OUT) out[b0] = rec;
+                    else if (MODE == CCD_ROWS && SRC == SRC_PACKED) record_in_place<T, MODE, Sink, LIB>(&A, &sink, rec);
+                    else put(rec, atomicAdd(&hdr->expand_count, 1));
+                }
+            }
+            filtered += last ? nee + nvf : 32 * (we + wv);
+            nee = max(nee - 32 * we, 0);
+            nvf = max(nvf - 32 * wv, 0);
+            __syncthreads();
+            if (tid == 0) {
+                ints[CI_EE] = nee;
+                ints[CI_VF] = nvf;
+            }
+            if (last || ints[CI_OUT] >= L::OUT / 2) flush();
+        } else if (last && ints[CI_OUT] > 0) {
+            flush();
+        }
+        if (last) break;
+        __syncthreads();
     }
-    // (the loop ends for the whole block at once)
-    if (MODE != CCD_MINCOL) {
-        const int ws = __reduce_add_sync(FULL, masked);
-        if (lane == 0 && ws) atomicAdd(&hdr->subtests, ws);
+    if (tid == 0) {
+        if (solved) atomicAdd(&hdr->solved, solved);
+        if (filtered) atomicAdd(&hdr->roots, filtered);
     }
 }
 
@@ -1327,16 +1462,33 @@ template <class T, int MODE, class Sink, int LIB, int SRC, int BM> cudaError_t p
 }
 
 template <class T, int MODE, class Sink, int LIB, int SRC, int BM>
-cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const int2* cand, int cand_cap, WsHeader* hdr, const T* x0,
-                              const T* x1, Forest F, long long* rows, T* times, int max_per_tri, int* mesh_counters,
-                              Weld W, Sink sink) {
+cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink) {
     cudaError_t e = prepare_ccd_narrow<T, MODE, Sink, LIB, SRC, BM>();
     if (e != cudaSuccess) return e;
-    k_ccd_narrow<T, MODE, Sink, LIB, SRC, BM><<<grid, CCD_BLOCK, CcdLayout<T, BM * CCD_BLOCK>::bytes, s>>>(
-        cand, cand_cap, hdr, x0, x1, F, rows, times, max_per_tri, mesh_counters, W, sink);
+    k_ccd_narrow<T, MODE, Sink, LIB, SRC, BM><<<grid, CCD_BLOCK, CcdLayout<T, BM * CCD_BLOCK>::bytes, s>>>(A, sink);
     return cudaSuccess;
 }
 
+// The contacts of the roots that passed the filter in k_ccd_narrow, one record a thread: the
+// contact's registers and code stay out of the narrow kernel, and its lanes are full.  523 k
+// contacts take 82 us (fp64; their tetrahedra's gathers and 28 atomics each).
+static constexpr int CONTACT_THREADS = 128;
+template <class T, class Sink, int LIB>
+__global__ void __launch_bounds__(CONTACT_THREADS)
+k_ccd_contacts(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink sink) {
+    const int n = min(*(volatile int*)&A.hdr->expand_count, A.W.expand_cap);
+    for (int c = blockIdx.x * CONTACT_THREADS + threadIdx.x; c < n; c += gridDim.x * CONTACT_THREADS) {
+        const int4 rec = A.W.expand[c];
+        contact_of_root<T, Sink, LIB>(A, sink, rec.x & SLOT_MASK, rec.y & SLOT_MASK, (rec.y >> 28) & 15,
+                                      (T)__hiloint2double(rec.w, rec.z));
+    }
+}
+
+template <class T, class Sink, int LIB>
+cudaError_t launch_ccd_contacts(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink) {
+    k_ccd_contacts<T, Sink, LIB><<<grid, CONTACT_THREADS, 0, s>>>(A, sink);
+    return cudaSuccess;
+}
 #endif  // CCC_NARROW_TU
 
 // The rows of the roots that passed the filter in k_ccd_narrow (its records in Weld.expand),

@@ -18,29 +18,39 @@
 
 namespace ccc {
 
-// the combinations the library launches: (type, mode, sink, math library)
-#define CCC_NARROW_INSTANCE(T, MODE, SINK, LIB, SRC, BM)                                                         \
-    template cudaError_t launch_ccd_narrow<T, MODE, SINK, LIB, SRC, BM>(int, cudaStream_t, const int2*, int,        \
-                                                                           WsHeader*, const T*, const T*, Forest,      \
-                                                                           long long*, T*, int, int*, Weld, SINK);     \
+// the combinations the library launches: (type, mode, sink, math library, source, batch)
+#define CCC_NARROW_INSTANCE(T, MODE, SINK, LIB, SRC, BM)                                                           \
+    template cudaError_t launch_ccd_narrow<T, MODE, SINK, LIB, SRC, BM>(int, cudaStream_t, const CcdArgs<T>&,        \
+                                                                           const SINK&);                              \
     template cudaError_t prepare_ccd_narrow<T, MODE, SINK, LIB, SRC, BM>();
-#define CCC_NARROW_TYPES(MODE, SINK, LIB, SRC, BM)                                                              \
-    CCC_NARROW_INSTANCE(float, MODE, SINK<float>, LIB, SRC, BM)                                                  \
-    CCC_NARROW_INSTANCE(double, MODE, SINK<double>, LIB, SRC, BM)
-// the reference-format operations (pairs from the candidate buffer), batches of 256
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_REFERENCE, SRC_CANDIDATES, 1)
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_PORTABLE, SRC_CANDIDATES, 1)
-CCC_NARROW_TYPES(CCD_IMPULSES, CornerSink, LIB_REFERENCE, SRC_CANDIDATES, 1)
-CCC_NARROW_TYPES(CCD_IMPULSES, CornerSink, LIB_PORTABLE, SRC_CANDIDATES, 1)
-CCC_NARROW_TYPES(CCD_MINCOL, CornerSink, LIB_PORTABLE, SRC_CANDIDATES, 1)
-// the resident engine's collision step (staged pairs, shared sub-tests), batches of 256 or
-// 512, and its impulse loop (candidate buffer, the exact leaf-box test)
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_REFERENCE, SRC_STAGED, 1)
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_PORTABLE, SRC_STAGED, 1)
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_REFERENCE, SRC_STAGED, 2)
-CCC_NARROW_TYPES(CCD_ROWS, CornerSink, LIB_PORTABLE, SRC_STAGED, 2)
-CCC_NARROW_TYPES(CCD_IMPULSES, LoopSink, LIB_REFERENCE, SRC_EXACT, 1)
-CCC_NARROW_TYPES(CCD_IMPULSES, LoopSink, LIB_PORTABLE, SRC_EXACT, 1)
+#define CCC_NARROW_TYPES(MODE, SINK, SRC, BM)                                                                      \
+    CCC_NARROW_INSTANCE(float, MODE, SINK<float>, LIB_REFERENCE, SRC, BM)                                           \
+    CCC_NARROW_INSTANCE(double, MODE, SINK<double>, LIB_REFERENCE, SRC, BM)                                         \
+    CCC_NARROW_INSTANCE(float, MODE, SINK<float>, LIB_PORTABLE, SRC, BM)                                            \
+    CCC_NARROW_INSTANCE(double, MODE, SINK<double>, LIB_PORTABLE, SRC, BM)
+#define CCC_CONTACT_TYPES(SINK)                                                                                    \
+    template cudaError_t launch_ccd_contacts<float, SINK<float>, LIB_REFERENCE>(int, cudaStream_t,                  \
+                                                                                   const CcdArgs<float>&,            \
+                                                                                   const SINK<float>&);               \
+    template cudaError_t launch_ccd_contacts<double, SINK<double>, LIB_REFERENCE>(int, cudaStream_t,                \
+                                                                                     const CcdArgs<double>&,         \
+                                                                                     const SINK<double>&);            \
+    template cudaError_t launch_ccd_contacts<float, SINK<float>, LIB_PORTABLE>(int, cudaStream_t,                   \
+                                                                                  const CcdArgs<float>&,             \
+                                                                                  const SINK<float>&);                \
+    template cudaError_t launch_ccd_contacts<double, SINK<double>, LIB_PORTABLE>(int, cudaStream_t,                 \
+                                                                                    const CcdArgs<double>&,          \
+                                                                                    const SINK<double>&);
+// the reference-format operations (pairs and masks from the candidate buffer), batches of 256
+CCC_NARROW_TYPES(CCD_ROWS, CornerSink, SRC_PACKED, 1)
+CCC_NARROW_TYPES(CCD_IMPULSES, CornerSink, SRC_PACKED, 1)
+CCC_CONTACT_TYPES(CornerSink)
+// the resident engine's collision step (shared sub-tests), batches of 256 or 512, and its
+// impulse loop
+CCC_NARROW_TYPES(CCD_ROWS, CornerSink, SRC_STAGED, 1)
+CCC_NARROW_TYPES(CCD_ROWS, CornerSink, SRC_STAGED, 2)
+CCC_NARROW_TYPES(CCD_IMPULSES, LoopSink, SRC_STAGED, 1)
+CCC_CONTACT_TYPES(LoopSink)
 
 // Element-wise evaluation of the solver's arithmetic building blocks, for tests that compare
 // them bit for bit with the CPU oracle and against CUDA's own elementary functions.

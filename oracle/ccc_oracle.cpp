@@ -1015,7 +1015,8 @@ ORC_API int orc_ddmul_check(int64_t n, uint64_t seed, int family, int64_t* out) 
         if (!same(ccc_certmul_k<2>(sq.hi, sq.lo, z).hi, ccc_certmul2_hi(sq.hi, sq.lo, z))) ++bad;
         ccc_dd pr = ccc_certmul_k<1>(y, 0.0, z);
         if (!same(ccc_certmul_k<2>(pr.hi, pr.lo, x).hi, ccc_certmul2_hi(pr.hi, pr.lo, x))) ++bad;
-        if (!same(ccc_cube_hi(x), ccc_certmul_k<2>(sq.hi, sq.lo, x).hi)) ++bad;
+        const ccc_powers pw = ccc_square_and_cube(x);
+        if (!same(pw.cube, ccc_certmul_k<2>(sq.hi, sq.lo, x).hi) || !same(pw.sq, sq.hi) || !same(pw.sq_lo, sq.lo)) ++bad;
     }
     out[0] = bad;
     out[1] = fast;
