@@ -286,67 +286,106 @@ __device__ __forceinline__ bool ccd_pair_shares_vertex(const T* __restrict__ x0,
     return eq != 0u;
 }
 
+// Whether the pair's leaf boxes (each triangle's boxes at x0 and x1 merged,
+// MergeTriBoundingBoxes, build_bvh.cu:452-460) overlap (checkOverlap, aabb.cu:107-111), one
+// axis at a time; fmin / fmax skip NaN and the comparisons do not tell -0 from +0, so the
+// order of the reductions does not change the answer.
+template <class T>
+__device__ __forceinline__ bool ccd_pair_leaf_overlap(const T* __restrict__ x0, const T* __restrict__ x1, long long i,
+                                                      long long j) {
+    bool ov = true;
+#pragma unroll 1
+    for (int ax = 0; ax < 3; ++ax) {
+        T la = __ldg(x0 + i * 9 + ax), ha = la, lb = __ldg(x0 + j * 9 + ax), hb = lb;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const T a0 = __ldg(x0 + i * 9 + 3 * c + ax), a1 = __ldg(x1 + i * 9 + 3 * c + ax);
+            const T b0 = __ldg(x0 + j * 9 + 3 * c + ax), b1 = __ldg(x1 + j * 9 + 3 * c + ax);
+            la = fmn(la, fmn(a0, a1));
+            ha = fmx(ha, fmx(a0, a1));
+            lb = fmn(lb, fmn(b0, b1));
+            hb = fmx(hb, fmx(b0, b1));
+        }
+        ov = ov && la <= hb && ha >= lb;
+    }
+    return ov;
+}
+
+// The smaller (larger) of two values, neither of them NaN.  A double's fmin is some six
+// instructions for the sake of NaN, a select three (the 64-mesh step's k_ccd_stage_mask 2,206 ->
+// 1,930 us, the fold's k_ccd_mask 109 -> 98 us); a float's is one.
+template <class T> __device__ __forceinline__ T select_min(T a, T b) { return sizeof(T) == 4 ? fmn(a, b) : (a < b ? a : b); }
+template <class T> __device__ __forceinline__ T select_max(T a, T b) { return sizeof(T) == 4 ? fmx(a, b) : (a < b ? b : a); }
+
 // The mask of sub-tests whose swept boxes overlap, for a pair that shares no vertex
-// (REJECT_RIGID: 0 as well for a pair whose sub-tests can have no root, see the end; LEAF: 0
-// as well for a pair whose leaf boxes, each triangle's boxes at x0 and x1 merged
-// (MergeTriBoundingBoxes, build_bvh.cu:452-460), do not overlap (checkOverlap,
-// aabb.cu:107-111)).
-template <class T, bool REJECT_RIGID, bool LEAF>
-__device__ __forceinline__ uint32_t ccd_pair_subbox_mask(const T* __restrict__ x0, const T* __restrict__ x1,
-                                                         long long i, long long j) {
+// (REJECT_RIGID: 0 as well for a pair whose sub-tests can have no root, see the end).
+// SELECT: double min and max by selects, right when no coordinate is NaN; *end sums up the end
+// positions, so it is NaN when one is (or when infinities of both signs meet).  *exact: the leaf
+// boxes overlap if the swept boxes of the triangles do: on each axis, every x0 + (x1 - x0) came
+// back to x1, or those boxes overlap by more than its rounding (3.4 2^-53 of the largest
+// coordinate).
+template <class T, bool REJECT_RIGID, bool SELECT>
+__device__ __forceinline__ uint32_t ccd_pair_subbox_axes(const T* __restrict__ x0, const T* __restrict__ x1,
+                                                         long long i, long long j, T* end, bool* exact) {
     const T* a0 = x0 + i * 9;
     const T* a1 = x1 + i * 9;
     const T* b0 = x0 + j * 9;
     const T* b1 = x1 + j * 9;
+    auto mn = [](T a, T b) { return SELECT ? select_min(a, b) : fmn(a, b); };
+    auto mx = [](T a, T b) { return SELECT ? select_max(a, b) : fmx(a, b); };
     uint32_t m = 0x7fffu;
     bool rigid = true;          // every vertex moves by the same displacement (on all axes so far)
-    bool leaf = true;           // the leaf boxes overlap (on all axes so far)
-    auto axis = [&](int ax) {
+    bool sure = true;
+    T sum = T(0);
+    // (one axis at a time keeps the registers of a kernel with several blocks an SM)
+#pragma unroll 1
+    for (int ax = 0; ax < 3; ++ax) {
         T alo[3], ahi[3], blo[3], bhi[3], dv[6];
-        T la = T(0), ha = T(0), lb = T(0), hb = T(0);
+        bool back = true;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            T av = __ldg(a0 + 3 * c + ax);
+            const T av = __ldg(a0 + 3 * c + ax);
             const T aw = __ldg(a1 + 3 * c + ax);
             dv[c] = aw - av;
-            T ae = av + dv[c];
-            alo[c] = fmn(av, ae);
-            ahi[c] = fmx(av, ae);
-            T bv = __ldg(b0 + 3 * c + ax);
+            const T ae = av + dv[c];
+            alo[c] = mn(av, ae);
+            ahi[c] = mx(av, ae);
+            const T bv = __ldg(b0 + 3 * c + ax);
             const T bw = __ldg(b1 + 3 * c + ax);
             dv[3 + c] = bw - bv;
-            T be = bv + dv[3 + c];
-            blo[c] = fmn(bv, be);
-            bhi[c] = fmx(bv, be);
-            if constexpr (LEAF) {
-                la = c ? fmn(la, fmn(av, aw)) : fmn(av, aw);
-                ha = c ? fmx(ha, fmx(av, aw)) : fmx(av, aw);
-                lb = c ? fmn(lb, fmn(bv, bw)) : fmn(bv, bw);
-                hb = c ? fmx(hb, fmx(bv, bw)) : fmx(bv, bw);
-            }
+            const T be = bv + dv[3 + c];
+            blo[c] = mn(bv, be);
+            bhi[c] = mx(bv, be);
+            back = back && ae == aw && be == bw;
+            if (SELECT) sum = sum + (ae + be);
         }
-        if constexpr (LEAF) leaf = leaf && la <= hb && ha >= lb;
         // the same displacement at all six vertices, finite, and start positions below half the
         // largest finite value so that every difference of two of them is finite too (the range
         // tests only where the displacements agree, which deforming pairs seldom do)
-        bool same = true;
+        if (REJECT_RIGID) {
+            bool same = true;
 #pragma unroll
-        for (int c = 1; c < 6; ++c) same = same && dv[c] == dv[0];
-        rigid = rigid && same;
-        if (rigid) {
-            const T half_max = sizeof(T) == 4 ? T(1.7e38) : T(8.9e307);
-            rigid = fabs(dv[0]) <= half_max;
+            for (int c = 1; c < 6; ++c) same = same && dv[c] == dv[0];
+            rigid = rigid && same;
+            if (rigid) {
+                const T half_max = sizeof(T) == 4 ? T(1.7e38) : T(8.9e307);
+                rigid = fabs(dv[0]) <= half_max;
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                rigid = rigid && fabs(__ldg(a0 + 3 * c + ax)) <= half_max && fabs(__ldg(b0 + 3 * c + ax)) <= half_max;
+                for (int c = 0; c < 3; ++c)
+                    rigid = rigid && fabs(__ldg(a0 + 3 * c + ax)) <= half_max && fabs(__ldg(b0 + 3 * c + ax)) <= half_max;
+            }
         }
         // edges 01, 02, 12 and the face
-        const T ealo[3] = {fmn(alo[0], alo[1]), fmn(alo[0], alo[2]), fmn(alo[1], alo[2])};
-        const T eahi[3] = {fmx(ahi[0], ahi[1]), fmx(ahi[0], ahi[2]), fmx(ahi[1], ahi[2])};
-        const T eblo[3] = {fmn(blo[0], blo[1]), fmn(blo[0], blo[2]), fmn(blo[1], blo[2])};
-        const T ebhi[3] = {fmx(bhi[0], bhi[1]), fmx(bhi[0], bhi[2]), fmx(bhi[1], bhi[2])};
-        const T falo = fmn(fmn(alo[0], alo[1]), alo[2]), fahi = fmx(fmx(ahi[0], ahi[1]), ahi[2]);
-        const T fblo = fmn(fmn(blo[0], blo[1]), blo[2]), fbhi = fmx(fmx(bhi[0], bhi[1]), bhi[2]);
+        const T ealo[3] = {mn(alo[0], alo[1]), mn(alo[0], alo[2]), mn(alo[1], alo[2])};
+        const T eahi[3] = {mx(ahi[0], ahi[1]), mx(ahi[0], ahi[2]), mx(ahi[1], ahi[2])};
+        const T eblo[3] = {mn(blo[0], blo[1]), mn(blo[0], blo[2]), mn(blo[1], blo[2])};
+        const T ebhi[3] = {mx(bhi[0], bhi[1]), mx(bhi[0], bhi[2]), mx(bhi[1], bhi[2])};
+        const T falo = mn(ealo[0], alo[2]), fahi = mx(eahi[0], ahi[2]);
+        const T fblo = mn(eblo[0], blo[2]), fbhi = mx(ebhi[0], bhi[2]);
+        if (!back) {
+            const T tol = (sizeof(T) == 8 ? T(4e-15) : T(4e-6)) * (fabs(falo) + fabs(fahi) + fabs(fblo) + fabs(fbhi));
+            sure = sure && fbhi - falo > tol && fahi - fblo > tol;
+        }
         uint32_t ma = 0;
 #pragma unroll
         for (int e0 = 0; e0 < 3; ++e0)
@@ -359,17 +398,39 @@ __device__ __forceinline__ uint32_t ccd_pair_subbox_mask(const T* __restrict__ x
             if (alo[c] <= fbhi && ahi[c] >= fblo) ma |= 1u << (12 + c);
         }
         m &= ma;
-    };
-    // (one axis at a time keeps the registers of a kernel with several blocks an SM)
-#pragma unroll 1
-    for (int ax = 0; ax < 3; ++ax) axis(ax);
+    }
+    *end = sum;
+    *exact = sure;
     // A pair whose six vertices all move by the same finite displacement (a static or rigidly
     // translating piece), with finite position differences, has in every sub-test
     // displacement differences of exactly zero: the t^3 and t^2 coefficients are exactly 0
     // (every term has such a factor and finite other factors), and the reference drops the
     // root of that linear case (collisions_continuous.cu:531-535), so no sub-test of the pair
     // can give a row or a contact.
-    return (REJECT_RIGID && rigid) || !leaf ? 0u : m;
+    return REJECT_RIGID && rigid ? 0u : m;
+}
+
+// (the double's NaN path, out of line: it is hardly ever taken)
+template <class T, bool REJECT_RIGID>
+__device__ __noinline__ uint32_t ccd_pair_subbox_nan(const T* __restrict__ x0, const T* __restrict__ x1, long long i,
+                                                     long long j) {
+    T end;
+    bool exact;
+    return ccd_pair_subbox_axes<T, REJECT_RIGID, false>(x0, x1, i, j, &end, &exact);
+}
+
+// ccd_pair_subbox_axes for any coordinates (LEAF: 0 as well for a pair whose leaf boxes do not
+// overlap; a pair with a sub-test has overlapping swept boxes, so the test itself is needed
+// only where those do not lie in the leaf boxes).
+template <class T, bool REJECT_RIGID, bool LEAF>
+__device__ __forceinline__ uint32_t ccd_pair_subbox_mask(const T* __restrict__ x0, const T* __restrict__ x1,
+                                                         long long i, long long j) {
+    T end;
+    bool exact;
+    uint32_t m = ccd_pair_subbox_axes<T, REJECT_RIGID, sizeof(T) == 8>(x0, x1, i, j, &end, &exact);
+    if (sizeof(T) == 8 && !(end == end)) m = ccd_pair_subbox_nan<T, REJECT_RIGID>(x0, x1, i, j);
+    if (LEAF && m && !exact && !ccd_pair_leaf_overlap<T>(x0, x1, i, j)) m = 0u;
+    return m;
 }
 
 // The same table packed into constants, so a runtime type k selects points without
