@@ -683,43 +683,22 @@ __device__ __forceinline__ bool weld_members(const Weld& W, int A, int B, int k,
     return true;
 }
 
-// Whether pair (A, B) solves its sub-test k: true when the sub-test is not shared or when
-// (A, B, k) is the smallest of its pairs; *shared tells which.  The members of a class are
-// in ascending corner id, so a vertex-face scan stops at the first pair that has the
-// sub-test.
-__device__ __forceinline__ bool weld_solves(const Weld& W, int A, int B, int k, int4 VA, int4 VB, bool* shared) {
-    *shared = false;
-    if (k >= 9) {
-        const bool vf = k >= 12;
-        const int4 Vface = vf ? VB : VA;
-        const int4 Vvert = vf ? VA : VB;
-        const int c = vf ? k - 12 : k - 9;
-        const int v = int4_at(Vvert, c);
-        if (((v | Vface.x | Vface.y | Vface.z) & CLS_NODEDUP) || class_size(Vvert, c) < 2) return true;
-        *shared = true;
-        const int end = v + class_size(Vvert, c);
-        for (int i = v; i < end; ++i) {
-            const int4 en = __ldg(W.fan + i);
-            const int t = en.x >> 2, cc = en.x & 3;
-            if (vf ? t >= B : t <= A) {
-                if (vf) break;             // the remaining corners are on later triangles
-                continue;
-            }
-            if (classes_meet(make_int4(en.y, en.z, en.w, 0), Vface)) continue;
-            return vf ? (t == A && cc == c) : (t == B && cc == c);
-        }
-        return true;    // (not reached: the pair itself has the sub-test)
+// Whether pair (A, B) solves its shared vertex-face sub-test k, that is whether it is the smallest
+// of the sub-test's pairs.  The members of a class are in ascending corner id, so the scan stops
+// at the first pair that has the sub-test.
+__device__ __forceinline__ bool weld_vf_solves(const Weld& W, int A, int B, int k, int4 VA, int4 VB) {
+    const bool vf = k >= 12;                     // vertex of A, face of B (else face of A)
+    const int4 Vface = vf ? VB : VA;
+    const int4 Vvert = vf ? VA : VB;
+    const int c = vf ? k - 12 : k - 9;
+    const int v = int4_at(Vvert, c), end = v + class_size(Vvert, c), own = 4 * (vf ? A : B) + c;
+    for (int i = v; i < end; ++i) {
+        const int4 en = __ldg(W.fan + i);
+        if (en.x == own) return true;            // (none before it)
+        if (!vf && (en.x >> 2) <= A) continue;
+        if (!classes_meet(make_int4(en.y, en.z, en.w, 0), Vface)) return false;
     }
-    int ma = A, mb = B, mk = k;
-    const bool sh = weld_members(W, A, B, k, VA, VB, [&](int a, int b, int kk) {
-        if (a < ma || (a == ma && (b < mb || (b == mb && kk < mk)))) {
-            ma = a;
-            mb = b;
-            mk = kk;
-        }
-    });
-    *shared = sh;
-    return !sh || (ma == A && mb == B && mk == k);
+    return true;    // (not reached: the pair itself has the sub-test)
 }
 
 // The pairs of sub-test k of pair (A, B) in (ma, mb, mk), at most WELD_FANCAP of them (a
@@ -789,6 +768,8 @@ __device__ __forceinline__ int reserve_rows(int* mesh_counters, const Forest& F,
 //    hdr->subtests counts the sub-tests of the masks.
 //  * k_ccd_stage_pending: the pending pairs' vertex-face sub-tests, spread over the lanes
 //    of a warp (a scan of the vertex's class each); then the pairs go to the live list.
+//    (Each pair's lane lists its sub-tests; a search for the pair and the n-th bit by each
+//    taking lane cost more than the scans: 765 -> 460 us on the 64-mesh step.)
 // Records: (slot i, slot j, the sub-tests to solve in bits 0..14 with the shared ones in
 // bits 15..29, pending vertex-face sub-tests).
 static constexpr int STAGE_THREADS = 256;
@@ -972,17 +953,18 @@ k_ccd_stage_mask(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, con
 
 static __global__ void __launch_bounds__(STAGE_THREADS, 8)
 k_ccd_stage_pending(int cand_cap, WsHeader* hdr, Weld W, const int4* __restrict__ pending, int4* __restrict__ live) {
-    // per warp: 32 pending pairs, their classes, pending sub-tests, the prefix of their
-    // counts and the sub-tests they solve; the lanes take the sub-tests 32 at a time
+    // per warp: 32 pending pairs, their classes, the sub-tests they solve, and their pending
+    // sub-tests (lane of the pair << 4 | type) one after the other; the lanes take those 32 at a
+    // time
     __shared__ int2 s_pr[STAGE_THREADS];
     __shared__ int4 s_va[STAGE_THREADS], s_vb[STAGE_THREADS];
-    __shared__ unsigned s_bits[STAGE_THREADS], s_word[STAGE_THREADS];
-    __shared__ int s_pre[STAGE_THREADS];
+    __shared__ unsigned s_word[STAGE_THREADS];
+    __shared__ unsigned short s_item[STAGE_WARPS][6 * 32];
     const int n = min(*(volatile int*)&hdr->pending_count, cand_cap);
-    const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31;
+    const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31, wq = tid >> 5;
     const unsigned FULL = 0xffffffffu;
     const int warps = gridDim.x * STAGE_WARPS;
-    for (int base = (blockIdx.x * STAGE_WARPS + (tid >> 5)) * 32; base < n; base += warps * 32) {
+    for (int base = (blockIdx.x * STAGE_WARPS + wq) * 32; base < n; base += warps * 32) {
         const int c = base + lane;
         unsigned pend = 0u, word = 0u;
         int2 pr = make_int2(0, 0);
@@ -990,29 +972,22 @@ k_ccd_stage_pending(int cand_cap, WsHeader* hdr, Weld W, const int4* __restrict_
             const int4 rec = pending[c];
             pr = make_int2(rec.x, rec.y);
             word = (unsigned)rec.z;
-            pend = (unsigned)rec.w;
+            pend = (unsigned)rec.w & 0x7e00u;        // (types 9 .. 14)
             s_va[tid] = __ldg(W.vid + pr.x);
             s_vb[tid] = __ldg(W.vid + pr.y);
         }
         s_pr[tid] = pr;
-        s_bits[tid] = pend;
         s_word[tid] = word;
         const int incl = warp_inclusive_scan(__popc(pend), lane);
-        s_pre[tid] = incl;
+        int at = incl - __popc(pend);
+        for (; pend; pend &= pend - 1) s_item[wq][at++] = (unsigned short)(lane << 4 | (__ffs(pend) - 1));
         const int total = __shfl_sync(FULL, incl, 31);
         __syncwarp();
         for (int r = lane; r < total; r += 32) {
-            int lo = 0, hi = 31;                       // the pair: first prefix above r
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (s_pre[w0 + mid] > r) hi = mid;
-                else lo = mid + 1;
-            }
-            const int p = w0 + lo;
-            const int k = __fns(s_bits[p], 0, r - (lo ? s_pre[p - 1] : 0) + 1);
-            bool sh = false;
-            if (weld_solves(W, s_pr[p].x, s_pr[p].y, k, s_va[p], s_vb[p], &sh))
-                atomicOr(&s_word[p], (1u << k) | (sh ? 1u << (15 + k) : 0u));
+            const int item = s_item[wq][r];
+            const int p = w0 + (item >> 4), k = item & 15;
+            if (weld_vf_solves(W, s_pr[p].x, s_pr[p].y, k, s_va[p], s_vb[p]))
+                atomicOr(&s_word[p], (1u << k) | (1u << (15 + k)));
         }
         __syncwarp();
         word = s_word[tid];
