@@ -165,102 +165,12 @@ template <class T> __device__ __forceinline__ bool sat(const Tri<T>& a, const Tr
 
 // ------------------------------------------------------------------ continuous collision
 
-// MovingTriangle (figures.cu:295-366): positions at t = 0 and displacement x1 - x0
-template <class T> struct MTri { V3<T> v[3], dv[3]; };
-template <class T> __device__ __forceinline__ MTri<T> load_mtri(const T* __restrict__ x0, const T* __restrict__ x1, int64_t i) {
-    Tri<T> a = load_tri(x0, i), b = load_tri(x1, i);
-    MTri<T> m;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { m.v[c] = a.v[c]; m.dv[c] = b.v[c] - a.v[c]; }
-    return m;
-}
-// MovingTriangle::ComputeBBoxVertex (346-351): box of v and v + dv
-template <class T> __device__ __forceinline__ Box<T> mvbox(const MTri<T>& t, int i) {
-    V3<T> a = t.v[i], b = t.v[i] + t.dv[i];
-    Box<T> r;
-    r.lo = mk<T>(fmn(a.x, b.x), fmn(a.y, b.y), fmn(a.z, b.z));
-    r.hi = mk<T>(fmx(a.x, b.x), fmx(a.y, b.y), fmx(a.z, b.z));
-    return r;
-}
-template <class T> __device__ __forceinline__ Box<T> svbox(const Tri<T>& t, int i) {
-    Box<T> r;
-    r.lo = t.v[i];
-    r.hi = t.v[i];
-    return r;
-}
-
-// Point table of the 15 sub-tests (collisions_continuous.cu:36-124): bits per point p:
-// side (first/second triangle of the pair) and corner.  Types 0..8 edge-edge with edges
-// {01, 02, 12}[k/3] and [k%3]; 9..11 face of the first vs vertex k-9 of the second;
-// 12..14 vertex k-12 of the first vs face of the second.
-__device__ __forceinline__ void type_points(int k, int side[4], int corner[4]) {
-    if (k < 9) {
-        int e0 = k / 3, e1 = k - 3 * (k / 3);
-        side[0] = 0; corner[0] = e0 == 2 ? 1 : 0;
-        side[1] = 0; corner[1] = e0 == 0 ? 1 : 2;
-        side[2] = 1; corner[2] = e1 == 2 ? 1 : 0;
-        side[3] = 1; corner[3] = e1 == 0 ? 1 : 2;
-    } else if (k < 12) {
-        side[0] = 0; corner[0] = 0;
-        side[1] = 0; corner[1] = 1;
-        side[2] = 0; corner[2] = 2;
-        side[3] = 1; corner[3] = k - 9;
-    } else {
-        side[0] = 0; corner[0] = k - 12;
-        side[1] = 1; corner[1] = 0;
-        side[2] = 1; corner[2] = 1;
-        side[3] = 1; corner[3] = 2;
-    }
-}
-
-// check_minimal_bbox_overlap (collisions_continuous.cu:234-318): swept sub-boxes, no threshold
-template <class T> __device__ __forceinline__ bool ccd_subbox(const MTri<T>& a, const MTri<T>& b, int k) {
-    int side[4], corner[4];
-    type_points(k, side, corner);
-    Box<T> b0, b1;
-    if (k < 9) {
-        b0 = merge(mvbox(a, corner[0]), mvbox(a, corner[1]));
-        b1 = merge(mvbox(b, corner[2]), mvbox(b, corner[3]));
-    } else if (k < 12) {
-        b0 = merge(merge(mvbox(a, 0), mvbox(a, 1)), mvbox(a, 2));
-        b1 = mvbox(b, k - 9);
-    } else {
-        b0 = mvbox(a, k - 12);
-        b1 = merge(merge(mvbox(b, 0), mvbox(b, 1)), mvbox(b, 2));
-    }
-    return overlap(b0, b1, (T)0);
-}
-
-// all 15 swept sub-box tests as a bit mask; the three per-vertex swept boxes of each
-// triangle are computed once
-template <class T> __device__ __forceinline__ uint32_t ccd_subbox_mask(const MTri<T>& a, const MTri<T>& b) {
-    Box<T> va[3], vb[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) { va[i] = mvbox(a, i); vb[i] = mvbox(b, i); }
-    Box<T> ea[3], eb[3];
-    ea[0] = merge(va[0], va[1]); ea[1] = merge(va[0], va[2]); ea[2] = merge(va[1], va[2]);
-    eb[0] = merge(vb[0], vb[1]); eb[1] = merge(vb[0], vb[2]); eb[2] = merge(vb[1], vb[2]);
-    Box<T> fa = merge(merge(va[0], va[1]), va[2]);
-    Box<T> fb = merge(merge(vb[0], vb[1]), vb[2]);
-    uint32_t m = 0;
-#pragma unroll
-    for (int e0 = 0; e0 < 3; ++e0)
-#pragma unroll
-        for (int e1 = 0; e1 < 3; ++e1)
-            if (overlap(ea[e0], eb[e1], (T)0)) m |= 1u << (3 * e0 + e1);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        if (overlap(fa, vb[i], (T)0)) m |= 1u << (9 + i);
-        if (overlap(va[i], fb, (T)0)) m |= 1u << (12 + i);
-    }
-    return m;
-}
-
 // The shared-vertex test and the 15 swept sub-box tests of a candidate pair (i, j), read
 // straight from the soups one axis at a time: both are conjunctions over the axes (equal
-// coordinates; intervals that overlap), so the per-axis results are ANDed.  Same boxes and
-// comparisons as share_vertex + ccd_subbox_mask (v and v + dv with dv = x1 - x0, min / max
-// merges, inclusive bounds), with a third of the live values.
+// coordinates; intervals that overlap), so the per-axis results are ANDed.  The boxes are the
+// reference's (check_minimal_bbox_overlap, collisions_continuous.cu:234-318, over
+// MovingTriangle::ComputeBBoxVertex, figures.cu:346-351): v and v + dv with dv = x1 - x0, min /
+// max merges, inclusive bounds.
 
 // shareVertex of the start positions (figures.cu:527-544): any vertex of i equal to one of
 // j on every axis
@@ -433,9 +343,13 @@ __device__ __forceinline__ uint32_t ccd_pair_subbox_mask(const T* __restrict__ x
     return m;
 }
 
-// The same table packed into constants, so a runtime type k selects points without
-// indexing local arrays: side(k, p) = bit 4k + p of CCD_SIDE_TABLE, corner(k, p) = the
-// 2-bit field 8 (k % 8) + 2p of CCD_CORNER_TABLE[k / 8].
+// Point table of the 15 sub-tests (collisions_continuous.cu:36-124): bits per point p:
+// side (first/second triangle of the pair) and corner.  Types 0..8 edge-edge with edges
+// {01, 02, 12}[k/3] and [k%3]; 9..11 face of the first vs vertex k-9 of the second;
+// 12..14 vertex k-12 of the first vs face of the second.
+// Packed into constants, so that a run-time type k selects points without indexing local
+// arrays: side(k, p) = bit 4k + p of CCD_SIDE_TABLE, corner(k, p) = the 2-bit field
+// 8 (k % 8) + 2p of CCD_CORNER_TABLE[k / 8].
 constexpr int ccd_side_of(int k, int p) { return k < 9 ? (p >= 2) : (k < 12 ? (p == 3) : (p >= 1)); }
 constexpr int ccd_corner_of(int k, int p) {
     return k < 9 ? (p == 0 ? (k / 3 == 2 ? 1 : 0) : p == 1 ? (k / 3 == 0 ? 1 : 2)
@@ -466,21 +380,27 @@ __device__ __forceinline__ int tet_corner(int k, int p) {
 
 template <class T> struct MTet { V3<T> v[4], dv[4]; };
 
+// element offsets of the four points of sub-test k in a soup (slots are below 2^28, so they fit
+// 32 bits; the type's sides and corners come in one word each)
+__device__ __forceinline__ void point_offsets(unsigned gi, unsigned gj, int k, unsigned o[4]) {
+    const unsigned sides = (unsigned)(CCD_SIDE_TABLE >> (4 * k));
+    const unsigned corners = (unsigned)((k < 8 ? CCD_CORNER_TABLE0 : CCD_CORNER_TABLE1) >> (8 * (k & 7)));
+    const unsigned oi = 9u * gi, oj = 9u * gj;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) o[p] = ((sides >> p) & 1u ? oj : oi) + 3u * ((corners >> (2 * p)) & 3u);
+}
+
 // tetrahedron of sub-test k read straight from the two soups: the four points at t = 0 and
 // their displacements x1 - x0 (make_tetrahedron, collisions_continuous.cu:36-124)
 template <class T>
 __device__ __forceinline__ MTet<T> load_tet(const T* __restrict__ x0, const T* __restrict__ x1, long long gi,
                                             long long gj, int k) {
     MTet<T> t;
-    // (the type's sides and corners in one word each; slots are below 2^28, so element
-    // offsets fit 32 bits)
-    const unsigned sides = (unsigned)(CCD_SIDE_TABLE >> (4 * k));
-    const unsigned corners = (unsigned)((k < 8 ? CCD_CORNER_TABLE0 : CCD_CORNER_TABLE1) >> (8 * (k & 7)));
-    const unsigned oi = 9u * (unsigned)gi, oj = 9u * (unsigned)gj;
+    unsigned o[4];
+    point_offsets((unsigned)gi, (unsigned)gj, k, o);
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-        const unsigned o = ((sides >> p) & 1u ? oj : oi) + 3u * ((corners >> (2 * p)) & 3u);
-        const T *pa = x0 + o, *pb = x1 + o;
+        const T *pa = x0 + o[p], *pb = x1 + o[p];
         const V3<T> a = mk<T>(__ldg(pa), __ldg(pa + 1), __ldg(pa + 2));
         const V3<T> b = mk<T>(__ldg(pb), __ldg(pb + 1), __ldg(pb + 2));
         t.v[p] = a;
@@ -489,17 +409,13 @@ __device__ __forceinline__ MTet<T> load_tet(const T* __restrict__ x0, const T* _
     return t;
 }
 
-template <class T> __device__ __forceinline__ MTet<T> make_tet(const MTri<T>& a, const MTri<T>& b, int k) {
-    int side[4], corner[4];
-    type_points(k, side, corner);
-    MTet<T> t;
+// the four points of sub-test k of a static pair
+template <class T>
+__device__ __forceinline__ void load_points(const T* __restrict__ tri, int gi, int gj, int k, V3<T> v[4]) {
+    unsigned o[4];
+    point_offsets((unsigned)gi, (unsigned)gj, k, o);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const MTri<T>& s = side[i] ? b : a;
-        t.v[i] = s.v[corner[i]];
-        t.dv[i] = s.dv[corner[i]];
-    }
-    return t;
+    for (int p = 0; p < 4; ++p) v[p] = mk<T>(__ldg(tri + o[p]), __ldg(tri + o[p] + 1), __ldg(tri + o[p] + 2));
 }
 
 // MovingTetraMatrix::coef3..coef0 (figures.cu:122-293): exact term order, summed from 0
@@ -990,21 +906,37 @@ __device__ __forceinline__ void apply_impulse(const MTet<T>& tet, long long gi, 
 
 // ------------------------------------------------------------------ proximity
 
-template <class T> __device__ __forceinline__ bool prox_subbox(const Tri<T>& a, const Tri<T>& b, int k, T th) {
-    int side[4], corner[4];
-    type_points(k, side, corner);
-    Box<T> b0, b1;
-    if (k < 9) {
-        b0 = merge(svbox(a, corner[0]), svbox(a, corner[1]));
-        b1 = merge(svbox(b, corner[2]), svbox(b, corner[3]));
-    } else if (k < 12) {
-        b0 = tri_box(a);
-        b1 = svbox(b, k - 9);
-    } else {
-        b0 = svbox(a, k - 12);
-        b1 = tri_box(b);
-    }
-    return overlap(b0, b1, th);
+// The sub-tests of a pair whose boxes come within th of each other (check_minimal_bbox_overlap
+// on static boxes, proximity_static.cu:96-203): bit k of type k, the first triangle's box
+// against the second's widened one (checkOverlap, aabb.cu:101-111), one axis at a time.
+template <class T>
+__device__ __forceinline__ uint32_t prox_subbox_mask(const Tri<T>& a, const Tri<T>& b, T th) {
+    uint32_t m = 0x7fffu;
+    auto axis = [&](T a0, T a1, T a2, T b0, T b1, T b2) {
+        const T av[3] = {a0, a1, a2}, bv[3] = {b0, b1, b2};
+        const T ealo[3] = {fmn(a0, a1), fmn(a0, a2), fmn(a1, a2)}, eahi[3] = {fmx(a0, a1), fmx(a0, a2), fmx(a1, a2)};
+        const T eblo[3] = {fmn(b0, b1), fmn(b0, b2), fmn(b1, b2)}, ebhi[3] = {fmx(b0, b1), fmx(b0, b2), fmx(b1, b2)};
+        const T falo = fmn(a0, fmn(a1, a2)), fahi = fmx(a0, fmx(a1, a2));
+        const T fblo = fmn(b0, fmn(b1, b2)) - th, fbhi = fmx(b0, fmx(b1, b2)) + th;
+        uint32_t ma = 0;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+            const T lo = eblo[f] - th, hi = ebhi[f] + th;
+#pragma unroll
+            for (int e = 0; e < 3; ++e)
+                if (ealo[e] <= hi && eahi[e] >= lo) ma |= 1u << (3 * e + f);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (falo <= bv[c] + th && fahi >= bv[c] - th) ma |= 1u << (9 + c);
+            if (av[c] <= fbhi && av[c] >= fblo) ma |= 1u << (12 + c);
+        }
+        m &= ma;
+    };
+    axis(a.v[0].x, a.v[1].x, a.v[2].x, b.v[0].x, b.v[1].x, b.v[2].x);
+    axis(a.v[0].y, a.v[1].y, a.v[2].y, b.v[0].y, b.v[1].y, b.v[2].y);
+    axis(a.v[0].z, a.v[1].z, a.v[2].z, b.v[0].z, b.v[1].z, b.v[2].z);
+    return m;
 }
 
 // vec_sq_diff returns float (utils.cu:57-61); the distance is sqrt in float
@@ -1024,13 +956,9 @@ template <class T> __device__ __forceinline__ void pt_seg(V3<T> p, V3<T> a, V3<T
     }
 }
 
-// compute_distance_edge_edge / compute_distance_triangle_node (proximity_static.cu:205-433)
-template <class T> __device__ __forceinline__ T prox_distance(const Tri<T>& a, const Tri<T>& b, int k) {
-    int side[4], corner[4];
-    type_points(k, side, corner);
-    V3<T> v[4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p) v[p] = (side[p] ? b : a).v[corner[p]];
+// compute_distance_edge_edge / compute_distance_triangle_node (proximity_static.cu:205-433), on the
+// four points of a sub-test of type k (load_points)
+template <class T> __device__ __forceinline__ T prox_distance(const V3<T> v[4], int k) {
     if (k < 9) {
         V3<T> da = v[1] - v[0], db = v[3] - v[2], dc = v[2] - v[0];
         T s = dot(cross(dc, db), cross(da, db)) / norm2(cross(da, db));
@@ -1048,8 +976,10 @@ template <class T> __device__ __forceinline__ T prox_distance(const Tri<T>& a, c
         if (!sv || !tv) return (T)-1;
         return (T)__fsqrt_rn(sq_diff_f(axpy(v[0], da, s), axpy(v[2], db, t)));
     }
-    int f0 = k < 12 ? 0 : 1, f1 = k < 12 ? 1 : 2, f2 = k < 12 ? 2 : 3, fv = k < 12 ? 3 : 0;
-    V3<T> e1 = v[f0] - v[f1], e2 = v[f2] - v[f1], ep = v[fv] - v[f1];
+    // (selects rather than run-time indices, which would move the points to local memory)
+    const bool inv = k >= 12;
+    const V3<T> f0 = inv ? v[1] : v[0], f1 = inv ? v[2] : v[1], f2 = inv ? v[3] : v[2], fv = inv ? v[0] : v[3];
+    V3<T> e1 = f0 - f1, e2 = f2 - f1, ep = fv - f1;
     T d00 = dot(e1, e1), d01 = dot(e1, e2), d11 = dot(e2, e2), d20 = dot(ep, e1), d21 = dot(ep, e2);
     T denom = fms2(d00, d11, d01, d01);
     T u = fms2(d11, d20, d01, d21) / denom;
@@ -1057,8 +987,8 @@ template <class T> __device__ __forceinline__ T prox_distance(const Tri<T>& a, c
     T vv = 1 - w - u;
     bool ok = (vv >= 0 && vv <= 1) && (w >= 0 && w <= 1) && (u >= 0 && u <= 1);
     if (!ok) return (T)-1;
-    V3<T> pt = lin3(v[f0], u, v[f1], vv, v[f2], w);
-    return (T)__fsqrt_rn(sq_diff_f(v[fv], pt));
+    V3<T> pt = lin3(f0, u, f1, vv, f2, w);
+    return (T)__fsqrt_rn(sq_diff_f(fv, pt));
 }
 
 }  // namespace ccc

@@ -85,3 +85,18 @@ def test_engine_rows_and_loop(cuda, oracle, name):
         eng.loop_step(1)
         assert int(eng.state([sid])["contacts"][0]) == len(er)
         eng.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("name,threshold", [(n, t) for n in MESHES for t in (0.0, 0.02, 0.3)])
+def test_proximity(cuda, oracle, name, threshold, dtype):
+    import cccollisions_b200 as C
+    x0 = _mesh(name)[0].astype(dtype)
+    F = len(x0)
+    X = torch.from_numpy(x0[None]).to(cuda)
+    boxes, tree = C.bvh(X)
+    (rows,) = C.find_proximity(boxes, tree, X, threshold, 15 * min(F, 400))
+    n = int((rows[0, :, 0] >= 0).sum())
+    bb, tr = oracle.bvh(x0)
+    assert Counter(map(tuple, rows[0, :n].tolist())) == Counter(map(tuple, oracle.proximity(bb, tr, x0, threshold)[0].tolist()))
