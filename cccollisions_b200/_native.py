@@ -44,6 +44,7 @@ SIGNATURES = {
     "ccc_workspace_size": (_I64, [_I, _I64, _I64, _I64]),
     "ccc_read_status": (_I, [_P, _I64, _P, _P]),
     "ccc_read_counters": (_I, [_P, _P, _P]),
+    "ccc_fill": (_I, [_P, _I64, _I64, _P, _I64, _I64, _P, _I64, _I64, _P]),
     "ccc_bvh": (_I, [_I, _P, _P, _I64, _I64, _P, _P, _P, _I64, _P]),
     "ccc_find_collisions": (_I, [_I, _P, _P, _P, _I64, _I64, _D, _I64, _P, _P, _I64, _P]),
     "ccc_find_collisions_continuous": (_I, [_I, _P, _P, _P, _P, _P, _I64, _I64, _I64, _I64, _P, _P, _P, _I64, _P]),

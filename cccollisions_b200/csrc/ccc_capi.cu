@@ -532,6 +532,25 @@ int64_t ccc_workspace_size(int op, int64_t B, int64_t F, int64_t maxc) {
     return layout(B, F, per, nodes).end;
 }
 
+int ccc_fill(void* p0, int64_t b0, int64_t v0, void* p1, int64_t b1, int64_t v1, void* p2, int64_t b2, int64_t v2,
+             void* stream) {
+    const FillJob j[3] = {{(uint32_t*)p0, b0 / 4, (uint32_t)v0, (uint32_t)((uint64_t)v0 >> 32)},
+                          {(uint32_t*)p1, b1 / 4, (uint32_t)v1, (uint32_t)((uint64_t)v1 >> 32)},
+                          {(uint32_t*)p2, b2 / 4, (uint32_t)v2, (uint32_t)((uint64_t)v2 >> 32)}};
+    int64_t words = 0;
+    const int64_t bytes[3] = {b0, b1, b2};
+    for (int i = 0; i < 3; ++i) {
+        if (bytes[i] < 0 || bytes[i] % 4 || (bytes[i] > 0 && (!j[i].p || ((uintptr_t)j[i].p & 3)))) return CCC_ERR_INVALID_ARG;
+        words += j[i].words;
+    }
+    if (words == 0) return CCC_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int g = (int)std::min<int64_t>((words + 4 * 256 - 1) / (4 * 256), (int64_t)num_sms() * 16);
+    CCC_LAUNCH("k_fill", s, k_fill<<<g, 256, 0, s>>>(j[0], j[1], j[2]));
+    CCC_LAUNCH_CHECK();
+    return CCC_OK;
+}
+
 int ccc_read_status(const void* ws, int64_t n_mesh, int32_t* out, void* stream) {
     if (!ws || !out || n_mesh < 0) return CCC_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;

@@ -112,6 +112,27 @@ static __global__ void k_uniform_offsets(int* nm, int* voff, int* poff, int* sid
 }
 
 // ---------------------------------------------------------------------------------------
+// Up to three arrays of 4-byte words filled with 8-byte patterns (lo, hi), 16 bytes a store
+// where an array is aligned for it.
+struct FillJob {
+    uint32_t* p;
+    long long words;
+    uint32_t lo, hi;
+};
+static __global__ void k_fill(FillJob a, FillJob b, FillJob c) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    auto fill = [&](const FillJob& j) {
+        const long long quads = ((uintptr_t)j.p & 15) == 0 ? j.words / 4 : 0;
+        const uint4 v = make_uint4(j.lo, j.hi, j.lo, j.hi);
+        for (long long i = t; i < quads; i += stride) reinterpret_cast<uint4*>(j.p)[i] = v;
+        for (long long i = 4 * quads + t; i < j.words; i += stride) j.p[i] = i & 1 ? j.hi : j.lo;
+    };
+    fill(a);
+    fill(b);
+    fill(c);
+}
+
+// ---------------------------------------------------------------------------------------
 // Import of exported tensors into traversal nodes (build_bvh_from_array_tree 667-705 and
 // set_rightmost_nodes 707-743).
 

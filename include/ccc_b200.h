@@ -109,6 +109,12 @@ int ccc_read_status(const void* ws, int64_t n_mesh, int32_t* out, void* stream);
  * sub-tests solved, roots in [0, 1] filtered. */
 int ccc_read_counters(const void* ws, int32_t* out, void* stream);
 
+/* Fills up to three device arrays of bytes0 .. bytes2 (multiples of 4) with repeated 8-byte
+ * patterns in one launch (an absent array is NULL with 0 bytes): the initial values that the
+ * outputs of the calls below need. */
+int ccc_fill(void* array0, int64_t bytes0, int64_t pattern0, void* array1, int64_t bytes1, int64_t pattern1,
+             void* array2, int64_t bytes2, int64_t pattern2, void* stream);
+
 /* bvh / bvh_motion — replaces build_bvh(triangles[, triangles_next], &bboxes, &tree)
  * (src/build_bvh.cu:381-449, 570-648; bindings src/cccollisions.cpp:102-132).
  * triangles_next may be NULL (static build).  Writes every row of bboxes and tree in the
