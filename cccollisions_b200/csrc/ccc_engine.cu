@@ -51,6 +51,7 @@ struct EngineLayout {
     int64_t tab, btab, bounds;
     int64_t x0, x1, masses, faces;
     int64_t leaf_tri, lparent, nparent, visits, nodes, qnodes, qcode, qleaf, nrange, front;
+    int64_t ntop, top_node, top_index, top_child;
     int64_t rows, times, cand;
     int64_t keys0, keys1, vals0, vals1, hist;
     int64_t verts0, verts1, vel, acc;
@@ -90,6 +91,10 @@ EngineLayout engine_layout(int64_t tsz, int64_t tc, int64_t vc, int64_t mc, int6
     L.qleaf = take(tc * 4);
     L.nrange = take(tc * 8);
     L.front = take(tc * 8);
+    L.ntop = take(mc * 8);              // top nodes of the refit (k_refit_plan): per slot id, per slot
+    L.top_node = take(tc * 4);
+    L.top_index = take(tc * 4);
+    L.top_child = take(tc * 8);
     L.rows = take(tc * maxcol * 3 * 8);
     L.times = take(tc * maxcol * tsz);
     L.cand_cap = tc * maxc;
@@ -109,11 +114,11 @@ EngineLayout engine_layout(int64_t tsz, int64_t tc, int64_t vc, int64_t mc, int6
     L.wtab = take(tc * 6 * 4);
     L.vidc = take(tc * 4 * 4);
     L.wcnt = take(tc * 4 * 4);
-    L.fan_end = take(tc * 4 * 4);
     L.fan = take(tc * 3 * 16);
     L.fan_tmp = take(tc * 3 * 16);      // the member list in order of arrival
     L.vid4 = take(tc * 16);
     L.twin4 = take(tc * 16);
+    L.fan_end = L.twin4;                // (the fill's cursors: the twins are written after it)
     L.third4 = take(tc * 16);
     L.pending = take(L.cand_cap * 16);
     L.live = take(L.cand_cap * 16);
@@ -266,20 +271,26 @@ int upload_table(ccc_engine* e, int which, const int32_t* ids, int64_t n, cudaSt
 // The refit's climbs are chains of dependent L2 round trips, so it runs about one leaf per
 // thread (up to 64 blocks per SM) rather than a grid-stride loop over few threads.
 inline int refit_grid(const ccc_engine* e) {
-    return (int)std::min<int64_t>(grid_for(e->tri_cap, REFIT_THREADS), (int64_t)num_sms() * 64);
+    return (int)std::min<int64_t>(e->tri_cap / REFIT_THREADS + e->mesh_cap, (int64_t)num_sms() * 64);
 }
 
+// blocks of `per` a mesh, about as many as are resident together
+inline int top_grid(const ccc_engine* e, int per) {
+    return per * (int)std::max<int64_t>(1, std::min<int64_t>(e->mesh_cap, num_sms() / per));
+}
+
+// (hdr->front is 0 before it: a step clears the header, the build only that word)
 template <class T> int refit(ccc_engine* e, const Tables& t, const int* flags, cudaStream_t s) {
-    if (cudaMemsetAsync(&e->hdr()->front, 0, sizeof(int), s) != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH("k_engine_refit", s, k_engine_refit_local<T><<<refit_grid(e), REFIT_THREADS, 0, s>>>(
         t.f, e->at<T>(e->L.x0), e->at<T>(e->L.x1), e->at<int>(e->L.leaf_tri), e->at<int>(e->L.lparent),
         e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
-        e->at<TNode>(e->L.nodes), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.front), (int)e->tri_cap, flags,
-        e->hdr()));
+        e->at<TNode>(e->L.nodes), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop), e->at<int2>(e->L.front),
+        (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_engine_refit_front", s, k_engine_refit_front<<<num_sms() * 8, 256, 0, s>>>(
-        t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes),
-        e->at<unsigned>(e->L.visits), e->at<int2>(e->L.front), (int)e->tri_cap, e->hdr()));
+    CCC_LAUNCH("k_engine_refit_front", s, k_engine_refit_top<<<top_grid(e, TOP_CLUSTER), TOP_THREADS, sizeof(TopShared), s>>>(
+        t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
+        e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
+        e->at<unsigned>(e->L.visits), e->at<int2>(e->L.front), (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
 }
@@ -466,7 +477,8 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     if (ntri == 0) return CCC_OK;
     Tables t = e->building();
     unsigned* bounds = e->at<unsigned>(e->L.bounds);
-    CCC_LAUNCH("k_reset_bounds", s, k_reset_bounds<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(t.f, bounds));
+    CCC_LAUNCH("k_reset_bounds", s, k_reset_bounds<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(
+        t.f, bounds, e->at<int2>(e->L.ntop)));
     CCC_LAUNCH_CHECK();
     unsigned long long* keys[2] = {e->at<unsigned long long>(e->L.keys0), e->at<unsigned long long>(e->L.keys1)};
     int* vals[2] = {e->at<int>(e->L.vals0), e->at<int>(e->L.vals1)};
@@ -502,7 +514,8 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     }
     CCC_LAUNCH("k_karras_build", s, k_karras_build<<<item_grid(), ITEM_THREADS, 0, s>>>(
         t.f, keys[cur], vals[cur], e->at<TNode>(e->L.nodes), e->at<int>(e->L.nparent), e->at<int>(e->L.lparent),
-        e->at<int>(e->L.leaf_tri), e->at<unsigned>(e->L.visits), e->at<int2>(e->L.nrange), &e->hdr()->status));
+        e->at<int>(e->L.leaf_tri), e->at<unsigned>(e->L.visits), e->at<int2>(e->L.nrange), e->at<int2>(e->L.ntop),
+        e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
     CCC_LAUNCH("k_qtree_depth", s, k_qtree_depth<<<item_grid(), ITEM_THREADS, 0, s>>>(
         t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), &e->hdr()->status));
@@ -511,6 +524,12 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
         t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<QNode>(e->L.qnodes),
         &e->hdr()->status));
     CCC_LAUNCH_CHECK();
+    CCC_LAUNCH("k_refit_plan", s, k_refit_plan<<<top_grid(e, 1), TOP_THREADS, sizeof(PlanShared), s>>>(
+        t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
+        e->at<int2>(e->L.ntop), e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
+        &e->hdr()->status));
+    CCC_LAUNCH_CHECK();
+    if (cudaMemsetAsync(&e->hdr()->front, 0, sizeof(int), s) != cudaSuccess) return CCC_ERR_CUDA;
     return refit<T>(e, t, nullptr, s);
 }
 
@@ -540,7 +559,11 @@ bool active_built(const ccc_engine* e) {
 // shared-memory attributes of the narrow-phase kernels an engine launches, set before any
 // stream capture
 template <class T> bool prepare_kernels() {
-    return prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
+    return cudaFuncSetAttribute(k_engine_refit_top, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(TopShared)) == cudaSuccess &&
+           cudaFuncSetAttribute(k_refit_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PlanShared)) ==
+               cudaSuccess &&
+           prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_PORTABLE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_IMPULSES, LoopSink<T>, LIB_PORTABLE, SRC_STAGED>() == cudaSuccess &&

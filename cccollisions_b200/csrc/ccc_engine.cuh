@@ -283,6 +283,10 @@ k_radix_scatter(const unsigned long long* __restrict__ kin, const int* __restric
 // their aux words (rightmost leaf position of an internal child, triangle id of a leaf),
 // the parent codes ((parent << 1) | side) of nodes and leaves and the leaf -> triangle map,
 // and clears the refit counters.
+static constexpr int REFIT_THREADS = 256;      // leaf positions of a refit block, from the mesh's first
+// whether a node's leaf range spans refit blocks
+__device__ __forceinline__ bool refit_crosses(int2 r) { return r.x / REFIT_THREADS != r.y / REFIT_THREADS; }
+
 __device__ __forceinline__ int karras_delta(const unsigned long long* k, int n, int i, int j) {
     if (j < 0 || j > n - 1) return -1;
     unsigned a = (unsigned)(k[i] & 0x3fffffffull), b = (unsigned)(k[j] & 0x3fffffffull);
@@ -293,7 +297,8 @@ static __global__ void k_karras_build(Forest F, const unsigned long long* __rest
                                       const int* __restrict__ vals, TNode* __restrict__ nodes,
                                       int* __restrict__ nparent, int* __restrict__ lparent,
                                       int* __restrict__ leaf_tri, unsigned* __restrict__ visits,
-                                      int2* __restrict__ nrange, int* __restrict__ status) {
+                                      int2* __restrict__ nrange, int2* __restrict__ ntop, int* __restrict__ top_node,
+                                      int* __restrict__ top_index, int* __restrict__ status) {
     const int M = forest_size(F);
     const int total_internal = __ldg(F.voff + M) - M;
     for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < total_internal; gi += gridDim.x * blockDim.x) {
@@ -348,6 +353,12 @@ static __global__ void k_karras_build(Forest F, const unsigned long long* __rest
         nrange[po + i] = make_int2(lo, hi);
         visits[po + i] = 0u;
         if (i == 0) nparent[po] = -1;
+        if (refit_crosses(make_int2(lo, hi))) {
+            // the mesh's nodes above the refit's blocks, in any order
+            const int f = atomicAdd(&ntop[__ldg(F.sid + m)].x, 1);
+            top_node[po + f] = i;
+            top_index[po + i] = f;
+        }
     }
 }
 
@@ -727,57 +738,69 @@ __device__ __forceinline__ void read_qslot(const QNode* qn, int code, float lo[3
 __device__ __forceinline__ float hmin4(float4 v) { return fminf(fminf(v.x, v.y), fminf(v.z, v.w)); }
 __device__ __forceinline__ float hmax4(float4 v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
 
-// Refit: every leaf writes its swept box (fp32, rounded outward) into its QNode slot and
-// climbs; at each binary node the second arrival (the one that finds the node's other
-// subtree done) unions the children and goes on, the first stops.  Two passes:
-//  * pass 1 (k_engine_refit_local): a block takes REFIT_THREADS consecutive leaf positions
-//    and refits every node whose leaf range lies inside them, in shared memory, round by
-//    round; an item whose parent reaches outside the block hands that arrival to pass 2
-//    through the frontier list;
-//  * pass 2 (k_engine_refit_front) finishes those climbs with device-scope fences, global
-//    arrival counters and L2 reads.  The global counters only ever grow and the arrival
-//    that finds an odd count is the second one, so they are never cleared (a node refit in
-//    pass 1 leaves its counter alone).  The kernel boundary makes every box written in
-//    pass 1 visible to pass 2.
-// Most nodes lie inside one block's range, so most of the refit is shared-memory work
-// instead of device fences and L2 round trips.  Meshes with MF_DONE set in mflags (when
-// given) are skipped.
-static constexpr int REFIT_THREADS = 256;
+// Refit: every leaf's swept box (fp32, rounded outward) into its QNode slot, then bottom-up the
+// box of every even-depth node into its own, in two passes:
+//  * pass 1 (k_engine_refit_local): a block takes REFIT_THREADS consecutive leaf positions of a
+//    mesh and refits every node whose leaf range lies inside them, in shared memory, round by
+//    round;
+//  * pass 2 (k_engine_refit_top): the nodes above the blocks ("top" nodes, some nine a block), one
+//    block of threads a mesh, again in shared memory, level by level in an order that the build
+//    lays down (k_refit_plan).
+// A mesh with more top nodes than pass 2 holds (TOP_CAP) is finished by climbs instead: in pass 1
+// an item whose parent is a top node hands that arrival over through the frontier list, and at
+// each node the second arrival (the one that finds the global counter odd, and so the node's
+// other subtree done) unions the children and goes on, with device-scope fences and L2 reads.
+// The counters only ever grow, so they are never cleared.  The kernel boundary makes every
+// box written in pass 1 visible to pass 2.
+// Meshes with MF_DONE set in mflags (when given) are skipped.
+static constexpr int TOP_CAP = 7680;           // (215 KB of shared memory: meshes of some 220,000 triangles)
+static constexpr int TOP_THREADS = 1024;
+static constexpr int TOP_CLUSTER = 4;          // blocks of a mesh (8: 105 against 88 us on 64 meshes, 13 against 14 served)
+static constexpr int TOP_LEVELS = 64;          // levels above the blocks (a tree has at most 62)
 
-// pass 1: a block's leaf positions [base, base + REFIT_THREADS) and the internal nodes of
-// each mesh whose leaf range lies inside them ("local" nodes; a node's index lies in its
-// range, so these are the nodes at the same positions).  The boxes live in shared memory,
-// indexed by position - base: the leaves' from the soups, the local nodes' computed in
-// rounds (a node whose two children were done in earlier rounds takes the union of their
-// boxes; fminf / fmaxf skip NaN, so the order of the unions does not matter).  Then every
-// leaf and every local even-depth node writes its box into its QNode slot, and each whose
-// parent is not local hands that arrival to pass 2 through the frontier list.
+// The chunks of pass 1 over the active table, numbered with at most one empty number a mesh:
+// mesh m's first is voff[m] / REFIT_THREADS + m.
+__device__ __forceinline__ int refit_chunk_mesh(const Forest& F, int M, int g) {
+    int lo = 0, hi = M - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(F.voff + mid) / REFIT_THREADS + mid <= g) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// pass 1: leaf positions [blo, blo + REFIT_THREADS) of a mesh and the internal nodes whose leaf
+// range lies inside them ("local" nodes; a node's index lies in its range, so these are the nodes
+// at the same positions).  The boxes live in shared memory, indexed by position - blo: the
+// leaves' from the soups, the local nodes' computed in rounds (a node whose two children were
+// done in earlier rounds takes the union of their boxes; fminf / fmaxf skip NaN, so the order
+// of the unions does not matter).  Then every leaf and every local even-depth node writes its
+// box into its QNode slot.
 template <class T>
 __global__ void __launch_bounds__(REFIT_THREADS)
 k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x1, const int* __restrict__ leaf_tri,
                      const int* __restrict__ lparent, const int* __restrict__ nparent,
                      const int* __restrict__ qcode, const int* __restrict__ qleaf, const int2* __restrict__ nrange,
-                     const TNode* __restrict__ nodes, QNode* qnodes, int2* __restrict__ front, int front_cap,
-                     const int* __restrict__ mflags, WsHeader* hdr) {
+                     const TNode* __restrict__ nodes, QNode* qnodes, const int2* __restrict__ ntop,
+                     int2* __restrict__ front, int front_cap, const int* __restrict__ mflags, WsHeader* hdr) {
     __shared__ float s_llo[3][REFIT_THREADS], s_lhi[3][REFIT_THREADS];    // leaf boxes
     __shared__ float s_nlo[3][REFIT_THREADS], s_nhi[3][REFIT_THREADS];    // local node boxes
     __shared__ unsigned short s_done[REFIT_THREADS];    // round a local node was done in (0: not yet)
     const int M = forest_size(F);
-    const int total = __ldg(F.voff + M);
+    const int chunks = M > 0 ? __ldg(F.voff + M) / REFIT_THREADS + M : 0;
     const int t = threadIdx.x;
-    for (int base = blockIdx.x * REFIT_THREADS; base < total; base += gridDim.x * REFIT_THREADS) {
-        const int v = base + t;
-        bool live = false, node_local = false;
-        int m = 0, vo = 0, po = 0, n = 0, p = 0, cl = 0, cr = 0;
-        if (v < total) {
-            m = find_mesh(F.voff, M, v, 0);
-            vo = __ldg(F.voff + m);
-            po = __ldg(F.poff + m);
-            n = __ldg(F.voff + m + 1) - vo;
-            p = v - vo;
-            live = n >= 2 && !(mflags && (__ldg(mflags + __ldg(F.sid + m)) & MF_DONE));
-        }
-        const int blo = base - vo, bhi = base + REFIT_THREADS - 1 - vo;     // the block in mesh positions
+    for (int g = blockIdx.x; g < chunks; g += gridDim.x) {
+        const int m = refit_chunk_mesh(F, M, g);
+        const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
+        const int sid = __ldg(F.sid + m);
+        const int blo = (g - (vo / REFIT_THREADS + m)) * REFIT_THREADS;
+        // (an empty number, a mesh that has stopped: the whole block)
+        if (blo >= n || n < 2 || (mflags && (__ldg(mflags + sid) & MF_DONE))) continue;
+        const bool climbs = __ldg(&ntop[sid].x) > TOP_CAP;
+        const int p = blo + t;
+        bool live = p < n, node_local = false;
+        int cl = 0, cr = 0;
         if (live) {
             // the leaf at position p
             const int tri = __ldg(leaf_tri + po + p);
@@ -798,7 +821,7 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
             // the internal node at position p, when its range lies inside the block
             if (live && p < n - 1) {
                 const int2 r = __ldg(nrange + po + p);
-                if (r.x >= blo && r.y <= bhi) {
+                if (!refit_crosses(r)) {
                     const int4 d = __ldg(&nodes[po + p].d);
                     cl = d.x;
                     cr = d.y;
@@ -809,9 +832,9 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
         }
         s_done[t] = 0;
         __syncthreads();
-        // rounds: children indices (position - base) of a local node lie in the block
-        const int il = node_local ? (cl < 0 ? vo + ~cl : vo + cl) - base : 0;
-        const int ir = node_local ? (cr < 0 ? vo + ~cr : vo + cr) - base : 0;
+        // rounds: children indices (position - blo) of a local node lie in the block
+        const int il = node_local ? ((cl < 0 ? ~cl : cl) - blo) & (REFIT_THREADS - 1) : 0;
+        const int ir = node_local ? ((cr < 0 ? ~cr : cr) - blo) & (REFIT_THREADS - 1) : 0;
         bool pending = node_local;
 #pragma unroll 1
         for (int round = 1; round <= REFIT_THREADS; ++round) {
@@ -844,21 +867,19 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
                 const float hi[3] = {s_lhi[0][t], s_lhi[1][t], s_lhi[2][t]};
                 write_qslot(qn, lq, lo, hi);
             }
-            // each item whose parent is not local hands the arrival at the parent to pass 2
-            for (int item = 0; item < 2; ++item) {
-                if (item == 1 && (!node_local || pending)) break;
-                if (item == 1) {
-                    const int qc = __ldg(qcode + po + p);
-                    if (qc >= 0) {
-                        if ((qc >> 2) >= n - 1) {
-                            atomicOr(&hdr->status, ST_MALFORMED_TREE);
-                        } else {
-                            const float lo[3] = {s_nlo[0][t], s_nlo[1][t], s_nlo[2][t]};
-                            const float hi[3] = {s_nhi[0][t], s_nhi[1][t], s_nhi[2][t]};
-                            write_qslot(qn, qc, lo, hi);
-                        }
-                    }
+            const int qc = node_local && !pending ? __ldg(qcode + po + p) : QCODE_ROOT;
+            if (qc >= 0) {
+                if ((qc >> 2) >= n - 1) {
+                    atomicOr(&hdr->status, ST_MALFORMED_TREE);
+                } else {
+                    const float lo[3] = {s_nlo[0][t], s_nlo[1][t], s_nlo[2][t]};
+                    const float hi[3] = {s_nhi[0][t], s_nhi[1][t], s_nhi[2][t]};
+                    write_qslot(qn, qc, lo, hi);
                 }
+            }
+            // (climbs) each item whose parent is not local hands its arrival over
+            for (int item = 0; item < 2 && climbs; ++item) {
+                if (item == 1 && (!node_local || pending)) break;
                 const int code = __ldg((item ? nparent : lparent) + po + p);
                 if (code < 0) continue;                           // the root
                 const int par = code >> 1;
@@ -866,8 +887,7 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
                     atomicOr(&hdr->status, ST_MALFORMED_TREE);
                     continue;
                 }
-                const int2 r = __ldg(nrange + po + par);
-                if (r.x >= blo && r.y <= bhi) continue;           // a local parent: done here
+                if (!refit_crosses(__ldg(nrange + po + par))) continue;    // a local parent: done here
                 const int f = atomicAdd(&hdr->front, 1);
                 if (f < front_cap) front[f] = make_int2(m, code);
                 else atomicOr(&hdr->status, ST_MALFORMED_TREE);
@@ -877,10 +897,227 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
     }
 }
 
-// pass 2: the climbs handed over by pass 1, from the node they reached (global protocol)
-static __global__ void k_engine_refit_front(Forest F, const int* __restrict__ nparent, const int* __restrict__ qcode,
-                                            QNode* qnodes, unsigned* visits, const int2* __restrict__ front,
-                                            int front_cap, WsHeader* hdr) {
+// The order of pass 2, laid down with the topology: the top nodes of a mesh by height above the
+// blocks (counting sort; a height is found in rounds, one more than the children's), each with
+// where its children's boxes are and its own slot code.  A child below comes from slots that
+// pass 1 writes: its own (a leaf, an even-depth node), or its two children's (an odd-depth
+// node, TOP_PAIR); a child above is ~ its place in the order.  ntop[sid] = (top nodes, levels),
+// level l's places from top_index[po + l].
+static constexpr int TOP_PAIR = 1 << 30;
+struct PlanShared {
+    int node[TOP_CAP];
+    int below[2][TOP_CAP];               // where the children's boxes are
+    unsigned short dep[2][TOP_CAP];      // the children that are top nodes (TOP_CAP: none)
+    unsigned short place[TOP_CAP];
+    unsigned char height[TOP_CAP];       // 0: not found yet
+    int start[TOP_LEVELS + 1];
+};
+static_assert(TOP_CAP < 65536, "top node indices are 16-bit");
+static __global__ void __launch_bounds__(TOP_THREADS)
+k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ qcode, const int* __restrict__ qleaf,
+             const int2* __restrict__ nrange, int2* __restrict__ ntop, int* __restrict__ top_node,
+             int* __restrict__ top_index, int2* __restrict__ top_child, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    PlanShared& S = *reinterpret_cast<PlanShared*>(smem);
+    const int M = forest_size(F);
+    for (int m = blockIdx.x; m < M; m += gridDim.x) {
+        const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
+        const int sid = __ldg(F.sid + m);
+        const int nt = ntop[sid].x;
+        if (nt == 0 || nt > TOP_CAP) continue;         // (block-uniform)
+        // where child c's box is: a slot code, ~ (index of a top node), or TOP_PAIR | the first of two
+        // slots; the last code of all for a malformed tree
+        auto where = [&](int c) {
+            if (c >= 0 && c < n - 1 && refit_crosses(__ldg(nrange + po + c))) {
+                const int f = top_index[po + c];
+                if (f >= 0 && f < nt) return ~f;
+            } else {
+                int code = c < 0 ? (~c < n ? __ldg(qleaf + po + ~c) : -1) : (c < n - 1 ? __ldg(qcode + po + c) : -1);
+                int pair = 0;
+                if (c >= 0 && code <= QCODE_ODD) {
+                    code = QCODE_ODD - code;
+                    pair = TOP_PAIR;
+                }
+                if (code >= 0 && (code >> 2) < n - 1 && !(pair && (code & 3) > 2)) return code | pair;
+            }
+            atomicOr(status, ST_MALFORMED_TREE);
+            return 0;
+        };
+        if (threadIdx.x <= TOP_LEVELS) S.start[threadIdx.x] = 0;
+        for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
+            const int i = top_node[po + f];
+            const int4 d = __ldg(&nodes[po + i].d);
+            const int a = where(d.x), b = where(d.y);
+            S.node[f] = i;
+            S.below[0][f] = a;
+            S.below[1][f] = b;
+            S.dep[0][f] = (unsigned short)(a < 0 ? ~a : TOP_CAP);
+            S.dep[1][f] = (unsigned short)(b < 0 ? ~b : TOP_CAP);
+            S.height[f] = 0;
+        }
+        __syncthreads();
+        int levels = 0;
+#pragma unroll 1
+        for (int round = 1; round <= TOP_LEVELS; ++round) {
+            bool left = false;
+            for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
+                if (S.height[f]) continue;
+                const int a = S.dep[0][f], b = S.dep[1][f];
+                const int ha = a < TOP_CAP ? S.height[a] : 0, hb = b < TOP_CAP ? S.height[b] : 0;
+                if ((a < TOP_CAP && (ha == 0 || ha >= round)) || (b < TOP_CAP && (hb == 0 || hb >= round))) {
+                    left = true;
+                    continue;
+                }
+                S.height[f] = (unsigned char)round;
+                atomicAdd(&S.start[round], 1);
+            }
+            levels = round;
+            if (!__syncthreads_or(left)) break;
+            // (not reached by a tree: a cycle; its nodes join the last level)
+            if (round == TOP_LEVELS && left) {
+                atomicOr(status, ST_MALFORMED_TREE);
+                for (int f = threadIdx.x; f < nt; f += TOP_THREADS)
+                    if (!S.height[f]) {
+                        S.height[f] = TOP_LEVELS;
+                        atomicAdd(&S.start[TOP_LEVELS], 1);
+                    }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int l = 1; l <= TOP_LEVELS; ++l) S.start[l] += S.start[l - 1];       // ends of the levels
+        __syncthreads();
+        if (threadIdx.x <= levels) top_index[po + min(threadIdx.x, n - 1)] = S.start[threadIdx.x];
+        if (threadIdx.x == 0) ntop[sid].y = levels;
+        __syncthreads();
+        for (int f = threadIdx.x; f < nt; f += TOP_THREADS)
+            S.place[f] = (unsigned short)atomicAdd(&S.start[S.height[f] - 1], 1);
+        __syncthreads();
+        for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
+            const int at = S.place[f], a = S.dep[0][f], b = S.dep[1][f];
+            top_child[po + at] = make_int2(a < TOP_CAP ? ~(int)S.place[a] : S.below[0][f],
+                                           b < TOP_CAP ? ~(int)S.place[b] : S.below[1][f]);
+            top_node[po + at] = __ldg(qcode + po + S.node[f]);
+        }
+        __syncthreads();
+    }
+}
+
+// pass 2, a cluster of TOP_CLUSTER blocks a mesh: all of them gather the boxes of the top nodes'
+// children below, into the first block's shared memory (one block alone is bound by its SM's
+// scattered 4-byte loads: 153 us on the 64 meshes); that block goes up the levels with a barrier
+// each; all of them write the even-depth nodes' slots.
+// Climbing took some two microseconds a level for its fence, its atomic and its reads through
+// L2 (20 levels above the blocks on 55,000 triangles): 5 small meshes 31 -> 8 us, 12 meshes 50
+// -> 16 us, 64 meshes 117 -> 88 us, ten served folds 40 -> 14 us; the plan is 27 us of a build of
+// the 12 meshes.  What is left is the gather's latency, some 400 cycles a level, and a launch.
+struct TopShared {
+    float lo[3][TOP_CAP], hi[3][TOP_CAP];
+    unsigned short dep[2][TOP_CAP];      // the children that are top nodes (TOP_CAP: none)
+};
+static __global__ void __cluster_dims__(TOP_CLUSTER, 1, 1) __launch_bounds__(TOP_THREADS)
+k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restrict__ qcode, QNode* qnodes,
+                   const int2* __restrict__ ntop, const int* __restrict__ top_node, const int* __restrict__ top_index,
+                   const int2* __restrict__ top_child, unsigned* visits, const int2* __restrict__ front,
+                   int front_cap, const int* __restrict__ mflags, WsHeader* hdr) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_end[TOP_LEVELS + 1];
+    const cg::cluster_group cluster = cg::this_cluster();
+    TopShared& S = *reinterpret_cast<TopShared*>(cluster.map_shared_rank(smem, 0));      // the first block's
+    const int rank = (int)cluster.block_rank();
+    // (warp by warp over the blocks, so that a small mesh's nodes spread over them too)
+    const int t0 = ((threadIdx.x >> 5) * TOP_CLUSTER + rank) * 32 + (threadIdx.x & 31);
+    const int M = forest_size(F);
+    for (int m = blockIdx.x / TOP_CLUSTER; m < M; m += gridDim.x / TOP_CLUSTER) {
+        const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
+        const int sid = __ldg(F.sid + m);
+        const int2 plan = __ldg(ntop + sid);
+        const int nt = plan.x, levels = min(plan.y, TOP_LEVELS);
+        if (nt == 0 || nt > TOP_CAP || (mflags && (__ldg(mflags + sid) & MF_DONE))) continue;     // (cluster-uniform)
+        QNode* qn = qnodes + po;
+        if (rank == 0 && threadIdx.x <= levels) s_end[threadIdx.x] = min(__ldg(top_index + po + min(threadIdx.x, n - 1)), nt);
+        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) {
+            const int2 ch = __ldg(top_child + po + f);
+            float lo[3], hi[3];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                lo[x] = __int_as_float(0x7f800000);
+                hi[x] = __int_as_float(0xff800000);
+            }
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int c = side ? ch.y : ch.x;
+                S.dep[side][f] = (unsigned short)(c < 0 ? min(~c, nt - 1) : TOP_CAP);
+                if (c < 0) continue;
+                const int code = c & ~TOP_PAIR;
+                float l[3], h[3];
+                read_qslot(qn, code, l, h);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    lo[x] = fminf(lo[x], l[x]);
+                    hi[x] = fmaxf(hi[x], h[x]);
+                }
+                if (c & TOP_PAIR) {
+                    read_qslot(qn, code + 1, l, h);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        lo[x] = fminf(lo[x], l[x]);
+                        hi[x] = fmaxf(hi[x], h[x]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                S.lo[x][f] = lo[x];
+                S.hi[x][f] = hi[x];
+            }
+        }
+        cluster.sync();
+        if (rank == 0) {
+            TopShared& L = *reinterpret_cast<TopShared*>(smem);
+            // the union of node f's boxes below and of its children above
+            auto unite = [&](int f) {
+                const int a = L.dep[0][f], b = L.dep[1][f];
+                const int ca = a < TOP_CAP ? a : f, cb = b < TOP_CAP ? b : f;
+                float lo[3], hi[3];
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    lo[x] = fminf(L.lo[x][f], fminf(L.lo[x][ca], L.lo[x][cb]));
+                    hi[x] = fmaxf(L.hi[x][f], fmaxf(L.hi[x][ca], L.hi[x][cb]));
+                }
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    L.lo[x][f] = lo[x];
+                    L.hi[x][f] = hi[x];
+                }
+            };
+            // the first level has no child above; the block takes the wide levels, a warp the rest,
+            // which has no use for the block's barrier
+            int l = 1;
+#pragma unroll 1
+            for (; l < levels && s_end[l + 1] - s_end[l] > 32; ++l) {
+                for (int f = s_end[l] + threadIdx.x; f < s_end[l + 1]; f += TOP_THREADS) unite(f);
+                __syncthreads();
+            }
+            if (threadIdx.x < 32) {
+#pragma unroll 1
+                for (; l < levels; ++l) {
+                    for (int f = s_end[l] + threadIdx.x; f < s_end[l + 1]; f += 32) unite(f);
+                    __syncwarp();
+                }
+            }
+        }
+        cluster.sync();
+        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) {
+            const int qc = __ldg(top_node + po + f);
+            if (qc < 0) continue;
+            const float lo[3] = {S.lo[0][f], S.lo[1][f], S.lo[2][f]}, hi[3] = {S.hi[0][f], S.hi[1][f], S.hi[2][f]};
+            if ((qc >> 2) >= n - 1) atomicOr(&hdr->status, ST_MALFORMED_TREE);
+            else write_qslot(qn, qc, lo, hi);
+        }
+        cluster.sync();      // (the next mesh overwrites the boxes; no block leaves before they are read)
+    }
+    // the climbs of the meshes with too many top nodes
     const int nf = min(*(volatile int*)&hdr->front, front_cap);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nf; i += gridDim.x * blockDim.x) {
         const int2 e = front[i];
@@ -1427,12 +1664,14 @@ __global__ void k_gather_soup(Forest F, VertTable vt, const int* __restrict__ co
 // Per-mesh resets over a table
 
 // centroid bounds of every mesh in the table to (empty): min words high, max words low
-static __global__ void k_reset_bounds(Forest F, unsigned* __restrict__ bounds) {
+// and no top nodes
+static __global__ void k_reset_bounds(Forest F, unsigned* __restrict__ bounds, int2* __restrict__ ntop) {
     const int M = forest_size(F);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         unsigned* b = bounds + 6 * __ldg(F.sid + m);
         b[0] = b[1] = b[2] = 0xffffffffu;
         b[3] = b[4] = b[5] = 0u;
+        ntop[__ldg(F.sid + m)] = make_int2(0, 0);
     }
 }
 
