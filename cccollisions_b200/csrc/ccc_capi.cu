@@ -193,34 +193,27 @@ int run_broad_phase(const void* bboxes, const int64_t* tree, const uint8_t* mask
     int cap = (int)P.L.cand_cap;
     if (P.L.wide) {
         QNode* nodes = (QNode*)P.nodes;
-        CCC_LAUNCH("k_import_nodes", s, k_import_wide<T><<<grid_for(internal, 128), 128, 0, s>>>(
-            (int)F, M, bb, tr, nodes, P.visits, P.rmk, P.table, P.moff, P.hdr));
+        CCC_LAUNCH("k_import_nodes", s, launch_chain(grid_for(internal, 128), 128, 0, s, k_import_wide<T>, (int)F, M, bb, tr, nodes, P.visits, P.rmk, P.table, P.moff, P.hdr));
         CCC_LAUNCH_CHECK();
-        CCC_LAUNCH("k_import_rightmost", s, k_import_rightmost_wide<<<grid_for(total, 256), 256, 0, s>>>(
-            (int)F, total, tr, P.visits, P.rmk, P.hdr));
+        CCC_LAUNCH("k_import_rightmost", s, launch_chain(grid_for(total, 256), 256, 0, s, k_import_rightmost_wide, (int)F, total, tr, P.visits, P.rmk, P.hdr));
         CCC_LAUNCH_CHECK();
         const int g = std::min(grid_for(total, WALK_WARPS), num_sms() * 8);
         with_walk<T>(mask != nullptr, exact_f32, [&](auto masked, auto exact) {
-            CCC_LAUNCH("k_traverse", s, k_walk_tensors<T, masked.value, exact.value><<<g, WALK_THREADS, 0, s>>>(
-                nodes, bb, tr, mask, P.rmk, (int)F, P.forest, th, P.cand, cap, P.hdr));
+            CCC_LAUNCH("k_traverse", s, launch_chain(g, WALK_THREADS, 0, s, k_walk_tensors<T, masked.value, exact.value>, nodes, bb, tr, mask, P.rmk, (int)F, P.forest, th, P.cand, cap, P.hdr));
         });
         CCC_LAUNCH_CHECK();
         return CCC_OK;
     }
     TNode* nodes = (TNode*)P.nodes;
-    CCC_LAUNCH("k_uniform_offsets", s, k_uniform_offsets<<<grid_for(B + 1, 256), 256, 0, s>>>(
-        P.table, P.moff, P.table + 4, P.table + 4 + B, M, (int)F));
+    CCC_LAUNCH("k_uniform_offsets", s, launch_chain(grid_for(B + 1, 256), 256, 0, s, k_uniform_offsets, P.table, P.moff, P.table + 4, P.table + 4 + B, M, (int)F));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_import_nodes", s, k_import_nodes<T><<<grid_for(internal, 256), 256, 0, s>>>(
-        P.moff, M, internal, bb, tr, nodes, &P.hdr->status));
+    CCC_LAUNCH("k_import_nodes", s, launch_chain(grid_for(internal, 256), 256, 0, s, k_import_nodes<T>, P.moff, M, internal, bb, tr, nodes, &P.hdr->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_import_rightmost", s, k_import_rightmost<<<grid_for(total, 256), 256, 0, s>>>(
-        P.moff, M, total, tr, nodes, P.visits, P.rmk, &P.hdr->status));
+    CCC_LAUNCH("k_import_rightmost", s, launch_chain(grid_for(total, 256), 256, 0, s, k_import_rightmost, P.moff, M, total, tr, nodes, P.visits, P.rmk, &P.hdr->status));
     CCC_LAUNCH_CHECK();
     const TensorLeaves<T> lv{bb, tr};
     with_walk<T>(mask != nullptr, exact_f32, [&](auto masked, auto exact) {
-        CCC_LAUNCH("k_traverse", s, k_traverse<T, masked.value, exact.value><<<grid_for(total, TRAV_THREADS), TRAV_THREADS, 0, s>>>(
-            nodes, lv, P.forest, mask, th, P.cand, cap, P.hdr, nullptr));
+        CCC_LAUNCH("k_traverse", s, launch_chain(grid_for(total, TRAV_THREADS), TRAV_THREADS, 0, s, k_traverse<T, masked.value, exact.value, TensorLeaves<T>>, nodes, lv, P.forest, mask, th, P.cand, cap, P.hdr, nullptr));
     });
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -254,11 +247,9 @@ int bvh_impl(const void* tri, const void* tri_next, int64_t B, int64_t F, void* 
         const int log_threads = level == 0 ? 8 : 10;
         const int chunks = grid_for(blocks, 1 << log_threads);
         if (log_threads == 8)
-            CCC_LAUNCH("k_bvh_levels", s, k_bvh_levels<T, 8><<<(unsigned)(B * chunks), 1 << 8, 0, s>>>(
-                x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
+            CCC_LAUNCH("k_bvh_levels", s, launch_chain((unsigned)(B * chunks), 1 << 8, 0, s, k_bvh_levels<T, 8>, x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
         else
-            CCC_LAUNCH("k_bvh_levels", s, k_bvh_levels<T, 10><<<(unsigned)(B * chunks), 1 << 10, 0, s>>>(
-                x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
+            CCC_LAUNCH("k_bvh_levels", s, launch_chain((unsigned)(B * chunks), 1 << 10, 0, s, k_bvh_levels<T, 10>, x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
         CCC_LAUNCH_CHECK();
         level += log_threads;
     }
@@ -275,7 +266,7 @@ int static_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_
     T th = (T)(float)threshold;
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, th, is_f32<T>() && th == 0, P, s);
     if (rc) return rc;
-    CCC_LAUNCH("k_static_narrow", s, k_static_narrow<T><<<narrow_grid(), NARROW_THREADS, 0, s>>>(P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest,
+    CCC_LAUNCH("k_static_narrow", s, launch_chain(narrow_grid(), NARROW_THREADS, 0, s, k_static_narrow<T>, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest,
                                                                 th, (long long*)out, (int)max_collisions, P.mesh_cnt));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -291,12 +282,10 @@ int te_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_t B,
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, (T)0, is_f32<T>(), P, s);
     if (rc) return rc;
     if (OP == TE_COLLISIONS) {
-        CCC_WITH_LIB(CCC_LAUNCH("k_te_narrow", s, k_te_narrow<T, OP, LIBV><<<narrow_grid(), NARROW_THREADS, 0, s>>>(
-            P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest, (long long*)rows, (T*)coefs, (int*)masks,
+        CCC_WITH_LIB(CCC_LAUNCH("k_te_narrow", s, launch_chain(narrow_grid(), NARROW_THREADS, 0, s, k_te_narrow<T, OP, LIBV>, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest, (long long*)rows, (T*)coefs, (int*)masks,
             (int)max_collisions, P.mesh_cnt)));
     } else {
-        CCC_LAUNCH("k_te_narrow", s, k_te_narrow<T, OP, LIB_PORTABLE><<<narrow_grid(), NARROW_THREADS, 0, s>>>(
-            P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest, (long long*)rows, (T*)coefs, (int*)masks,
+        CCC_LAUNCH("k_te_narrow", s, launch_chain(narrow_grid(), NARROW_THREADS, 0, s, k_te_narrow<T, OP, LIB_PORTABLE>, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest, (long long*)rows, (T*)coefs, (int*)masks,
             (int)max_collisions, P.mesh_cnt));
     }
     CCC_LAUNCH_CHECK();
@@ -345,8 +334,7 @@ template <class T> CcdArgs<T> ccd_args(const Prepared& P, const void* x0, const 
 // the sub-test masks of the candidates, into the candidate buffer (MASK_PACK) or as rows
 template <class T, int USE>
 int run_masks(const Prepared& P, const CcdArgs<T>& A, long long* rows, int max_per_tri, cudaStream_t s) {
-    CCC_LAUNCH("k_ccd_mask", s, k_ccd_mask<T, USE><<<wave(P.L.cand_cap, STAGE_THREADS, 3), STAGE_THREADS, 0, s>>>(
-        P.cand, A.cand_cap, P.hdr, A.x0, A.x1, const_cast<unsigned short*>(A.masks), nullptr, P.forest, rows,
+    CCC_LAUNCH("k_ccd_mask", s, launch_chain(wave(P.L.cand_cap, STAGE_THREADS, 3), STAGE_THREADS, 0, s, k_ccd_mask<T, USE>, P.cand, A.cand_cap, P.hdr, A.x0, A.x1, const_cast<unsigned short*>(A.masks), nullptr, P.forest, rows,
         max_per_tri, P.mesh_cnt));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -395,7 +383,7 @@ int prox_impl(const void* bboxes, const int64_t* tree, const void* tri, int64_t 
     T th = (T)(float)threshold;
     rc = run_broad_phase<T>(bboxes, tree, nullptr, B, F, th, is_f32<T>() && th == 0, P, s);
     if (rc) return rc;
-    CCC_LAUNCH("k_prox_narrow", s, k_prox_narrow<T><<<narrow_grid(), NARROW_THREADS, 0, s>>>(P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest,
+    CCC_LAUNCH("k_prox_narrow", s, launch_chain(narrow_grid(), NARROW_THREADS, 0, s, k_prox_narrow<T>, P.cand, (int)P.L.cand_cap, P.hdr, (const T*)tri, P.forest,
                                                               th, (long long*)rows, (int)maxc, P.mesh_cnt));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -437,8 +425,7 @@ int from_rows_impl(const int64_t* rows, const void* roots, int64_t B, int64_t N,
     if (cudaMemsetAsync(hdr, 0, (char*)(mesh_cnt + B) - (char*)hdr, s) != cudaSuccess) return CCC_ERR_CUDA;
     if (B * N == 0) return CCC_OK;
     int g = (int)std::min<int64_t>(grid_for(B * N, NARROW_THREADS), (int64_t)narrow_grid());
-    CCC_WITH_LIB(CCC_LAUNCH("k_impulses_from_rows", s, k_impulses_from_rows<T, LIBV><<<g, NARROW_THREADS, 0, s>>>(
-        (const long long*)rows, (const T*)roots, (int)B, N, (int)F, (const T*)x0, (const T*)x1, (const T*)masses,
+    CCC_WITH_LIB(CCC_LAUNCH("k_impulses_from_rows", s, launch_chain(g, NARROW_THREADS, 0, s, k_impulses_from_rows<T, LIBV>, (const long long*)rows, (const T*)roots, (int)B, N, (int)F, (const T*)x0, (const T*)x1, (const T*)masses,
         (T*)dv, (T*)dx, (int*)cnt)));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -546,7 +533,7 @@ int ccc_fill(void* p0, int64_t b0, int64_t v0, void* p1, int64_t b1, int64_t v1,
     if (words == 0) return CCC_OK;
     cudaStream_t s = (cudaStream_t)stream;
     const int g = (int)std::min<int64_t>((words + 4 * 256 - 1) / (4 * 256), (int64_t)num_sms() * 16);
-    CCC_LAUNCH("k_fill", s, k_fill<<<g, 256, 0, s>>>(j[0], j[1], j[2]));
+    CCC_LAUNCH("k_fill", s, launch_chain(g, 256, 0, s, k_fill, j[0], j[1], j[2]));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
 }

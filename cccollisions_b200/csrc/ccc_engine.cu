@@ -281,14 +281,12 @@ inline int top_grid(const ccc_engine* e, int per) {
 
 // (hdr->front is 0 before it: a step clears the header, the build only that word)
 template <class T> int refit(ccc_engine* e, const Tables& t, const int* flags, cudaStream_t s) {
-    CCC_LAUNCH("k_engine_refit", s, k_engine_refit_local<T><<<refit_grid(e), REFIT_THREADS, 0, s>>>(
-        t.f, e->at<T>(e->L.x0), e->at<T>(e->L.x1), e->at<int>(e->L.leaf_tri), e->at<int>(e->L.lparent),
+    CCC_LAUNCH("k_engine_refit", s, launch_chain(refit_grid(e), REFIT_THREADS, 0, s, k_engine_refit_local<T>, t.f, e->at<T>(e->L.x0), e->at<T>(e->L.x1), e->at<int>(e->L.leaf_tri), e->at<int>(e->L.lparent),
         e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
         e->at<TNode>(e->L.nodes), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop), e->at<int2>(e->L.front),
         (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_engine_refit_front", s, k_engine_refit_top<<<top_grid(e, TOP_CLUSTER), TOP_THREADS, sizeof(TopShared), s>>>(
-        t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
+    CCC_LAUNCH("k_engine_refit_front", s, launch_chain(top_grid(e, TOP_CLUSTER), TOP_THREADS, sizeof(TopShared), s, k_engine_refit_top, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
         e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
         e->at<unsigned>(e->L.visits), e->at<int2>(e->L.front), (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
@@ -299,24 +297,19 @@ template <class T> int refit(ccc_engine* e, const Tables& t, const int* flags, c
 template <class T> int traverse(ccc_engine* e, const Tables& t, const int* flags, const int4* vid, cudaStream_t s) {
     int g = num_sms() * SHAPES[e->shape].trav;
     if (SHAPES[e->shape].warp)
-        CCC_LAUNCH("k_traverse", s, k_traverse_w<<<g, TRAV_THREADS, 0, s>>>(
-            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+        CCC_LAUNCH("k_traverse", s, launch_chain(g, TRAV_THREADS, 0, s, k_traverse_w, e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     else if (SHAPES[e->shape].stage == 0 && vid)
-        CCC_LAUNCH("k_traverse", s, k_traverse_walk<true><<<g, WALK_THREADS, 0, s>>>(
-            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+        CCC_LAUNCH("k_traverse", s, launch_chain(g, WALK_THREADS, 0, s, k_traverse_walk<true>, e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     else if (SHAPES[e->shape].stage == 0)
-        CCC_LAUNCH("k_traverse", s, k_traverse_walk<false><<<g, WALK_THREADS, 0, s>>>(
-            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+        CCC_LAUNCH("k_traverse", s, launch_chain(g, WALK_THREADS, 0, s, k_traverse_walk<false>, e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     else if (SHAPES[e->shape].stage == 1)
-        CCC_LAUNCH("k_traverse", s, k_traverse_q<1><<<g, TRAV_THREADS, 0, s>>>(
-            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+        CCC_LAUNCH("k_traverse", s, launch_chain(g, TRAV_THREADS, 0, s, k_traverse_q<1>, e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     else
-        CCC_LAUNCH("k_traverse", s, k_traverse_q<2><<<g, TRAV_THREADS, 0, s>>>(
-            e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
+        CCC_LAUNCH("k_traverse", s, launch_chain(g, TRAV_THREADS, 0, s, k_traverse_q<2>, e->at<QNode>(e->L.qnodes), e->at<int>(e->L.qleaf), e->at<int>(e->L.leaf_tri), t.f, e->at<int2>(e->L.cand),
             (int)e->L.cand_cap, e->hdr(), flags, vid));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -333,22 +326,17 @@ template <class T> int weld(ccc_engine* e, const Tables& t, cudaStream_t s) {
     int* vidc = e->at<int>(L.vidc);
     int* cnt = e->at<int>(L.wcnt);
     int* fan_end = e->at<int>(L.fan_end);
-    CCC_LAUNCH("k_weld_insert", s, k_weld_insert<T><<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, x0, x1, e->at<int>(L.wtab), vidc, cnt, e->hdr()));
+    CCC_LAUNCH("k_weld_insert", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_weld_insert<T>, t.f, x0, x1, e->at<int>(L.wtab), vidc, cnt, e->hdr()));
     CCC_LAUNCH_CHECK();
     // (the table is not read after k_weld_insert: its space holds the classes' first entries)
     int* fan_start = e->at<int>(L.wtab);
-    CCC_LAUNCH("k_weld_alloc", s, k_weld_alloc<<<item_grid(), WELD_THREADS, 0, s>>>(
-        t.f, vidc, cnt, fan_start, fan_end, e->hdr()));
+    CCC_LAUNCH("k_weld_alloc", s, launch_chain(item_grid(), WELD_THREADS, 0, s, k_weld_alloc, t.f, vidc, cnt, fan_start, fan_end, e->hdr()));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_weld_fill", s, k_weld_fill<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, vidc, fan_start, fan_end, e->at<int4>(L.fan_tmp)));
+    CCC_LAUNCH("k_weld_fill", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_weld_fill, t.f, vidc, fan_start, fan_end, e->at<int4>(L.fan_tmp)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_weld_rank", s, k_weld_rank<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, vidc, fan_start, cnt, e->at<int4>(L.fan_tmp), e->at<int4>(L.fan)));
+    CCC_LAUNCH("k_weld_rank", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_weld_rank, t.f, vidc, fan_start, cnt, e->at<int4>(L.fan_tmp), e->at<int4>(L.fan)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_weld_tri", s, k_weld_tri<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, vidc, cnt, fan_start, e->at<int4>(L.fan), e->at<int4>(L.vid4), e->at<int4>(L.twin4),
+    CCC_LAUNCH("k_weld_tri", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_weld_tri, t.f, vidc, cnt, fan_start, e->at<int4>(L.fan), e->at<int4>(L.vid4), e->at<int4>(L.twin4),
         e->at<int4>(L.third4)));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -363,12 +351,10 @@ Weld engine_weld(ccc_engine* e) {
 
 // the sub-tests of every candidate pair, for the narrow phase (k_ccd_stage_*)
 template <class T> int stage(ccc_engine* e, cudaStream_t s) {
-    CCC_LAUNCH("k_ccd_stage_mask", s, k_ccd_stage_mask<T><<<num_sms() * 3, STAGE_THREADS, 0, s>>>(
-        e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), e->at<T>(e->L.x0), e->at<T>(e->L.x1), engine_weld(e),
+    CCC_LAUNCH("k_ccd_stage_mask", s, launch_chain(num_sms() * 3, STAGE_THREADS, 0, s, k_ccd_stage_mask<T>, e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), e->at<T>(e->L.x0), e->at<T>(e->L.x1), engine_weld(e),
         e->at<int4>(e->L.live), e->at<int4>(e->L.pending)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_ccd_stage_pending", s, k_ccd_stage_pending<<<num_sms() * 8, STAGE_THREADS, 0, s>>>(
-        (int)e->L.cand_cap, e->hdr(), engine_weld(e), e->at<int4>(e->L.pending), e->at<int4>(e->L.live)));
+    CCC_LAUNCH("k_ccd_stage_pending", s, launch_chain(num_sms() * 8, STAGE_THREADS, 0, s, k_ccd_stage_pending, (int)e->L.cand_cap, e->hdr(), engine_weld(e), e->at<int4>(e->L.pending), e->at<int4>(e->L.live)));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
 }
@@ -421,8 +407,7 @@ template <class T> int ccd_step(ccc_engine* e, cudaStream_t s) {
             g, s, A, CornerSink<T>{})));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_ccd_expand", s, k_ccd_expand<T><<<num_sms() * 8, EXPAND_THREADS, 0, s>>>(
-        e->hdr(), engine_weld(e), t.f, e->at<long long>(e->L.rows), e->at<T>(e->L.times), (int)e->maxcol,
+    CCC_LAUNCH("k_ccd_expand", s, launch_chain(num_sms() * 8, EXPAND_THREADS, 0, s, k_ccd_expand<T>, e->hdr(), engine_weld(e), t.f, e->at<long long>(e->L.rows), e->at<T>(e->L.times), (int)e->maxcol,
         e->at<int>(e->L.mesh_cnt)));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
@@ -445,8 +430,7 @@ template <class T> int loop_step(ccc_engine* e, int max_iter, cudaStream_t s) {
     W.expand = e->at<int4>(e->L.pending);
     W.expand_cap = (int)e->L.cand_cap;
     const CcdArgs<T> A = engine_args<T>(e, t.f, W);
-    CCC_LAUNCH("k_ccd_mask", s, k_ccd_mask<T, MASK_LIST><<<num_sms() * 3, STAGE_THREADS, 0, s>>>(
-        e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), A.x0, A.x1, nullptr, e->at<int4>(e->L.live), t.f,
+    CCC_LAUNCH("k_ccd_mask", s, launch_chain(num_sms() * 3, STAGE_THREADS, 0, s, k_ccd_mask<T, MASK_LIST>, e->at<int2>(e->L.cand), (int)e->L.cand_cap, e->hdr(), A.x0, A.x1, nullptr, e->at<int4>(e->L.live), t.f,
         nullptr, 0, A.mesh_counters));
     CCC_LAUNCH_CHECK();
     LoopSink<T> sink{e->at<T>(e->L.masses), e->at<int>(e->L.faces), t.vt, e->at<long long>(e->L.acc), contacts};
@@ -460,14 +444,11 @@ template <class T> int loop_step(ccc_engine* e, int max_iter, cudaStream_t s) {
         num_sms() * 8, s, A, sink)));
     if (le != cudaSuccess) return CCC_ERR_CUDA;
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_loop_update", s, k_loop_update<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(
-        t.f, contacts, e->at<int>(e->L.iters), flags, max_iter));
+    CCC_LAUNCH("k_loop_update", s, launch_chain(grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s, k_loop_update, t.f, contacts, e->at<int>(e->L.iters), flags, max_iter));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_loop_apply", s, k_loop_apply<T><<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, t.vt, contacts, e->at<long long>(e->L.acc), e->at<T>(e->L.verts1), e->at<T>(e->L.vel)));
+    CCC_LAUNCH("k_loop_apply", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_loop_apply<T>, t.f, t.vt, contacts, e->at<long long>(e->L.acc), e->at<T>(e->L.verts1), e->at<T>(e->L.vel)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_gather_soup", s, k_gather_soup<T><<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, t.vt, contacts, e->at<int>(e->L.faces), e->at<T>(e->L.verts1), e->at<T>(e->L.x1), &e->hdr()->status));
+    CCC_LAUNCH("k_gather_soup", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_gather_soup<T>, t.f, t.vt, contacts, e->at<int>(e->L.faces), e->at<T>(e->L.verts1), e->at<T>(e->L.x1), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
     return CCC_OK;
 }
@@ -477,8 +458,7 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     if (ntri == 0) return CCC_OK;
     Tables t = e->building();
     unsigned* bounds = e->at<unsigned>(e->L.bounds);
-    CCC_LAUNCH("k_reset_bounds", s, k_reset_bounds<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(
-        t.f, bounds, e->at<int2>(e->L.ntop)));
+    CCC_LAUNCH("k_reset_bounds", s, launch_chain(grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s, k_reset_bounds, t.f, bounds, e->at<int2>(e->L.ntop)));
     CCC_LAUNCH_CHECK();
     unsigned long long* keys[2] = {e->at<unsigned long long>(e->L.keys0), e->at<unsigned long long>(e->L.keys1)};
     int* vals[2] = {e->at<int>(e->L.vals0), e->at<int>(e->L.vals1)};
@@ -486,11 +466,11 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     // (8 + 4 bytes an item), which the sort first writes after k_morton
     float2* cxy = reinterpret_cast<float2*>(keys[1]);
     float* cz = reinterpret_cast<float*>(vals[1]);
-    CCC_LAUNCH("k_mesh_bounds", s, k_mesh_bounds<T><<<item_grid(), ITEM_THREADS, 0, s>>>(t.f, e->at<T>(e->L.x0),
+    CCC_LAUNCH("k_mesh_bounds", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_mesh_bounds<T>, t.f, e->at<T>(e->L.x0),
                                                                                         e->at<T>(e->L.x1), bounds,
                                                                                         cxy, cz));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_morton", s, k_morton<<<item_grid(), ITEM_THREADS, 0, s>>>(t.f, cxy, cz, bounds, keys[0], vals[0]));
+    CCC_LAUNCH("k_morton", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_morton, t.f, cxy, cz, bounds, keys[0], vals[0]));
     CCC_LAUNCH_CHECK();
     int mesh_bits = 0;
     while (((int64_t)1 << mesh_bits) < nb) ++mesh_bits;
@@ -501,31 +481,27 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
-        CCC_LAUNCH("k_radix_hist", s, k_radix_hist<<<nblk, SORT_THREADS, 0, s>>>(keys[cur], n, shift, hist, nblk));
+        CCC_LAUNCH("k_radix_hist", s, launch_chain(nblk, SORT_THREADS, 0, s, k_radix_hist, keys[cur], n, shift, hist, nblk));
         CCC_LAUNCH_CHECK();
         int* rowtot = hist + e->L.hist_len;
-        CCC_LAUNCH("k_radix_rowscan", s, k_radix_rowscan<<<256, SORT_THREADS, 0, s>>>(hist, nblk, rowtot));
+        CCC_LAUNCH("k_radix_rowscan", s, launch_chain(256, SORT_THREADS, 0, s, k_radix_rowscan, hist, nblk, rowtot));
         CCC_LAUNCH_CHECK();
-        CCC_LAUNCH("k_radix_scatter", s, k_radix_scatter<<<nblk, SORT_THREADS, 0, s>>>(keys[cur], vals[cur], keys[1 - cur],
+        CCC_LAUNCH("k_radix_scatter", s, launch_chain(nblk, SORT_THREADS, 0, s, k_radix_scatter, keys[cur], vals[cur], keys[1 - cur],
                                                                                    vals[1 - cur], n, shift, hist,
                                                                                    rowtot, nblk));
         CCC_LAUNCH_CHECK();
         cur = 1 - cur;
     }
-    CCC_LAUNCH("k_karras_build", s, k_karras_build<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, keys[cur], vals[cur], e->at<TNode>(e->L.nodes), e->at<int>(e->L.nparent), e->at<int>(e->L.lparent),
+    CCC_LAUNCH("k_karras_build", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_karras_build, t.f, keys[cur], vals[cur], e->at<TNode>(e->L.nodes), e->at<int>(e->L.nparent), e->at<int>(e->L.lparent),
         e->at<int>(e->L.leaf_tri), e->at<unsigned>(e->L.visits), e->at<int2>(e->L.nrange), e->at<int2>(e->L.ntop),
         e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_qtree_depth", s, k_qtree_depth<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), &e->hdr()->status));
+    CCC_LAUNCH("k_qtree_depth", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_qtree_depth, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_qtree_slots", s, k_qtree_slots<<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<QNode>(e->L.qnodes),
+    CCC_LAUNCH("k_qtree_slots", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_qtree_slots, t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<QNode>(e->L.qnodes),
         &e->hdr()->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_refit_plan", s, k_refit_plan<<<top_grid(e, 1), TOP_THREADS, sizeof(PlanShared), s>>>(
-        t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
+    CCC_LAUNCH("k_refit_plan", s, launch_chain(top_grid(e, 1), TOP_THREADS, sizeof(PlanShared), s, k_refit_plan, t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
         e->at<int2>(e->L.ntop), e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
         &e->hdr()->status));
     CCC_LAUNCH_CHECK();
@@ -535,16 +511,13 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
 
 template <class T> int loop_prepare(ccc_engine* e, int64_t ntri, int64_t nb, cudaStream_t s) {
     Tables t = e->building();
-    CCC_LAUNCH("k_loop_reset", s, k_loop_reset<<<grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s>>>(
-        t.f, e->at<int>(e->L.iters), e->at<int>(e->L.flags)));
+    CCC_LAUNCH("k_loop_reset", s, launch_chain(grid_for(e->mesh_cap, ITEM_THREADS), ITEM_THREADS, 0, s, k_loop_reset, t.f, e->at<int>(e->L.iters), e->at<int>(e->L.flags)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_zero_acc", s, k_zero_acc<<<item_grid(), ITEM_THREADS, 0, s>>>(t.f, t.vt, e->at<long long>(e->L.acc)));
+    CCC_LAUNCH("k_zero_acc", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_zero_acc, t.f, t.vt, e->at<long long>(e->L.acc)));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_gather_soup", s, k_gather_soup<T><<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, t.vt, nullptr, e->at<int>(e->L.faces), e->at<T>(e->L.verts0), e->at<T>(e->L.x0), &e->hdr()->status));
+    CCC_LAUNCH("k_gather_soup", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_gather_soup<T>, t.f, t.vt, nullptr, e->at<int>(e->L.faces), e->at<T>(e->L.verts0), e->at<T>(e->L.x0), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_gather_soup", s, k_gather_soup<T><<<item_grid(), ITEM_THREADS, 0, s>>>(
-        t.f, t.vt, nullptr, e->at<int>(e->L.faces), e->at<T>(e->L.verts1), e->at<T>(e->L.x1), &e->hdr()->status));
+    CCC_LAUNCH("k_gather_soup", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_gather_soup<T>, t.f, t.vt, nullptr, e->at<int>(e->L.faces), e->at<T>(e->L.verts1), e->at<T>(e->L.x1), &e->hdr()->status));
     CCC_LAUNCH_CHECK();
     return build_trees<T>(e, ntri, nb, s);
 }
@@ -899,19 +872,16 @@ int ccc_engine_pack_rows(ccc_engine* e, int64_t* out_rows, void* out_times, int6
     if (e->tri_cap * e->maxcol >= ((int64_t)1 << 31)) return CCC_ERR_INVALID_ARG;   // int32 offsets
     cudaStream_t s = (cudaStream_t)stream;
     Forest F = e->active().f;
-    CCC_LAUNCH("k_pack_offsets", s, k_pack_offsets<<<1, PACK_SCAN_THREADS, 0, s>>>(
-        F, e->at<int>(e->L.mesh_cnt), (int)e->maxcol, &e->hdr()->status, out_meta));
+    CCC_LAUNCH("k_pack_offsets", s, launch_chain(1, PACK_SCAN_THREADS, 0, s, k_pack_offsets, F, e->at<int>(e->L.mesh_cnt), (int)e->maxcol, &e->hdr()->status, out_meta));
     CCC_LAUNCH_CHECK();
     if (capacity == 0) return CCC_OK;
     int64_t work = std::min<int64_t>(capacity, e->active_tris * e->maxcol);
     int g = (int)std::max<int64_t>(1, std::min<int64_t>(grid_for(work, 256), (int64_t)num_sms() * 8));
     if (e->dtype)
-        CCC_LAUNCH("k_pack_rows", s, k_pack_rows<double><<<g, 256, 0, s>>>(
-            F, out_meta, e->at<long long>(e->L.rows), e->at<double>(e->L.times), (int)e->maxcol, (long long*)out_rows,
+        CCC_LAUNCH("k_pack_rows", s, launch_chain(g, 256, 0, s, k_pack_rows<double>, F, out_meta, e->at<long long>(e->L.rows), e->at<double>(e->L.times), (int)e->maxcol, (long long*)out_rows,
             (double*)out_times, capacity, &e->hdr()->status));
     else
-        CCC_LAUNCH("k_pack_rows", s, k_pack_rows<float><<<g, 256, 0, s>>>(
-            F, out_meta, e->at<long long>(e->L.rows), e->at<float>(e->L.times), (int)e->maxcol, (long long*)out_rows,
+        CCC_LAUNCH("k_pack_rows", s, launch_chain(g, 256, 0, s, k_pack_rows<float>, F, out_meta, e->at<long long>(e->L.rows), e->at<float>(e->L.times), (int)e->maxcol, (long long*)out_rows,
             (float*)out_times, capacity, &e->hdr()->status));
     CCC_LAUNCH_CHECK();
     return CCC_OK;

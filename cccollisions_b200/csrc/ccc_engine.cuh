@@ -65,6 +65,7 @@ static constexpr int BOUNDS_CHUNK = 256;
 template <class T>
 __global__ void k_mesh_bounds(Forest F, const T* __restrict__ x0, const T* __restrict__ x1,
                               unsigned* __restrict__ bounds, float2* __restrict__ cxy, float* __restrict__ cz) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     const unsigned FULL = 0xffffffffu;
@@ -143,6 +144,7 @@ __device__ __forceinline__ unsigned quantize1024(float c, float lo, float hi) {
 static __global__ void k_morton(Forest F, const float2* __restrict__ cxy, const float* __restrict__ cz,
                          const unsigned* __restrict__ bounds, unsigned long long* __restrict__ keys,
                          int* __restrict__ vals) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -168,6 +170,7 @@ static constexpr int SORT_TILE = SORT_THREADS * SORT_ROUNDS;
 // counts[d * nblk + b] = number of keys of tile b with digit d
 static __global__ void __launch_bounds__(SORT_THREADS)
 k_radix_hist(const unsigned long long* __restrict__ keys, int n, int shift, int* __restrict__ counts, int nblk) {
+    chain_begin();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -207,6 +210,7 @@ __device__ __forceinline__ int sort_block_exclusive_scan(int v, int* wsum, int* 
 static constexpr int ROWSCAN_ITEMS = 4;
 static __global__ void __launch_bounds__(SORT_THREADS)
 k_radix_rowscan(int* __restrict__ counts, int nblk, int* __restrict__ rowtot) {
+    chain_begin();
     __shared__ int wsum[SORT_THREADS / 32 + 1];
     int* row = counts + (long long)blockIdx.x * nblk;
     int carry = 0;                                   // (the same in every thread)
@@ -236,6 +240,7 @@ static __global__ void __launch_bounds__(SORT_THREADS)
 k_radix_scatter(const unsigned long long* __restrict__ kin, const int* __restrict__ vin,
                 unsigned long long* __restrict__ kout, int* __restrict__ vout, int n, int shift,
                 const int* __restrict__ offs, const int* __restrict__ rowtot, int nblk) {
+    chain_begin();
     constexpr int WARPS = SORT_THREADS / 32;
     __shared__ int whist[WARPS][256];
     __shared__ int base[256];
@@ -299,6 +304,7 @@ static __global__ void k_karras_build(Forest F, const unsigned long long* __rest
                                       int* __restrict__ leaf_tri, unsigned* __restrict__ visits,
                                       int2* __restrict__ nrange, int2* __restrict__ ntop, int* __restrict__ top_node,
                                       int* __restrict__ top_index, int* __restrict__ status) {
+    chain_begin();
     const int M = forest_size(F);
     const int total_internal = __ldg(F.voff + M) - M;
     for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < total_internal; gi += gridDim.x * blockDim.x) {
@@ -376,6 +382,7 @@ static constexpr int QCODE_ODD = -2;
 // get their slot code from k_qtree_slots
 static __global__ void k_qtree_depth(Forest F, const int* __restrict__ nparent, int* __restrict__ qcode,
                                      int* __restrict__ status) {
+    chain_begin();
     const int M = forest_size(F);
     const int total_internal = __ldg(F.voff + M) - M;
     for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < total_internal; gi += gridDim.x * blockDim.x) {
@@ -398,6 +405,7 @@ static __global__ void k_qtree_depth(Forest F, const int* __restrict__ nparent, 
 // slot code of every leaf (qleaf) and even-depth internal node (qcode) they hold
 static __global__ void k_qtree_slots(Forest F, const TNode* __restrict__ nodes, int* __restrict__ qcode,
                                      int* __restrict__ qleaf, QNode* __restrict__ qnodes, int* __restrict__ status) {
+    chain_begin();
     const int M = forest_size(F);
     const int total_internal = __ldg(F.voff + M) - M;
     for (int gi = blockIdx.x * blockDim.x + threadIdx.x; gi < total_internal; gi += gridDim.x * blockDim.x) {
@@ -508,6 +516,7 @@ __device__ __forceinline__ WeldItem weld_item(const Forest& F, int M, int v) {
 template <class T>
 __global__ void k_weld_insert(Forest F, const T* __restrict__ x0, const T* __restrict__ x1, int* tab,
                               int* __restrict__ vidc, int* cnt, WsHeader* hdr) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -567,6 +576,7 @@ static constexpr int WELD_THREADS = 256;
 static __global__ void __launch_bounds__(WELD_THREADS)
 k_weld_alloc(Forest F, const int* __restrict__ vidc, const int* __restrict__ cnt, int* __restrict__ fan_start,
              int* __restrict__ fan_end, WsHeader* hdr) {
+    chain_begin();
     __shared__ int wsum[WELD_THREADS / 32];
     __shared__ int base_s;
     const int M = forest_size(F);
@@ -609,6 +619,7 @@ k_weld_alloc(Forest F, const int* __restrict__ vidc, const int* __restrict__ cnt
 
 static __global__ void k_weld_fill(Forest F, const int* __restrict__ vidc, const int* __restrict__ fan_start,
                                    int* fan_end, int4* __restrict__ fan) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -627,6 +638,7 @@ static __global__ void k_weld_fill(Forest F, const int* __restrict__ vidc, const
 // go to the place of their rank in their class, one thread an entry
 static __global__ void k_weld_rank(Forest F, const int* __restrict__ vidc, const int* __restrict__ fan_start,
                                    const int* __restrict__ cnt, const int4* __restrict__ tmp, int4* __restrict__ fan) {
+    chain_begin();
     const int M = forest_size(F);
     const long long entries = 3LL * __ldg(F.voff + M);       // every corner is in one class
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < entries;
@@ -648,6 +660,7 @@ static __global__ void k_weld_rank(Forest F, const int* __restrict__ vidc, const
 static __global__ void k_weld_tri(Forest F, const int* __restrict__ vidc, const int* __restrict__ cnt,
                                   const int* __restrict__ fan_start, const int4* __restrict__ fan,
                                   int4* __restrict__ vid, int4* __restrict__ twin, int4* __restrict__ third) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -784,6 +797,7 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
                      const int* __restrict__ qcode, const int* __restrict__ qleaf, const int2* __restrict__ nrange,
                      const TNode* __restrict__ nodes, QNode* qnodes, const int2* __restrict__ ntop,
                      int2* __restrict__ front, int front_cap, const int* __restrict__ mflags, WsHeader* hdr) {
+    chain_begin();
     __shared__ float s_llo[3][REFIT_THREADS], s_lhi[3][REFIT_THREADS];    // leaf boxes
     __shared__ float s_nlo[3][REFIT_THREADS], s_nhi[3][REFIT_THREADS];    // local node boxes
     __shared__ unsigned short s_done[REFIT_THREADS];    // round a local node was done in (0: not yet)
@@ -917,6 +931,7 @@ static __global__ void __launch_bounds__(TOP_THREADS)
 k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ qcode, const int* __restrict__ qleaf,
              const int2* __restrict__ nrange, int2* __restrict__ ntop, int* __restrict__ top_node,
              int* __restrict__ top_index, int2* __restrict__ top_child, int* __restrict__ status) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     PlanShared& S = *reinterpret_cast<PlanShared*>(smem);
     const int M = forest_size(F);
@@ -1020,6 +1035,7 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
                    const int2* __restrict__ ntop, const int* __restrict__ top_node, const int* __restrict__ top_index,
                    const int2* __restrict__ top_child, unsigned* visits, const int2* __restrict__ front,
                    int front_cap, const int* __restrict__ mflags, WsHeader* hdr) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_end[TOP_LEVELS + 1];
     const cg::cluster_group cluster = cg::this_cluster();
@@ -1207,6 +1223,7 @@ static __global__ void __launch_bounds__(WALK_THREADS, 8)
 k_traverse_walk(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, const int* __restrict__ leaf_tri,
                 Forest F, int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const int* __restrict__ mflags,
                 const int4* __restrict__ vid) {
+    chain_begin();
     __shared__ WalkWarp S[WALK_WARPS];
     const EngineWalk<CLASSES> pol{qnodes, qleaf, leaf_tri, mflags, vid};
     walk_forest(pol, qnodes, F, cand, cand_cap, hdr, S[threadIdx.x >> 5]);
@@ -1227,6 +1244,7 @@ static __global__ void __launch_bounds__(TRAV_THREADS)
 k_traverse_q(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, const int* __restrict__ leaf_tri,
              Forest F, int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const int* __restrict__ mflags,
              const int4* __restrict__ vid) {
+    chain_begin();
     int stack[STACK_DEPTH];          // per-thread, in local memory (L1): shared memory holds the buffer
     __shared__ int2 cbuf[TRAV_BUF][TRAV_THREADS];     // candidate buffer (see flush_candidates)
     __shared__ QNode top[trav_stage_count(SD)];
@@ -1398,6 +1416,7 @@ static __global__ void __launch_bounds__(TRAV_THREADS)
 k_traverse_w(const QNode* __restrict__ qnodes, const int* __restrict__ qleaf, const int* __restrict__ leaf_tri,
              Forest F, int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const int* __restrict__ mflags,
              const int4* __restrict__ vid) {
+    chain_begin();
     __shared__ int2 cbuf[TRAV_BUF][TRAV_THREADS];     // candidate buffer (see flush_candidates)
     __shared__ __align__(16) int nbuf_s[TRAV_THREADS / 32][32];    // each warp's staged QNode
     const unsigned FULL = 0xffffffffu;
@@ -1592,6 +1611,7 @@ template <class T> struct LoopSink {
 // contacts takes this iteration's corrections and stops at max_iter iterations
 static __global__ void k_loop_update(Forest F, const int* __restrict__ contacts, int* __restrict__ iters,
                                      int* __restrict__ flags, int max_iter) {
+    chain_begin();
     const int M = forest_size(F);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         int sid = __ldg(F.sid + m);
@@ -1611,6 +1631,7 @@ static __global__ void k_loop_update(Forest F, const int* __restrict__ contacts,
 template <class T>
 __global__ void k_loop_apply(Forest F, VertTable vt, const int* __restrict__ contacts, long long* __restrict__ acc,
                              T* __restrict__ verts1, T* __restrict__ vel) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(vt.vvoff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -1638,6 +1659,7 @@ __global__ void k_loop_apply(Forest F, VertTable vt, const int* __restrict__ con
 template <class T>
 __global__ void k_gather_soup(Forest F, VertTable vt, const int* __restrict__ contacts, const int* __restrict__ faces,
                               const T* __restrict__ verts, T* __restrict__ soup, int* status) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(F.voff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -1666,6 +1688,7 @@ __global__ void k_gather_soup(Forest F, VertTable vt, const int* __restrict__ co
 // centroid bounds of every mesh in the table to (empty): min words high, max words low
 // and no top nodes
 static __global__ void k_reset_bounds(Forest F, unsigned* __restrict__ bounds, int2* __restrict__ ntop) {
+    chain_begin();
     const int M = forest_size(F);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         unsigned* b = bounds + 6 * __ldg(F.sid + m);
@@ -1677,6 +1700,7 @@ static __global__ void k_reset_bounds(Forest F, unsigned* __restrict__ bounds, i
 
 // loop counters and flags of every mesh in the table
 static __global__ void k_loop_reset(Forest F, int* __restrict__ iters, int* __restrict__ flags) {
+    chain_begin();
     const int M = forest_size(F);
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         int sid = __ldg(F.sid + m);
@@ -1687,6 +1711,7 @@ static __global__ void k_loop_reset(Forest F, int* __restrict__ iters, int* __re
 
 // vertex accumulators of every mesh in the table
 static __global__ void k_zero_acc(Forest F, VertTable vt, long long* __restrict__ acc) {
+    chain_begin();
     const int M = forest_size(F);
     const int total = __ldg(vt.vvoff + M);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < total; v += gridDim.x * blockDim.x) {
@@ -1704,6 +1729,7 @@ static __global__ void k_zero_acc(Forest F, VertTable vt, long long* __restrict_
 static constexpr int PACK_SCAN_THREADS = 1024;
 static __global__ void __launch_bounds__(PACK_SCAN_THREADS)
 k_pack_offsets(Forest F, const int* __restrict__ mesh_cnt, int maxcol, const int* status, int* __restrict__ meta) {
+    chain_begin();
     __shared__ int warp_sum[PACK_SCAN_THREADS / 32];
     __shared__ int carry;
     const int M = forest_size(F);
@@ -1746,6 +1772,7 @@ template <class T>
 static __global__ void k_pack_rows(Forest F, const int* __restrict__ meta, const long long* __restrict__ rows,
                                    const T* __restrict__ times, int maxcol, long long* __restrict__ out_rows,
                                    T* __restrict__ out_times, long long capacity, int* status) {
+    chain_begin();
     const int M = forest_size(F);
     const long long total = __ldg(meta + M);
     const long long n = min(total, capacity);

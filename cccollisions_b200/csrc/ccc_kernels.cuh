@@ -21,6 +21,15 @@ namespace cg = cooperative_groups;
 
 namespace ccc {
 
+// Every kernel that launch_chain launches begins with this: the launch lets it start as the
+// blocks of the kernel before it in the stream end, which hides most of a launch's latency (968
+// triangles' impulses, ten kernels, 113 -> 103 us; building and stepping 12 meshes, 45 kernels,
+// 1,282 -> 1,204 us); here it waits until that kernel is complete and its writes are visible.
+// (Letting the next kernel start as soon as this one's last block runs, by an explicit trigger,
+// made the kernels that fill the GPU share it with blocks that only wait: the 256 x 256 fold
+// 1,148 -> 1,254 us, the 64-mesh step 10.69 -> 11.62 ms.)
+__device__ __forceinline__ void chain_begin() { cudaGridDependencySynchronize(); }
+
 enum StatusBits {
     ST_CAND_OVERFLOW = 1,     // more candidate pairs than max_candidates_per_triangle * F
     ST_OUT_OVERFLOW = 2,      // more result rows than the output tensor holds
@@ -102,6 +111,7 @@ __device__ __forceinline__ int forest_slot_mesh(const Forest& f, int M, long lon
 // packed mesh table for the reference API (B meshes of F triangles): nm = B,
 // voff[i] = poff[i] = i * F, sid[i] = i
 static __global__ void k_uniform_offsets(int* nm, int* voff, int* poff, int* sid, int M, int F) {
+    chain_begin();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *nm = M;
     if (i <= M) voff[i] = i * F;
@@ -120,6 +130,7 @@ struct FillJob {
     uint32_t lo, hi;
 };
 static __global__ void k_fill(FillJob a, FillJob b, FillJob c) {
+    chain_begin();
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
     auto fill = [&](const FillJob& j) {
         const long long quads = ((uintptr_t)j.p & 15) == 0 ? j.words / 4 : 0;
@@ -150,6 +161,7 @@ template <class T> __device__ __forceinline__ void box_to_f32(const T* p, float 
 template <class T>
 __global__ void k_import_nodes(const int* __restrict__ moff, int M, int total_internal, const T* __restrict__ bboxes,
                                const long long* __restrict__ tree, TNode* __restrict__ nodes, int* status) {
+    chain_begin();
     int gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= total_internal) return;
     int m = find_mesh(moff, M, gi, 1);
@@ -190,6 +202,7 @@ __global__ void k_import_nodes(const int* __restrict__ moff, int M, int total_in
 // rightmost leaf position of every internal subtree, written into the parent's aux slot
 static __global__ void k_import_rightmost(const int* __restrict__ moff, int M, int total, const long long* __restrict__ tree,
                                    TNode* nodes, int* __restrict__ visits, int* __restrict__ rmk, int* status) {
+    chain_begin();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
     int m = find_mesh(moff, M, g, 0);
@@ -284,6 +297,7 @@ template <class T, bool MASKED, bool EXACT_F32, class Leaves>
 __global__ void __launch_bounds__(TRAV_THREADS)
 k_traverse(const TNode* __restrict__ nodes, Leaves leaves, Forest F, const uint8_t* __restrict__ mask, T th,
            int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const int* __restrict__ mflags) {
+    chain_begin();
     int stack[STACK_DEPTH];          // per-thread, in local memory (L1): shared memory holds the buffer
     __shared__ int2 cbuf[TRAV_BUF][TRAV_THREADS];
     int nbuf = 0;
@@ -418,6 +432,7 @@ template <class T>
 __global__ void __launch_bounds__(NARROW_THREADS)
 k_static_narrow(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T* __restrict__ tri, Forest F,
                 T th, long long* __restrict__ rows, int max_per_tri, int* __restrict__ mesh_counters) {
+    chain_begin();
     const int M = forest_size(F);
     int n = min(hdr->cand_count, cand_cap);
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
@@ -449,6 +464,7 @@ __global__ void __launch_bounds__(NARROW_THREADS)
 k_te_narrow(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T* __restrict__ tri, Forest F,
             long long* __restrict__ rows, T* __restrict__ coefs, int* __restrict__ masks, int max_per_tri,
             int* __restrict__ mesh_counters) {
+    chain_begin();
     const int M = forest_size(F);
     int n = min(hdr->cand_count, cand_cap);
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
@@ -901,6 +917,7 @@ template <class T>
 __global__ void __launch_bounds__(STAGE_THREADS, 3)
 k_ccd_stage_mask(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T* __restrict__ x0,
                  const T* __restrict__ x1, Weld W, int4* __restrict__ live, int4* __restrict__ pending) {
+    chain_begin();
     __shared__ int2 q_pr[STAGE_WARPS][64];
     __shared__ int4 q_va[STAGE_WARPS][64], q_vb[STAGE_WARPS][64];
     const int n = min(*(volatile int*)&hdr->cand_count, cand_cap);
@@ -974,6 +991,7 @@ k_ccd_stage_mask(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, con
 
 static __global__ void __launch_bounds__(STAGE_THREADS, 8)
 k_ccd_stage_pending(int cand_cap, WsHeader* hdr, Weld W, const int4* __restrict__ pending, int4* __restrict__ live) {
+    chain_begin();
     // per warp: 32 pending pairs, their classes, the sub-tests they solve, and their pending
     // sub-tests (lane of the pair << 4 | type) one after the other; the lanes take those 32 at a
     // time
@@ -1035,6 +1053,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, 3)
 k_ccd_mask(int2* cand, int cand_cap, WsHeader* hdr, const T* __restrict__ x0, const T* __restrict__ x1,
            unsigned short* __restrict__ masks, int4* __restrict__ live, Forest F, long long* __restrict__ rows,
            int max_per_tri, int* __restrict__ mesh_counters) {
+    chain_begin();
     __shared__ int2 q_pr[STAGE_WARPS][64];
     __shared__ int q_at[STAGE_WARPS][64];
     const int n = min(*(volatile int*)&hdr->cand_count, cand_cap);
@@ -1188,6 +1207,7 @@ __device__ __noinline__ void record_in_place(const CcdArgs<T>* A, const Sink* si
 template <class T, int MODE, class Sink, int LIB, int SRC, int BM>
 __global__ void __launch_bounds__(CCD_BLOCK, ccd_min_blocks(BM))
 k_ccd_narrow(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink sink) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NB = BM * CCD_BLOCK;
     constexpr int NW = CCD_BLOCK / 32;
@@ -1509,8 +1529,8 @@ template <class T, int MODE, class Sink, int LIB, int SRC, int BM>
 cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink) {
     cudaError_t e = prepare_ccd_narrow<T, MODE, Sink, LIB, SRC, BM>();
     if (e != cudaSuccess) return e;
-    k_ccd_narrow<T, MODE, Sink, LIB, SRC, BM><<<grid, CCD_BLOCK, CcdLayout<T, BM * CCD_BLOCK>::bytes, s>>>(A, sink);
-    return cudaSuccess;
+    return launch_chain(grid, CCD_BLOCK, CcdLayout<T, BM * CCD_BLOCK>::bytes, s,
+                        k_ccd_narrow<T, MODE, Sink, LIB, SRC, BM>, A, sink);
 }
 
 // The contacts of the roots that passed the filter in k_ccd_narrow, one record a thread: the
@@ -1520,6 +1540,7 @@ static constexpr int CONTACT_THREADS = 128;
 template <class T, class Sink, int LIB>
 __global__ void __launch_bounds__(CONTACT_THREADS)
 k_ccd_contacts(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink sink) {
+    chain_begin();
     const int n = min(*(volatile int*)&A.hdr->expand_count, A.W.expand_cap);
     for (int c = blockIdx.x * CONTACT_THREADS + threadIdx.x; c < n; c += gridDim.x * CONTACT_THREADS) {
         const int4 rec = A.W.expand[c];
@@ -1530,8 +1551,7 @@ k_ccd_contacts(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sin
 
 template <class T, class Sink, int LIB>
 cudaError_t launch_ccd_contacts(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink) {
-    k_ccd_contacts<T, Sink, LIB><<<grid, CONTACT_THREADS, 0, s>>>(A, sink);
-    return cudaSuccess;
+    return launch_chain(grid, CONTACT_THREADS, 0, s, k_ccd_contacts<T, Sink, LIB>, A, sink);
 }
 #endif  // CCC_NARROW_TU
 
@@ -1543,6 +1563,7 @@ template <class T>
 __global__ void __launch_bounds__(EXPAND_THREADS)
 k_ccd_expand(WsHeader* hdr, Weld W, Forest F, long long* __restrict__ rows, T* __restrict__ times, int max_per_tri,
              int* __restrict__ mesh_counters) {
+    chain_begin();
     const unsigned FULL = 0xffffffffu;
     const int M = forest_size(F);
     const int n = min(*(volatile int*)&hdr->expand_count, W.expand_cap);
@@ -1592,6 +1613,7 @@ template <class T>
 __global__ void __launch_bounds__(NARROW_THREADS)
 k_prox_narrow(const int2* __restrict__ cand, int cand_cap, WsHeader* hdr, const T* __restrict__ tri, Forest F, T th,
               long long* __restrict__ rows, int max_per_tri, int* __restrict__ mesh_counters) {
+    chain_begin();
     // less than 32 left over, and 32 pairs' sub-tests
     __shared__ int2 s_ee[PROX_WARPS][32 + 9 * 32], s_vf[PROX_WARPS][32 + 6 * 32];
     const unsigned FULL = 0xffffffffu;
@@ -1656,6 +1678,7 @@ __global__ void __launch_bounds__(NARROW_THREADS)
 k_impulses_from_rows(const long long* __restrict__ rows, const T* __restrict__ roots, int B, long long N, int F,
                      const T* __restrict__ x0, const T* __restrict__ x1, const T* __restrict__ masses,
                      T* __restrict__ dv_out, T* __restrict__ dx_out, int* __restrict__ cnt_out) {
+    chain_begin();
     long long total = (long long)B * N;
     for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < total;
          r += (long long)gridDim.x * blockDim.x) {

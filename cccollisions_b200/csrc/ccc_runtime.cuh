@@ -27,6 +27,24 @@ int num_sms();
 inline int64_t align_up(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 
+// Launch of a kernel that begins with chain_begin(): it may start while the kernel before it in
+// the stream drains (programmatic stream serialization).  Kernels that do not begin so must not
+// be launched with it.
+template <class... P, class... A>
+cudaError_t launch_chain(int grid, int block, size_t smem, cudaStream_t s, void (*kernel)(P...), A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace ccc
 
 #define CCC_LAUNCH(name, s, ...)                  \

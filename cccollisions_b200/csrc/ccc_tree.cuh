@@ -74,6 +74,7 @@ template <class T, int LOG_THREADS>
 __global__ void __launch_bounds__(1 << LOG_THREADS)
 k_bvh_levels(const T* __restrict__ x0, const T* __restrict__ x1, int n, int chunks, int level, T* bboxes,
              long long* __restrict__ tree, WsHeader* hdr, int* __restrict__ mesh_cnt) {
+    chain_begin();
     constexpr int THREADS = 1 << LOG_THREADS;
     __shared__ T wbox[6][THREADS / 32];
     const int m = blockIdx.x / chunks, t = threadIdx.x, lane = t & 31;
@@ -183,6 +184,7 @@ template <class T>
 __global__ void k_import_wide(int n, int meshes, const T* __restrict__ bboxes, const long long* __restrict__ tree,
                               QNode* __restrict__ qnodes, int* __restrict__ visits, int* __restrict__ rmk,
                               int* __restrict__ table, int* __restrict__ moff, WsHeader* hdr) {
+    chain_begin();
     const int gi = blockIdx.x * blockDim.x + threadIdx.x;
     const int internal = meshes * (n - 1);
     // the packed mesh table (Forest): count, offsets, data offsets, slot ids
@@ -274,6 +276,7 @@ __global__ void k_import_wide(int n, int meshes, const T* __restrict__ bboxes, c
 // the rightmost leaf position below every internal node of a general tree, by climbs
 static __global__ void k_import_rightmost_wide(int n, int total, const long long* __restrict__ tree,
                                                int* __restrict__ visits, int* __restrict__ rmk, WsHeader* hdr) {
+    chain_begin();
     if (!*(volatile int*)&hdr->general) return;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= total) return;
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 8)
 k_walk_tensors(const QNode* __restrict__ qnodes, const T* __restrict__ bboxes, const long long* __restrict__ tree,
                const uint8_t* __restrict__ mask, const int* __restrict__ rmk, int n, Forest F, T th,
                int2* __restrict__ cand, int cand_cap, WsHeader* hdr) {
+    chain_begin();
     __shared__ WalkWarp S[WALK_WARPS];
     const TensorWalk<T, MASKED, EXACT_F32> pol{bboxes, tree, mask, rmk, th, n, *(volatile int*)&hdr->general};
     walk_forest(pol, qnodes, F, cand, cand_cap, hdr, S[threadIdx.x >> 5]);
