@@ -441,7 +441,7 @@ def run_ours(args, rank, world, dev):
                     "rows_equal_batched": bool(e2e_equal)},
             "work": {"autotuned_shape": shape, "candidates": cnt["candidates"], "subtests": cnt["subtests"],
                      "subtests_solved": cnt["solved"], "pairs_with_work": cnt["live_pairs"],
-                     "roots_in_unit_interval": cnt["roots"], "collision_rows": int(sum(nrow)), "status": cnt["status"],
+                     "roots_filtered": cnt["roots"], "collision_rows": int(sum(nrow)), "status": cnt["status"],
                      "tree_boxes": "fp32"},
             "kernel_ms_per_step": {k: r3(v[0] / v[1]) for k, v in kern.items()},
             "fp64": {"kernel": "k_ccd_narrow", "units": "sub-tests solved", "achieved_gflops": r3(fp64_gflops),

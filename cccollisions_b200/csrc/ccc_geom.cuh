@@ -692,6 +692,145 @@ template <class T> __device__ __forceinline__ bool ccd_filter(const MTet<T>& tet
     return is_inside(inv ? p1 : p0, inv ? p2 : p1, inv ? p3 : p2, inv ? p0 : p3);
 }
 
+// |x| + |y| + |z|: at least the length
+__device__ __forceinline__ float reach(V3<float> a) { return fabsf(a.x) + fabsf(a.y) + fabsf(a.z); }
+template <class T> __device__ __forceinline__ V3<float> to_float(V3<T> a) { return mk<float>((float)a.x, (float)a.y, (float)a.z); }
+
+// at least the largest of the components (a double's by its upper word: conversions are slow)
+__device__ __forceinline__ float largest(V3<float> a, V3<float> b) {
+    return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(b.x))), fmaxf(fabsf(b.y), fabsf(b.z)));
+}
+__device__ __forceinline__ float largest(V3<double> a, V3<double> b) {
+    auto hi = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+    const int m = max(max(max(hi(a.x), hi(a.y)), max(hi(a.z), hi(b.x))), max(hi(b.y), hi(b.z)));
+    return (float)__hiloint2double(m + 1, 0);
+}
+
+// The vectors that decide the filter of sub-test k, at the start (0) and their displacements (1):
+// edges a and b of an edge-edge sub-test and what is between their origins, or two edges of the
+// face from one of its corners and the vertex from there (the corner that needs no more
+// differences than those of the coefficients).
+struct FilterFrame {
+    V3<float> a0, b0, c0, a1, b1, c1;
+    float da, db, dc;           // at least the lengths of the displacements
+    float size;                 // at least the sum of the lengths, at all times in [0, 1]
+    float pos;                  // at least the error of a vector, here and in the filter itself
+};
+
+template <class T> __device__ __forceinline__ FilterFrame filter_frame(const MTet<T>& tet, int k) {
+    FilterFrame F;
+    const bool ee = k < 9, last = k >= 12;
+    const V3<float> w0 = to_float(tet.v[0] - tet.v[3]), w1 = to_float(tet.v[1] - tet.v[3]), w2 = to_float(tet.v[2] - tet.v[3]);
+    const V3<float> u0 = to_float(tet.dv[0] - tet.dv[3]), u1 = to_float(tet.dv[1] - tet.dv[3]), u2 = to_float(tet.dv[2] - tet.dv[3]);
+    const float z1 = last ? 0.0f : 1.0f, s2 = ee ? -1.0f : 1.0f, z2 = ee ? 0.0f : z1;
+    const float z3 = ee ? 1.0f : 0.0f, z4 = last ? 1.0f : -1.0f;
+    F.a0 = w1 - w0 * z1;
+    F.a1 = u1 - u0 * z1;
+    F.b0 = w2 * s2 - w0 * z2;
+    F.b1 = u2 * s2 - u0 * z2;
+    F.c0 = w2 * z3 + w0 * z4;
+    F.c1 = u2 * z3 + u0 * z4;
+    F.da = reach(F.a1);
+    F.db = reach(F.b1);
+    F.dc = reach(F.c1);
+    F.size = (reach(F.a0) + F.da) + (reach(F.b0) + F.db) + (reach(F.c0) + F.dc);
+    F.pos = (sizeof(T) == 8 ? 1.2e-14f : 6e-6f) * largest(tet.v[3], tet.dv[3]) + 2e-6f * F.size;
+    return F;
+}
+
+// True when ccd_filter, as it rounds in T, returns false at every time of [0, 1] within dt of t.
+// With the vectors V = va, vb, vc of the frame at t (errors at most ea, eb, ec over those times),
+// n = va x vb and det = |n|^2, both filters ask for the signs of the same two numbers: the parameters
+// are s / det and p / det for two edges, the face's barycentric coordinates s / det, -p / det and
+// (det - s + p) / det for a vertex, whichever corner the filter itself starts from.  Each sum here
+// is trusted only beyond what the vectors' errors can change, by the triangle inequality over
+// the lengths' bounds: 2e-6 of the frame's size covers the rounding of this function's and a float
+// filter's differences and products (below 1e-6), `low` that of the filter's Gram products (24
+// roundings of numbers below size^4) and, by its constant part, underflow.  det is positive, so
+// that no quotient is NaN (which would pass); NaN and overflow here end in `false`.
+template <class T> __device__ __forceinline__ bool filter_fails(const FilterFrame& F, int k, float t, float dt) {
+    const bool ee = k < 9;
+    const float ea = fmaf(dt, F.da, F.pos), eb = fmaf(dt, F.db, F.pos), ec = fmaf(dt, F.dc, F.pos);
+    const V3<float> va = axpy(F.a0, F.a1, t), vb = axpy(F.b0, F.b1, t), vc = axpy(F.c0, F.c1, t);
+    const float la = reach(va), lb = reach(vb), lc = reach(vc);
+    const V3<float> n = cross(va, vb), gs = cross(vc, vb), gp = cross(vc, va);
+    const float ln = reach(n), ls = reach(gs), lp = reach(gp);
+    const float en = fmaf(la, eb, fmaf(lb, ea, ea * eb)), es = fmaf(lc, eb, fmaf(lb, ec, eb * ec)),
+                ep = fmaf(lc, ea, fmaf(la, ec, ea * ec));
+    const float low = (sizeof(T) == 8 ? 1e-13f : 2e-6f) * F.size * F.size * F.size * F.size + 1e-30f;
+    const float s = dot(gs, n), p = dot(gp, n), det = dot(n, n);
+    const float ms = fmaf(ls, en, fmaf(ln, es, fmaf(es, en, low))), mp = fmaf(lp, en, fmaf(ln, ep, fmaf(ep, en, low)));
+    const float md = fmaf(2.0f * ln, en, fmaf(en, en, low));
+    const bool out = s < -ms || (ee ? (p < -mp || s - det > ms + md || p - det > mp + md)
+                                    : (p > mp || (s - p) - det > ms + mp + md));
+    return out && det > md && fabsf(s) + fabsf(p) + det < 1e30f;
+}
+
+// True when every root in [0, 1] that the solver can return for the cubic cf of sub-test k is sure
+// to fail the filter: some 250 fp32 and 30 fp64 instructions instead of the solver's 1,700 and the
+// filter's gathers.  The roots leave |p| < m (see cubic_misses; where the discriminant shows three
+// real roots by more than its rounding, only the first of its bounds counts: 2.8e-14 |a| r^3, taken
+// as 1e-12), so that each lies in one of the intervals tested:
+//  * one crossing: p keeps the sign of its slope on [0, 1] and has both signs at the ends, by more
+//    than m: every root is within (m + |p(t)|) / slope of any t, here two Newton steps' from the chord;
+//  * p(0) is zero within m (coplanar at the start, as every sub-test within a flat sheet): with
+//    p = d + t q(t), t |q(t)| <= m + |d|.  q of one sign, at least `least`: t <= (m + |d|) / least.
+//    q monotone with a root t' in between: t or |t - t'| is at most 2 (m + |d|) / (slope t').
+// Everything else goes to the solver, as do calls too small for the time to matter (the caller).
+//
+// Measured: none of 2^32 moving tetrahedra of twelve families (flat, far from the origin, nearly
+// rigid, parallel edges, roots at the filter's borders, degenerate, ..) that it drops has a root
+// that passes, in either precision and with both sets of elementary functions; three certain roots
+// left at most 5e-16 |a| r^3 in 2^31 cubics.  It drops 56 % of the sub-tests of the 64 meshes and 65 %
+// of the cloth over the sphere (flat at the start), 23 % of the fold's 13.0 M.
+template <class T> __device__ __forceinline__ bool roots_fail(const MTet<T>& tet, int k, const T cf[4]) {
+    const double a = cf[0], b = cf[1], c = cf[2], d = cf[3];
+    const float fa = (float)a, fb = (float)b, fc = (float)c, fd = (float)d;
+    const float A = fabsf(fa), B = fabsf(fb), C = fabsf(fc), D = fabsf(fd);
+    const float inv = __frcp_rn(A), q = B * inv;
+    const float r3 = fmaxf(fmaxf(q * q * B, C * __fsqrt_rn(C * inv)), D);
+    const double X = b * b, Y = a * c, Z = a * a * d;
+    const double f = 3.0 * Y - X, g = b * (2.0 * X - 9.0 * Y) + 27.0 * Z;
+    const bool three = 0.25 * g * g + f * f * f < -1e-10 * (X * X * X + fabs(Y * Y * Y) + Z * Z);
+    const float sum = A + B + C;
+    const float m = (three ? 1e-12f : 1e-3f) * r3 + 1e-6f * sum;
+    const float e1 = (float)((a + b) + (c + d));
+    const bool zero = D <= m;
+    // the polynomial whose root is looked for: p itself, or q = (p - d) / t when p(0) is about 0
+    const float q3 = zero ? 0.0f : fa, q2 = zero ? fa : fb, q1 = zero ? fb : fc, q0 = zero ? fc : fd;
+    const float qe = zero ? (float)((a + b) + c) : e1;
+    // its slope's Bernstein coefficients on [0, 1]
+    const float s0 = q1, s1 = q1 + q2, s2 = fmaf(2.0f, q2, fmaf(3.0f, q3, q1));
+    const bool mono = (s0 < 0.0f) == (s2 < 0.0f) && (zero || (s0 < 0.0f) == (s1 < 0.0f));
+    const float slope = fminf(fminf(fabsf(s0), zero ? 3e38f : fabsf(s1)), fabsf(s2)) - 4e-6f * sum;
+    const bool crosses = (q0 < 0.0f) != (qe < 0.0f);
+    const float least = fminf(fminf(fabsf(q0), fabsf(qe)), fabsf(fmaf(0.5f, q1, q0))) - 4e-6f * sum;
+    const bool definite = zero && !crosses && (q0 < 0.0f) == (fmaf(0.5f, q1, q0) < 0.0f) && least > 0.0f;
+    const bool one = crosses && mono && slope > 0.0f && (zero || (D > m && fabsf(e1) > m));
+    if (!(fabs(a) >= CCC_EPS && (definite || one))) return false;
+    float t = 0.0f, dt;
+    if (one) {
+        t = __fdividef(q0, q0 - qe);
+#pragma unroll
+        for (int it = 0; it < 2; ++it) {
+            const float p = fmaf(fmaf(fmaf(q3, t, q2), t, q1), t, q0);
+            const float ps = fmaf(fmaf(3.0f * q3, t, 2.0f * q2), t, q1);
+            t = fminf(fmaxf(t - __fdividef(p, ps), 0.0f), 1.0f);
+        }
+        // off: how far the root of q may be from t
+        const float off = __fdividef(fabsf(fmaf(fmaf(fmaf(q3, t, q2), t, q1), t, q0)) + 4e-6f * (sum + (zero ? 0.0f : D)), slope);
+        dt = zero ? 2.0f * __fdividef(m + D, slope * (t - off)) + off : __fdividef(m, slope) + off;
+        if (!(t > off)) return false;
+    } else {
+        dt = __fdividef(m + D, least);
+    }
+    dt = 1.0001f * dt + 1e-6f;
+    const FilterFrame F = filter_frame<T>(tet, k);
+    bool out = filter_fails<T>(F, k, t, dt);
+    if (one && zero) out = out && filter_fails<T>(F, k, 0.0f, dt);
+    return out;
+}
+
 // ------------------------------------------------------------------ impulses
 
 #define CCC_THICKNESS 2e-3   // collisions_impulses.cu:12-14

@@ -541,8 +541,9 @@ template <class T> struct CornerSink {
 // block-synchronous: blocks of CCD_BLOCK threads take CCD_BLOCK pairs at a time and queue
 // their sub-tests, and each stage of the solve runs on a full block of its own queue's
 // entries, so that every warp of the block runs the same stage's code at the same time:
-//   (1) the cubic's coefficients; sub-tests without a root in [0, 1] for certain end here
-//       (cubic_misses), the others are queued with their coefficients;
+//   (1) the cubic's coefficients; sub-tests that for certain have no root in [0, 1]
+//       (cubic_misses) or none that passes the filter (roots_fail) end here, the others are queued
+//       with their coefficients;
 //   (2) the solver prefix, which classifies them, and the roots, ordered by solver branch; the
 //       roots in [0, 1] are queued, edge-edge ones from the front of their array and
 //       vertex-face ones from its back;
@@ -557,13 +558,17 @@ template <class T> struct CornerSink {
 // the fold's impulses 1,698 -> 109 (masks) + 752 + 82 us (contacts), ten served folds 931 ->
 // 94 + 445 + 39 us an iteration, the cloth over the sphere 214 -> 21 + 161 us, 968 triangles
 // 45 -> 5 + 15 + 6 us; the 64-mesh step, whose masks were apart already, 5,336 -> 4,950 us.
-// What bounds it: instruction issue (52-57 % of the slots at 26-28 of 32 lanes; some 2,100
-// instructions per 32 sub-tests, a quarter of them in the FP64 pipe), with waits for fixed
+// roots_fail on top of that: the 64 meshes 4,913 -> 4,119 us, ten served folds 5,339 -> 4,813 us in
+// all, 12 meshes 303 -> 249 us, the cloth over the sphere 159 -> 138 us, the fold the same (750 us:
+// what it saves there it costs, most of it conversions to fp32 at 8 cycles a warp).
+// What bounds it: instruction issue (52-57 % of the slots at 26-28 of 32 lanes; before roots_fail
+// some 2,100 instructions per 32 sub-tests, a quarter of them in the FP64 pipe), with waits for fixed
 // latencies 2.6, barriers 2.0 and memory 1.6-2.6 warps an issue.  Blocks of 128 threads: 5,219
-// against 5,168 us on the 64 meshes, 801 against 759 us on the fold.
+// against 5,168 us on the 64 meshes, 801 against 759 us on the fold (before roots_fail).
 static constexpr int CCD_BLOCK = 256;
-// resident blocks per SM (64 registers a thread, 54 KB of shared memory a block)
-constexpr int ccd_min_blocks(int bm) { return bm == 1 ? 4 : 2; }
+// resident blocks per SM (80 registers a thread, 54 KB of shared memory a block); four of 64
+// registers spill in roots_fail: 4,637 us on the 64 meshes, 793 us on the fold
+constexpr int ccd_min_blocks(int bm) { return bm == 1 ? 3 : 2; }
 static_assert(CCD_BLOCK % 32 == 0 && CCD_BLOCK <= 1024, "CCD_BLOCK");
 
 constexpr size_t align16(size_t x) { return (x + 15) / 16 * 16; }
@@ -1242,6 +1247,9 @@ k_ccd_narrow(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink 
     // pairs of an intake: a whole block's, or fewer when the grid would not have work for every
     // block (a small call's blocks then end after one batch)
     const int per = min(CCD_BLOCK, max(16, (int)((n + (long long)gridDim.x - 1) / gridDim.x)));
+    // whether the sub-tests' work is worth roots_fail: a block with one short batch only waits for
+    // it (968 triangles 14.3 us without, 16.5 us with it)
+    const bool ahead = per == CCD_BLOCK;
     long long base = (long long)blockIdx.x * per;
 
     // a record of a passing root, past the block's buffer: to the list, or in place
@@ -1341,7 +1349,8 @@ k_ccd_narrow(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink 
                     const MTet<T> tet = load_tet(A.x0, A.x1, it.x & SLOT_MASK, it.y & SLOT_MASK, (it.y >> 28) & 15);
                     cubic_coeffs(tet, cf);
                     go = !(cf[0] == 0 && cf[1] == 0) &&          // (the linear case has no root that is kept)
-                         !cubic_misses<T>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]);
+                         !cubic_misses<T>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]) &&
+                         !(ahead && roots_fail(tet, (it.y >> 28) & 15, cf));
                 }
                 const unsigned m = __ballot_sync(FULL, go);
                 unsigned b0 = 0;

@@ -218,9 +218,9 @@ class Engine:
     def counters(self) -> dict:
         """Synchronises; work counters of the last step: status word, candidate pairs (in a
         collision step, those whose triangles share no vertex), sub-tests with overlapping
-        sub-boxes, roots in [0, 1] filtered, sub-tests solved
-        (each repeated sub-test is solved once for all the pairs that have it) and the
-        candidate pairs with sub-tests to solve."""
+        sub-boxes, roots in [0, 1] put to the filter (those sure to fail it are not),
+        sub-tests solved (each repeated sub-test is solved once for all the pairs that have
+        it) and the candidate pairs with sub-tests to solve."""
         out = (ctypes.c_int32 * 6)()
         N.check(N.lib().ccc_engine_counters(self.handle, out, _stream(self.device)), "ccc_engine_counters")
         return {"status": int(out[0]), "candidates": int(out[1]), "subtests": int(out[2]), "roots": int(out[3]),

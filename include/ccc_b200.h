@@ -106,7 +106,7 @@ int ccc_read_status(const void* ws, int64_t n_mesh, int32_t* out, void* stream);
 
 /* Work counters of the last operation on a workspace (no counterpart in the reference):
  * synchronises the stream and writes 4 ints: status word, candidate pairs, continuous
- * sub-tests solved, roots in [0, 1] filtered. */
+ * sub-tests solved, roots in [0, 1] put to the filter. */
 int ccc_read_counters(const void* ws, int32_t* out, void* stream);
 
 /* Fills up to three device arrays of bytes0 .. bytes2 (multiples of 4) with repeated 8-byte

@@ -144,7 +144,7 @@ int ccc_engine_pack_rows(ccc_engine* e, int64_t* out_rows, void* out_times, int6
  * word, candidate pairs (in a collision step, those whose triangles share no vertex: the
  * others are dropped during the traversal), continuous sub-tests (pair, type) whose swept
  * sub-boxes overlap,
- * roots in [0, 1] filtered, sub-tests solved, and candidate pairs with sub-tests to solve.
+ * roots in [0, 1] put to the filter, sub-tests solved, and candidate pairs with sub-tests to solve.
  * A sub-test that several pairs of a mesh have with the same tetrahedron (a vertex-face
  * test over the triangles around the vertex, an edge-edge test over the two triangles of an
  * edge) is solved once, and its rows or contacts are written for each of those pairs. */
