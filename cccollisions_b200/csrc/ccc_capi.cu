@@ -325,6 +325,7 @@ template <class T> CcdArgs<T> ccd_args(const Prepared& P, const void* x0, const 
     A.x1 = (const T*)x1;
     A.F = P.forest;
     A.mesh_counters = P.mesh_cnt;
+    A.resident = num_sms() * ccd_min_blocks(1);
     // (the nodes are not read after the traversal)
     A.W.expand = (int4*)P.nodes;
     A.W.expand_cap = (int)std::min<int64_t>((P.L.cand - P.L.nodes) / (int64_t)sizeof(int4), (int64_t)1 << 30);

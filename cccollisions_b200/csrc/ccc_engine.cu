@@ -367,6 +367,7 @@ template <class T> CcdArgs<T> engine_args(ccc_engine* e, const Forest& f, const 
     A.x1 = e->at<T>(e->L.x1);
     A.F = f;
     A.mesh_counters = e->at<int>(e->L.mesh_cnt);
+    A.resident = num_sms() * ccd_min_blocks(1);
     A.W = W;
     return A;
 }
@@ -395,6 +396,7 @@ template <class T> int ccd_step(ccc_engine* e, cudaStream_t s) {
     const int batch = SHAPES[e->shape].batch;
     const int g = num_sms() * ccd_min_blocks(batch) * SHAPES[e->shape].narrow;
     CcdArgs<T> A = engine_args<T>(e, t.f, engine_weld(e));
+    A.resident = num_sms() * ccd_min_blocks(batch);
     A.rows = e->at<long long>(e->L.rows);
     A.times = e->at<T>(e->L.times);
     A.max_per_tri = (int)e->maxcol;
