@@ -56,7 +56,8 @@ struct WsHeader {
     int pending_count; // engine staging: pairs left with vertex-face sub-tests to place
     int expand_count;  // engine narrow phase: records for k_ccd_expand (Weld.expand)
     int general;       // imported tree: not the radix tree of the positions
-    int pad[5];
+    int walk_next;     // groups of queries that the walk's warps took after their first
+    int pad[4];
 };
 
 struct __align__(16) TNode {
