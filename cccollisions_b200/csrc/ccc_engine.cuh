@@ -1554,37 +1554,45 @@ __device__ __forceinline__ bool to_fix(double x, long long& q) {
     return true;
 }
 
+// the impulse of one point of a contact as the seven words of the vertex slot it goes to (the slot,
+// or -1 when it goes nowhere)
+template <class T>
+__device__ __forceinline__ long long loop_point(const MTet<T>& tet, long long gi, long long gj, int k,
+                                                const Contact<T>& ct, const ImpulseScale<T>& sc, int pt, int vbase,
+                                                int nv, const int* faces, int* status, long long* q) {
+    V3<T> imp, idx;
+    impulse_point(tet, k, pt, ct, sc, imp, idx);
+    const bool ok = to_fix((double)idx.x, q[0]) && to_fix((double)idx.y, q[1]) && to_fix((double)idx.z, q[2]) &&
+                    to_fix((double)imp.x, q[3]) && to_fix((double)imp.y, q[4]) && to_fix((double)imp.z, q[5]);
+    if (!ok) {
+        atomicOr(status, ST_NONFINITE);
+        return -1;
+    }
+    const int vid = __ldg(faces + (tet_side(k, pt) ? gj : gi) * 3 + tet_corner(k, pt));
+    if (vid < 0 || vid >= nv) {
+        atomicOr(status, ST_MALFORMED_TREE);
+        return -1;
+    }
+    q[6] = 1;
+    return (long long)vbase + vid;
+}
+
 // the contact's four point impulses, added to the vertices they move
 template <class T>
 __device__ __forceinline__ void loop_impulse(const MTet<T>& tet, long long gi, long long gj, int k, T root,
                                              const Contact<T>& ct, int m, const int* faces, const VertTable& vt,
                                              long long* acc, int* status) {
-    ImpulseScale<T> sc = impulse_scale(ct, root);
+    const ImpulseScale<T> sc = impulse_scale(ct, root);
     const int vbase = __ldg(vt.vpoff + m);
     const int nv = __ldg(vt.vvoff + m + 1) - __ldg(vt.vvoff + m);
 #pragma unroll 1
     for (int pt = 0; pt < 4; ++pt) {
-        V3<T> imp, idx;
-        impulse_point(tet, k, pt, ct, sc, imp, idx);
-        long long tri = tet_side(k, pt) ? gj : gi;
-        int corner = tet_corner(k, pt);
-        long long q[6];
-        bool ok = to_fix((double)idx.x, q[0]) && to_fix((double)idx.y, q[1]) && to_fix((double)idx.z, q[2]) &&
-                  to_fix((double)imp.x, q[3]) && to_fix((double)imp.y, q[4]) && to_fix((double)imp.z, q[5]);
-        if (!ok) {
-            atomicOr(status, ST_NONFINITE);
-            continue;
-        }
-        int vid = __ldg(faces + tri * 3 + corner);
-        if (vid < 0 || vid >= nv) {
-            atomicOr(status, ST_MALFORMED_TREE);
-            continue;
-        }
-        long long vslot = (long long)vbase + vid;
+        long long q[7];
+        const long long vslot = loop_point(tet, gi, gj, k, ct, sc, pt, vbase, nv, faces, status, q);
+        if (vslot < 0) continue;
         unsigned long long* a = reinterpret_cast<unsigned long long*>(acc + vslot * 8);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) atomicAdd(a + c, (unsigned long long)q[c]);
-        atomicAdd(a + 6, 1ull);
+        for (int c = 0; c < 7; ++c) atomicAdd(a + c, (unsigned long long)q[c]);
     }
 }
 
@@ -1604,6 +1612,46 @@ template <class T> struct LoopSink {
         const unsigned peers = __match_any_sync(__activemask(), m);
         if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(contacts + __ldg(F.sid + m), __popc(peers));
         loop_impulse(tet, gi, gj, k, root, ct, m, faces, vt, acc, status);
+    }
+    // The contacts of a warp's lanes (of those with `valid`), all lanes taking part: the seven
+    // words of a vertex are added by neighbouring lanes, in two sectors.  Ten served folds' 12
+    // iterations 459 -> 403 us, and 318 us with four blocks an SM (128 registers; three 350, five
+    // 367 us).
+    static constexpr int MIN_BLOCKS = 4;
+    struct Points {
+        unsigned long long v[32 * 7];
+        long long at[32];
+    };
+    __device__ __forceinline__ void add_all(bool valid, const MTet<T>& tet, long long gi, long long gj, int k, T root,
+                                            const Contact<T>& ct, const Forest& F, int M, int* status, Points& S) const {
+        const int lane = threadIdx.x & 31;
+        ImpulseScale<T> sc;
+        int vbase = 0, nv = 0;
+        if (valid) {
+            const int m = forest_slot_mesh(F, M, gi);
+            // (one atomic for the lanes of a mesh, whose contacts all go to one word: k_ccd_contacts
+            // 118 -> 39 us an iteration of ten served folds)
+            const unsigned peers = __match_any_sync(__activemask(), m);
+            if (lane == __ffs(peers) - 1) atomicAdd(contacts + __ldg(F.sid + m), __popc(peers));
+            sc = impulse_scale(ct, root);
+            vbase = __ldg(vt.vpoff + m);
+            nv = __ldg(vt.vvoff + m + 1) - __ldg(vt.vvoff + m);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int pt = 0; pt < 4; ++pt) {
+            long long at = -1;
+            if (valid) at = loop_point(tet, gi, gj, k, ct, sc, pt, vbase, nv, faces, status, (long long*)S.v + 7 * lane);
+            S.at[lane] = at;
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {
+                const int l = (lane + 32 * r) / 7, w = lane + 32 * r - 7 * l;
+                const long long o = S.at[l];
+                if (o >= 0) atomicAdd(reinterpret_cast<unsigned long long*>(acc) + o * 8 + w, S.v[7 * l + w]);
+            }
+            __syncwarp();
+        }
     }
 };
 

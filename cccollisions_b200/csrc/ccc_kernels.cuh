@@ -556,6 +556,46 @@ template <class T> struct CornerSink {
                                         const Contact<T>& ct, const Forest&, int, int*) const {
         apply_impulse(tet, gi, gj, k, root, ct, dv, dx, cnt);
     }
+    // The contacts of a warp's lanes (of those with `valid`), all lanes taking part: the three
+    // components of a point are added by neighbouring lanes, so that an instruction touches
+    // some 16 sectors instead of 32.  What bounds k_ccd_contacts is those sectors in L2: 523 k
+    // contacts (fp64) 82 -> 52 us, 34 k listed ones (fp32) 7.4 -> 5.4 us.
+    static constexpr int MIN_BLOCKS = 1;    // k_ccd_contacts: 3 or 4 a SM (168, 128 registers) 55 us
+    struct Points {
+        T v[32 * 7];            // change of velocity and of position per lane, odd stride
+        long long at[32];
+    };
+    __device__ __forceinline__ void add_all(bool valid, const MTet<T>& tet, long long gi, long long gj, int k, T root,
+                                            const Contact<T>& ct, const Forest&, int, int*, Points& S) const {
+        const int lane = threadIdx.x & 31;
+        ImpulseScale<T> sc;
+        if (valid) sc = impulse_scale(ct, root);
+#pragma unroll
+        for (int pt = 0; pt < 4; ++pt) {
+            long long corner = -1;
+            if (valid) {
+                V3<T> imp, idx;
+                impulse_point(tet, k, pt, ct, sc, imp, idx);
+                corner = (tet_side(k, pt) ? gj : gi) * 3 + tet_corner(k, pt);
+                T* v = S.v + 7 * lane;
+                v[0] = imp.x; v[1] = imp.y; v[2] = imp.z;
+                v[3] = idx.x; v[4] = idx.y; v[5] = idx.z;
+                atomicAdd(cnt + corner, 1);
+            }
+            S.at[lane] = corner;
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const int l = (lane + 32 * r) / 3, d = lane + 32 * r - 3 * l;
+                const long long at = S.at[l];
+                if (at >= 0) {
+                    atomicAdd(dv + at * 3 + d, S.v[7 * l + d]);
+                    atomicAdd(dx + at * 3 + d, S.v[7 * l + 3 + d]);
+                }
+            }
+            __syncwarp();
+        }
+    }
 };
 
 // Continuous narrow phase (collisions_continuous.cu:14-765, collisions_impulses.cu:24-1067),
@@ -1194,15 +1234,21 @@ template <class T, class Sink, int LIB>
 cudaError_t launch_ccd_contacts(int grid, cudaStream_t s, const CcdArgs<T>& A, const Sink& sink);
 
 #ifdef CCC_NARROW_TU
-// the contact of one root (i, j, type, time) and its impulses
+// the contact of one root (i, j, type, time)
 template <class T, class Sink, int LIB>
-__device__ __forceinline__ void contact_of_root(const CcdArgs<T>& A, const Sink& sink, int i, int j, int k, T root) {
-    const MTet<T> tet = load_tet(A.x0, A.x1, i, j, k);
+__device__ __forceinline__ Contact<T> contact_of_tet(const MTet<T>& tet, const Sink& sink, int i, int j, int k, T root) {
     T mq[4];
 #pragma unroll
     for (int pt = 0; pt < 4; ++pt)
         mq[pt] = sink.masses[(long long)(tet_side(k, pt) ? j : i) * 3 + tet_corner(k, pt)];
-    const Contact<T> ct = contact<T, LIB>(tet, k, root, mq);
+    return contact<T, LIB>(tet, k, root, mq);
+}
+
+// ... and its impulses
+template <class T, class Sink, int LIB>
+__device__ __forceinline__ void contact_of_root(const CcdArgs<T>& A, const Sink& sink, int i, int j, int k, T root) {
+    const MTet<T> tet = load_tet(A.x0, A.x1, i, j, k);
+    const Contact<T> ct = contact_of_tet<T, Sink, LIB>(tet, sink, i, j, k, root);
     sink.add(tet, i, j, k, root, ct, A.F, forest_size(A.F), &A.hdr->status);
 }
 
@@ -1567,18 +1613,31 @@ cudaError_t launch_ccd_narrow(int grid, cudaStream_t s, const CcdArgs<T>& A, con
 }
 
 // The contacts of the roots that passed the filter in k_ccd_narrow, one record a thread: the
-// contact's registers and code stay out of the narrow kernel, and its lanes are full.  523 k
-// contacts take 82 us (fp64; their tetrahedra's gathers and 28 atomics each).
+// contact's registers and code stay out of the narrow kernel, and its lanes are full.  The sums
+// are added by the warp together (Sink::add_all).
 static constexpr int CONTACT_THREADS = 128;
 template <class T, class Sink, int LIB>
-__global__ void __launch_bounds__(CONTACT_THREADS)
+__global__ void __launch_bounds__(CONTACT_THREADS, Sink::MIN_BLOCKS)
 k_ccd_contacts(const __grid_constant__ CcdArgs<T> A, const __grid_constant__ Sink sink) {
     chain_begin();
+    __shared__ typename Sink::Points S[CONTACT_THREADS / 32];
+    const int lane = threadIdx.x & 31;
     const int n = min(*(volatile int*)&A.hdr->expand_count, A.W.expand_cap);
-    for (int c = blockIdx.x * CONTACT_THREADS + threadIdx.x; c < n; c += gridDim.x * CONTACT_THREADS) {
-        const int4 rec = A.W.expand[c];
-        contact_of_root<T, Sink, LIB>(A, sink, rec.x & SLOT_MASK, rec.y & SLOT_MASK, (rec.y >> 28) & 15,
-                                      (T)__hiloint2double(rec.w, rec.z));
+    for (int c = blockIdx.x * CONTACT_THREADS + threadIdx.x; c - lane < n; c += gridDim.x * CONTACT_THREADS) {
+        int i = 0, j = 0, k = 0;
+        T root = T(0);
+        MTet<T> tet;
+        Contact<T> ct;
+        if (c < n) {
+            const int4 rec = A.W.expand[c];
+            i = rec.x & SLOT_MASK;
+            j = rec.y & SLOT_MASK;
+            k = (rec.y >> 28) & 15;
+            root = (T)__hiloint2double(rec.w, rec.z);
+            tet = load_tet(A.x0, A.x1, i, j, k);
+            ct = contact_of_tet<T, Sink, LIB>(tet, sink, i, j, k, root);
+        }
+        sink.add_all(c < n, tet, i, j, k, root, ct, A.F, forest_size(A.F), &A.hdr->status, S[threadIdx.x >> 5]);
     }
 }
 
@@ -1712,20 +1771,35 @@ k_impulses_from_rows(const long long* __restrict__ rows, const T* __restrict__ r
                      const T* __restrict__ x0, const T* __restrict__ x1, const T* __restrict__ masses,
                      T* __restrict__ dv_out, T* __restrict__ dx_out, int* __restrict__ cnt_out) {
     chain_begin();
-    long long total = (long long)B * N;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < total;
+    using Sink = CornerSink<T>;
+    __shared__ typename Sink::Points S[NARROW_THREADS / 32];
+    const Sink sink{masses, dv_out, dx_out, cnt_out};
+    const int lane = threadIdx.x & 31;
+    const long long total = (long long)B * N;
+    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r - lane < total;
          r += (long long)gridDim.x * blockDim.x) {
-        long long b = r / N;
-        long long i = rows[r * 3 + 0], j = rows[r * 3 + 1], kk = rows[r * 3 + 2];
-        if (i < 0 || j < 0 || i >= F || j >= F || kk < 0 || kk >= 15) continue;
-        int k = (int)kk;
-        long long gi = b * F + i, gj = b * F + j;
-        T root = roots[r];
-        MTet<T> tet = load_tet(x0, x1, gi, gj, k);
-        T mq[4];
-        for (int pt = 0; pt < 4; ++pt) mq[pt] = masses[(tet_side(k, pt) ? gj : gi) * 3 + tet_corner(k, pt)];
-        Contact<T> ct = contact<T, LIB>(tet, k, root, mq);
-        apply_impulse(tet, gi, gj, k, root, ct, dv_out, dx_out, cnt_out);
+        long long gi = 0, gj = 0;
+        int k = 0;
+        T root = T(0);
+        MTet<T> tet;
+        Contact<T> ct;
+        bool valid = r < total;
+        if (valid) {
+            const long long b = r / N;
+            const long long i = rows[r * 3 + 0], j = rows[r * 3 + 1], kk = rows[r * 3 + 2];
+            valid = !(i < 0 || j < 0 || i >= F || j >= F || kk < 0 || kk >= 15);
+            if (valid) {
+                k = (int)kk;
+                gi = b * F + i;
+                gj = b * F + j;
+                root = roots[r];
+                tet = load_tet(x0, x1, gi, gj, k);
+                T mq[4];
+                for (int pt = 0; pt < 4; ++pt) mq[pt] = masses[(tet_side(k, pt) ? gj : gi) * 3 + tet_corner(k, pt)];
+                ct = contact<T, LIB>(tet, k, root, mq);
+            }
+        }
+        if (__any_sync(0xffffffffu, valid)) sink.add_all(valid, tet, gi, gj, k, root, ct, Forest{}, 0, nullptr, S[threadIdx.x >> 5]);
     }
 }
 
