@@ -62,7 +62,9 @@ METRIC = "triangle-steps/sec batched+served vs plain (exact pair sets); p50/p99 
 UNIT = "triangle-steps/s"
 MAXC, MAXCOL = 32, 16            # no candidate overflow on any of the 64 meshes
 FP64_PEAK_NOMINAL_GFLOPS = 37000.0   # B200 FP64 datasheet figure (not measured here)
-FLOPS_PER_SUBTEST = 252          # coefficients 162 + Cardano and filter 90 (transcendentals as 1)
+# coefficients 162 + Cardano and filter 90 (transcendentals as 1): the reference's work on each
+# sub-test, most of which end after the coefficients here
+FLOPS_PER_SUBTEST = 252
 # DRAM bytes (read + write) of one k_ccd_narrow launch per sub-test solved, from ncu's
 # dram__bytes_read.sum + dram__bytes_write.sum on the 32-mesh batched step; the 64-mesh
 # launch is too large for a full capture, so its traffic is this figure times its own count.
@@ -406,7 +408,7 @@ def run_ours(args, rank, world, dev):
     # both ends of the step (2 x 2 x 72 bytes); it writes 32 bytes per row
     narrow_bytes = cnt["live_pairs"] * (16 + 2 * 2 * 72) + int(sum(nrow)) * 32
     achieved = narrow_bytes / (per_launch / 1e3) / 1e9 if dname == "k_ccd_narrow" else None
-    # the refit is two passes (block-local, then the climbs that leave a block)
+    # the refit is two passes (block-local, then the levels above the blocks)
     r1 = kern.get("k_engine_refit", (float("nan"), 1))
     r2 = kern.get("k_engine_refit_front", (0.0, 1))
     refit_ms = r1[0] / r1[1] + r2[0] / r2[1]

@@ -6,8 +6,9 @@
 // position order, bboxes row = (min xyz, max xyz), tree row = (parent, left, right, tri id),
 // -1 for "none".  Mesh m's rows start at 2*moff[m] - m.
 //
-// Traversal works on a compact copy of the internal nodes (TNode, 64 B): both child boxes
-// rounded outward to fp32 plus child references, so one node visit is four 16-byte loads.
+// Traversal works on copies of the internal nodes with their child boxes rounded outward to fp32
+// and child references: four-wide QNodes (ccc_walk.cuh), or binary TNodes (64 B, four 16-byte
+// loads a visit) in workspaces without room for those.
 #pragma once
 
 #include <atomic>
@@ -48,7 +49,7 @@ struct WsHeader {
     int status;
     int cand_count;
     int subtests;      // continuous sub-tests (pair, type) whose swept sub-boxes overlap
-    int roots;         // roots in [0, 1] filtered
+    int roots;         // roots in [0, 1] put to the filter
     int front;         // engine refit: climbs handed from the block pass to the global pass
     int solved;        // sub-tests solved (fewer than subtests when repeated ones are shared)
     int fan_cursor;    // engine corner classes: member list slots handed out
