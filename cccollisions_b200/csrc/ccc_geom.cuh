@@ -778,10 +778,10 @@ template <class T> __device__ __forceinline__ bool filter_fails(const FilterFram
 //    q monotone with a root t' in between: t or |t - t'| is at most 2 (m + |d|) / (slope t').
 // Everything else goes to the solver, as do calls too small for the time to matter (the caller).
 //
-// Measured: none of 2^32 moving tetrahedra of twelve families (flat, far from the origin, nearly
+// Measured: none of 2^33 moving tetrahedra of twelve families (flat, far from the origin, nearly
 // rigid, parallel edges, roots at the filter's borders, degenerate, ..) that it drops has a root
 // that passes, in either precision and with both sets of elementary functions; three certain roots
-// left at most 5e-16 |a| r^3 in 2^31 cubics.  It drops 56 % of the sub-tests of the 64 meshes and 65 %
+// left at most 6e-16 |a| r^3 in 2^31 cubics.  It drops 56 % of the sub-tests of the 64 meshes and 65 %
 // of the cloth over the sphere (flat at the start), 23 % of the fold's 13.0 M.
 template <class T> __device__ __forceinline__ bool roots_fail(const MTet<T>& tet, int k, const T cf[4]) {
     const double a = cf[0], b = cf[1], c = cf[2], d = cf[3];
