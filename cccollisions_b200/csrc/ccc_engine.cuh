@@ -756,9 +756,9 @@ __device__ __forceinline__ float hmax4(float4 v) { return fmaxf(fmaxf(v.x, v.y),
 //  * pass 1 (k_engine_refit_local): a block takes REFIT_THREADS consecutive leaf positions of a
 //    mesh and refits every node whose leaf range lies inside them, in shared memory, round by
 //    round;
-//  * pass 2 (k_engine_refit_top): the nodes above the blocks ("top" nodes, some nine a block), one
-//    block of threads a mesh, again in shared memory, level by level in an order that the build
-//    lays down (k_refit_plan).
+//  * pass 2 (k_engine_refit_top): the nodes above the blocks ("top" nodes, some nine a block), a
+//    cluster of TOP_CLUSTER blocks a mesh, again in shared memory, level by level in an order that
+//    the build lays down (k_refit_plan).
 // A mesh with more top nodes than pass 2 holds (TOP_CAP) is finished by climbs instead: in pass 1
 // an item whose parent is a top node hands that arrival over through the frontier list, and at
 // each node the second arrival (the one that finds the global counter odd, and so the node's
@@ -1039,6 +1039,9 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_end[TOP_LEVELS + 1];
     const cg::cluster_group cluster = cg::this_cluster();
+    // (a block's shared memory may be written by the others only once it has begun, which
+    // chain_begin, a wait for the kernel before, does not say)
+    cluster.sync();
     TopShared& S = *reinterpret_cast<TopShared*>(cluster.map_shared_rank(smem, 0));      // the first block's
     const int rank = (int)cluster.block_rank();
     // (warp by warp over the blocks, so that a small mesh's nodes spread over them too)
