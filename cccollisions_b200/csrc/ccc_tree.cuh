@@ -159,9 +159,10 @@ k_bvh_levels(const T* __restrict__ x0, const T* __restrict__ x1, int n, int chun
 // tree built from them) the intersection is the slot's own box.
 //
 // The rightmost leaf position below a node, which the order rule needs, is known without a
-// climb when the children are those of the radix tree of the positions (bvh and bvh_motion,
-// the reference's too); a tree with any other child raises hdr->general, and
-// k_import_rightmost_wide then climbs for all of them.  Measured for a bvh_motion tree of 52,738
+// climb when the tree is the radix tree of the positions (bvh and bvh_motion, the reference's
+// too); one with any other child, or with a child that names another parent, raises
+// hdr->general, and k_import_rightmost_wide then climbs for all of them and reports a parent
+// column that does not lead to the root.  Measured for a bvh_motion tree of 52,738
 // triangles (fp64): binary nodes and climbs 34 us, four-wide nodes and no climb 10 us.
 template <class T> __device__ __forceinline__ void box_outward(const T* p, float lo[3], float hi[3]) {
 #pragma unroll
@@ -247,7 +248,8 @@ __global__ void k_import_wide(int n, int meshes, const T* __restrict__ bboxes, c
         }
     };
     const int c0 = child(k, 0), c1 = child(k, 1);
-    if (c0 != regular.x || c1 != regular.y) hdr->general = 1;
+    // (the parents too: a wrong one is for the climbs to find)
+    if (c0 != regular.x || c1 != regular.y || __ldg(tr + c0 * 4LL) != k || __ldg(tr + c1 * 4LL) != k) hdr->general = 1;
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
         const int c = side ? c1 : c0;
