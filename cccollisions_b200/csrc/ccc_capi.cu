@@ -246,10 +246,18 @@ int bvh_impl(const void* tri, const void* tri_next, int64_t B, int64_t F, void* 
         const int64_t blocks = (F + ((int64_t)1 << level) - 1) >> level;      // of 2^level positions
         const int log_threads = level == 0 ? 8 : 10;
         const int chunks = grid_for(blocks, 1 << log_threads);
+        // threads a mesh: as many as it needs, or more while every SM does not have a block
+        int log_mesh = 0;
+        while (log_mesh < log_threads &&
+               (((int64_t)1 << log_mesh) < blocks || grid_for(B, 1 << (log_threads - log_mesh)) < num_sms()))
+            ++log_mesh;
+        const int grid = grid_for(B, 1 << (log_threads - log_mesh)) * chunks;
         if (log_threads == 8)
-            CCC_LAUNCH("k_bvh_levels", s, launch_chain((unsigned)(B * chunks), 1 << 8, 0, s, k_bvh_levels<T, 8>, x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
+            CCC_LAUNCH("k_bvh_levels", s, launch_chain(grid, 1 << 8, 0, s, k_bvh_levels<T, 8>, x0, x1, (int)B, (int)F, chunks,
+                                                       log_mesh, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
         else
-            CCC_LAUNCH("k_bvh_levels", s, launch_chain((unsigned)(B * chunks), 1 << 10, 0, s, k_bvh_levels<T, 10>, x0, x1, (int)F, chunks, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
+            CCC_LAUNCH("k_bvh_levels", s, launch_chain(grid, 1 << 10, 0, s, k_bvh_levels<T, 10>, x0, x1, (int)B, (int)F, chunks,
+                                                       log_mesh, level, (T*)bboxes, (long long*)tree, hdr, mesh_cnt));
         CCC_LAUNCH_CHECK();
         level += log_threads;
     }

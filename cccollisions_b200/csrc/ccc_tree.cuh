@@ -64,6 +64,10 @@ template <class T> __device__ __forceinline__ Box<T> shfl_down_box(const Box<T>&
 // left in bboxes), LOG_THREADS levels a launch: up to five by shuffles, the rest over the
 // warps' boxes in shared memory.  An internal node unites its children in the order left,
 // right (CreateHierarchy, build_bvh.cu:145-209).
+// A mesh takes 2^log_mesh threads of a block (with more blocks of positions than a block of
+// threads, `chunks` whole ones): a block for every mesh leaves most threads idle on large batches
+// of tiny meshes (bvh of 1,000,000 meshes of two triangles, fp32: 1,301 -> 119 us; 30,000 of 300
+// triangles 546 -> 388 us).
 //
 // The levels are known in advance, so no thread climbs with arrival counters (a device-wide
 // fence, an atomic and two dependent reads through L2 a level), and the topology needs no
@@ -72,22 +76,23 @@ template <class T> __device__ __forceinline__ Box<T> shfl_down_box(const Box<T>&
 // launch latency and, at the large sizes, the row-wise stores.
 template <class T, int LOG_THREADS>
 __global__ void __launch_bounds__(1 << LOG_THREADS)
-k_bvh_levels(const T* __restrict__ x0, const T* __restrict__ x1, int n, int chunks, int level, T* bboxes,
-             long long* __restrict__ tree, WsHeader* hdr, int* __restrict__ mesh_cnt) {
+k_bvh_levels(const T* __restrict__ x0, const T* __restrict__ x1, int meshes, int n, int chunks, int log_mesh, int level,
+             T* bboxes, long long* __restrict__ tree, WsHeader* hdr, int* __restrict__ mesh_cnt) {
     chain_begin();
     constexpr int THREADS = 1 << LOG_THREADS;
     __shared__ T wbox[6][THREADS / 32];
-    const int m = blockIdx.x / chunks, t = threadIdx.x, lane = t & 31;
-    const long long lo64 = ((long long)(blockIdx.x - m * chunks) * THREADS + t) << level;
+    const int t = threadIdx.x, lane = t & 31, group = blockIdx.x / chunks;
+    const int m = (group << (LOG_THREADS - log_mesh)) + (t >> log_mesh);
+    const long long lo64 = ((long long)(blockIdx.x - group * chunks) * THREADS + (t & ((1 << log_mesh) - 1))) << level;
     const long long base = (long long)m * (2LL * n - 1);
     T* bb = bboxes + base * 6;
     long long* tr = tree + base * 4;
-    const bool live = lo64 < n;
+    const bool live = m < meshes && lo64 < n;
     const int lo = live ? (int)lo64 : 0;
     if (level == 0) {
         // the workspace's status and counters, which no part of the build can raise
         if (blockIdx.x == 0 && t < (int)(sizeof(WsHeader) / sizeof(int))) reinterpret_cast<int*>(hdr)[t] = 0;
-        if (lo64 == 0) mesh_cnt[m] = 0;
+        if (live && lo64 == 0) mesh_cnt[m] = 0;
     }
     Box<T> b;
     b.lo = b.hi = mk<T>(T(0), T(0), T(0));
