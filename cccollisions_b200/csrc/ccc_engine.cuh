@@ -911,6 +911,25 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
     }
 }
 
+// The first of the meshes m, m + step, m + 2 step, .. for which `wanted` holds (M: none of them), found
+// by a block of TOP_THREADS together.  A mesh of at most REFIT_THREADS triangles has no top nodes,
+// and going over 20,000 of 12 triangles one by one took k_engine_refit_top 408 us (14 so).
+template <class Fn> __device__ __forceinline__ int next_mesh(int m, int M, int step, unsigned* s_first, Fn&& wanted) {
+    static_assert(TOP_THREADS == 32 * 32, "a warp reads the warps' results");
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (long long from = m; from < M; from += (long long)step * TOP_THREADS) {
+        const long long at = from + (long long)step * threadIdx.x;
+        const unsigned w = __reduce_min_sync(FULL, at < M && wanted((int)at) ? threadIdx.x : TOP_THREADS);
+        if (lane == 0) s_first[threadIdx.x >> 5] = w;
+        __syncthreads();
+        const unsigned first = __reduce_min_sync(FULL, s_first[lane]);
+        __syncthreads();
+        if (first < TOP_THREADS) return (int)(from + (long long)step * first);
+    }
+    return M;
+}
+
 // The order of pass 2, laid down with the topology: the top nodes of a mesh by height above the
 // blocks (counting sort; a height is found in rounds, one more than the children's), each with
 // where its children's boxes are and its own slot code.  A child below comes from slots that
@@ -933,13 +952,21 @@ k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ 
              int* __restrict__ top_index, int2* __restrict__ top_child, int* __restrict__ status) {
     chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ unsigned s_first[32];
     PlanShared& S = *reinterpret_cast<PlanShared*>(smem);
     const int M = forest_size(F);
+    auto planned = [&](int m) {
+        const int nt = ntop[__ldg(F.sid + m)].x;
+        return nt > 0 && nt <= TOP_CAP;
+    };
     for (int m = blockIdx.x; m < M; m += gridDim.x) {
+        if (!planned(m)) {                              // (block-uniform)
+            m = next_mesh(m + gridDim.x, M, gridDim.x, s_first, planned);
+            if (m >= M) break;
+        }
         const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
         const int sid = __ldg(F.sid + m);
         const int nt = ntop[sid].x;
-        if (nt == 0 || nt > TOP_CAP) continue;         // (block-uniform)
         // where child c's box is: a slot code, ~ (index of a top node), or TOP_PAIR | the first of two
         // slots; the last code of all for a malformed tree
         auto where = [&](int c) {
@@ -1038,6 +1065,7 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
     chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_end[TOP_LEVELS + 1];
+    __shared__ unsigned s_first[32];
     const cg::cluster_group cluster = cg::this_cluster();
     // (a block's shared memory may be written by the others only once it has begun, which
     // chain_begin, a wait for the kernel before, does not say)
@@ -1046,13 +1074,19 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
     const int rank = (int)cluster.block_rank();
     // (warp by warp over the blocks, so that a small mesh's nodes spread over them too)
     const int t0 = ((threadIdx.x >> 5) * TOP_CLUSTER + rank) * 32 + (threadIdx.x & 31);
-    const int M = forest_size(F);
-    for (int m = blockIdx.x / TOP_CLUSTER; m < M; m += gridDim.x / TOP_CLUSTER) {
+    const int M = forest_size(F), clusters = gridDim.x / TOP_CLUSTER;
+    auto refit = [&](int m) {
+        const int sid = __ldg(F.sid + m), nt = __ldg(&ntop[sid].x);
+        return nt > 0 && nt <= TOP_CAP && !(mflags && (__ldg(mflags + sid) & MF_DONE));
+    };
+    for (int m = blockIdx.x / TOP_CLUSTER; m < M; m += clusters) {
+        if (!refit(m)) {                                // (cluster-uniform)
+            m = next_mesh(m + clusters, M, clusters, s_first, refit);
+            if (m >= M) break;
+        }
         const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
-        const int sid = __ldg(F.sid + m);
-        const int2 plan = __ldg(ntop + sid);
+        const int2 plan = __ldg(ntop + __ldg(F.sid + m));
         const int nt = plan.x, levels = min(plan.y, TOP_LEVELS);
-        if (nt == 0 || nt > TOP_CAP || (mflags && (__ldg(mflags + sid) & MF_DONE))) continue;     // (cluster-uniform)
         QNode* qn = qnodes + po;
         if (rank == 0 && threadIdx.x <= levels) s_end[threadIdx.x] = min(__ldg(top_index + po + min(threadIdx.x, n - 1)), nt);
         for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) {
