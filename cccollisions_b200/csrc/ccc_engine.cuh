@@ -771,22 +771,65 @@ static constexpr int TOP_THREADS = 1024;
 static constexpr int TOP_CLUSTER = 4;          // blocks of a mesh (8: 105 against 88 us on 64 meshes, 13 against 14 served)
 static constexpr int TOP_LEVELS = 64;          // levels above the blocks (a tree has at most 62)
 
+// A piece of pass 1: work items [from, to), at most REFIT_THREADS, which are a chunk of mesh `first`
+// or several whole meshes from it.
+struct RefitPiece {
+    int from, to, first;
+    bool several;
+};
+
 // The chunks of pass 1 over the active table, numbered with at most one empty number a mesh:
 // mesh m's first is voff[m] / REFIT_THREADS + m.
-__device__ __forceinline__ int refit_chunk_mesh(const Forest& F, int M, int g) {
+__device__ __forceinline__ bool refit_chunk(const Forest& F, int M, int g, RefitPiece& piece) {
     int lo = 0, hi = M - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (__ldg(F.voff + mid) / REFIT_THREADS + mid <= g) lo = mid;
         else hi = mid - 1;
     }
-    return lo;
+    const int vo = __ldg(F.voff + lo), end = __ldg(F.voff + lo + 1);
+    const int from = vo + (g - (vo / REFIT_THREADS + lo)) * REFIT_THREADS;
+    piece = RefitPiece{from, min(from + REFIT_THREADS, end), lo, false};
+    return from < end;
 }
 
-// pass 1: leaf positions [blo, blo + REFIT_THREADS) of a mesh and the internal nodes whose leaf
-// range lies inside them ("local" nodes; a node's index lies in its range, so these are the nodes
-// at the same positions).  The boxes live in shared memory, indexed by position - blo: the
-// leaves' from the soups, the local nodes' computed in rounds (a node whose two children were
+// Where the meshes are that small that most chunks would hold a few triangles: the pieces of the
+// window of work items [g W, (g + 1) W), half as wide as a block.  The meshes that begin in it
+// take its one or two pieces: all but the last of them end in it, and go together with the last
+// one's first chunk when they fit.  A chunk further on in a mesh is its window's, but a last one
+// shorter than W, which the mesh's next or another may share a window with, is the window before's,
+// where the mesh has nothing else.
+static constexpr int REFIT_WINDOW = REFIT_THREADS / 2;
+__device__ __forceinline__ int refit_window(const Forest& F, int M, int total, int g, RefitPiece piece[2]) {
+    const int begin = g * REFIT_WINDOW, stop = min(begin + REFIT_WINDOW, total);
+    int m = find_mesh(F.voff, M, begin, 0);
+    const int vo = __ldg(F.voff + m);
+    if (vo < begin) {
+        const int end = __ldg(F.voff + m + 1), j = g - vo / REFIT_WINDOW;      // (1 or more)
+        const int from = vo + (j + 1) / 2 * REFIT_THREADS;
+        if (from < end && (j & 1) == (end - from < REFIT_WINDOW)) {
+            piece[0] = RefitPiece{from, min(from + REFIT_THREADS, end), m, false};
+            return 1;
+        }
+        if (end >= stop) return 0;
+        ++m;
+    }
+    const int last = find_mesh(F.voff, M, stop - 1, 0);
+    const int from = __ldg(F.voff + m), at = __ldg(F.voff + last);
+    const int to = min(at + REFIT_THREADS, __ldg(F.voff + last + 1));
+    if (to - from <= REFIT_THREADS) {
+        piece[0] = RefitPiece{from, to, m, m < last};
+        return 1;
+    }
+    piece[0] = RefitPiece{at, to, last, false};
+    piece[1] = RefitPiece{from, at, m, true};
+    return 2;
+}
+
+// pass 1: REFIT_THREADS leaf positions of a mesh, from a multiple of REFIT_THREADS, or all of several
+// small meshes, and the internal nodes whose leaf range lies inside them ("local" nodes; a node's
+// index lies in its range, so these are the nodes at the same positions).  The boxes live in
+// shared memory, indexed by work item - first one: the leaves' from the soups, the local nodes' computed in rounds (a node whose two children were
 // done in earlier rounds takes the union of their boxes; fminf / fmaxf skip NaN, so the order
 // of the unions does not matter).  Then every leaf and every local even-depth node writes its
 // box into its QNode slot.
@@ -802,18 +845,30 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
     __shared__ float s_nlo[3][REFIT_THREADS], s_nhi[3][REFIT_THREADS];    // local node boxes
     __shared__ unsigned short s_done[REFIT_THREADS];    // round a local node was done in (0: not yet)
     const int M = forest_size(F);
-    const int chunks = M > 0 ? __ldg(F.voff + M) / REFIT_THREADS + M : 0;
+    const int total = M > 0 ? __ldg(F.voff + M) : 0;
+    // (windows where the average mesh is smaller than a block: 20,000 meshes of 12 triangles 176 -> 48
+    // us, 5,000 of 200 triangles 130 -> 135 us)
+    const bool windows = total / REFIT_THREADS < M;
+    const int pieces = windows ? (total + REFIT_WINDOW - 1) / REFIT_WINDOW : total / REFIT_THREADS + M;
     const int t = threadIdx.x;
-    for (int g = blockIdx.x; g < chunks; g += gridDim.x) {
-        const int m = refit_chunk_mesh(F, M, g);
+    RefitPiece piece[2];
+    int left = 0;
+    for (int g = blockIdx.x; g < pieces || left > 0;) {
+        if (left == 0) {
+            left = windows ? refit_window(F, M, total, g, piece) : (int)refit_chunk(F, M, g, piece[0]);
+            g += gridDim.x;
+            if (left == 0) continue;
+        }
+        const RefitPiece P = piece[--left];
+        const int v = P.from + t;
+        const int m = P.several && v < P.to ? find_mesh(F.voff, M, v, 0) : P.first;
         const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
         const int sid = __ldg(F.sid + m);
-        const int blo = (g - (vo / REFIT_THREADS + m)) * REFIT_THREADS;
-        // (an empty number, a mesh that has stopped: the whole block)
-        if (blo >= n || n < 2 || (mflags && (__ldg(mflags + sid) & MF_DONE))) continue;
+        const bool skip = n < 2 || (mflags && (__ldg(mflags + sid) & MF_DONE));
+        if (skip && !P.several) continue;                // (the whole block)
         const bool climbs = __ldg(&ntop[sid].x) > TOP_CAP;
-        const int p = blo + t;
-        bool live = p < n, node_local = false;
+        const int p = v - vo, first = P.from - vo;       // first: the piece's first item, in the mesh's positions
+        bool live = v < P.to && !skip, node_local = false;
         int cl = 0, cr = 0;
         if (live) {
             // the leaf at position p
@@ -846,9 +901,9 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
         }
         s_done[t] = 0;
         __syncthreads();
-        // rounds: children indices (position - blo) of a local node lie in the block
-        const int il = node_local ? ((cl < 0 ? ~cl : cl) - blo) & (REFIT_THREADS - 1) : 0;
-        const int ir = node_local ? ((cr < 0 ? ~cr : cr) - blo) & (REFIT_THREADS - 1) : 0;
+        // rounds: the items of a local node's children lie in the block
+        const int il = node_local ? ((cl < 0 ? ~cl : cl) - first) & (REFIT_THREADS - 1) : 0;
+        const int ir = node_local ? ((cr < 0 ? ~cr : cr) - first) & (REFIT_THREADS - 1) : 0;
         bool pending = node_local;
 #pragma unroll 1
         for (int round = 1; round <= REFIT_THREADS; ++round) {
