@@ -268,8 +268,7 @@ int upload_table(ccc_engine* e, int which, const int32_t* ids, int64_t n, cudaSt
     return CCC_OK;
 }
 
-// The refit's climbs are chains of dependent L2 round trips, so it runs about one leaf per
-// thread (up to 64 blocks per SM) rather than a grid-stride loop over few threads.
+// A block for every chunk of the refit within blocks, up to 64 per SM.
 inline int refit_grid(const ccc_engine* e) {
     return (int)std::min<int64_t>(e->tri_cap / REFIT_THREADS + e->mesh_cap, (int64_t)num_sms() * 64);
 }
@@ -277,6 +276,11 @@ inline int refit_grid(const ccc_engine* e) {
 // blocks of `per` a mesh, about as many as are resident together
 inline int top_grid(const ccc_engine* e, int per) {
     return per * (int)std::max<int64_t>(1, std::min<int64_t>(e->mesh_cap, num_sms() / per));
+}
+// ... and all of those where a mesh may have too many top nodes: its climbs need the threads, however
+// few meshes there are (one of 400,000 triangles: 177 -> 61 us)
+inline int refit_top_grid(const ccc_engine* e) {
+    return e->tri_cap > 25 * (int64_t)TOP_CAP ? num_sms() / TOP_CLUSTER * TOP_CLUSTER : top_grid(e, TOP_CLUSTER);
 }
 
 // (hdr->front is 0 before it: a step clears the header, the build only that word)
@@ -286,7 +290,7 @@ template <class T> int refit(ccc_engine* e, const Tables& t, const int* flags, c
         e->at<TNode>(e->L.nodes), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop), e->at<int2>(e->L.front),
         (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_engine_refit_front", s, launch_chain(top_grid(e, TOP_CLUSTER), TOP_THREADS, sizeof(TopShared), s, k_engine_refit_top, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
+    CCC_LAUNCH("k_engine_refit_front", s, launch_chain(refit_top_grid(e), TOP_THREADS, sizeof(TopShared), s, k_engine_refit_top, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
         e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
         e->at<unsigned>(e->L.visits), e->at<int2>(e->L.front), (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();

@@ -109,3 +109,32 @@ def test_small_meshes_share_the_refits_blocks(cuda):
     table, which goes over the same triangles with full blocks; with shared ones about as long."""
     times = _step_times(cuda)
     assert times["k_engine_refit"] < 2 * times["k_weld_insert"]
+
+
+@pytest.mark.gpu
+def test_one_large_mesh_has_the_threads_for_its_climbs(cuda):
+    """A mesh with more nodes above the refit's blocks than its upper pass holds is finished by
+    climbs, and takes as long in an engine for one mesh as in one for many."""
+    from cccollisions_b200 import _native as N
+    from cccollisions_b200.engine import Engine
+    g = torch.Generator(device=cuda).manual_seed(2)
+    x0, x1 = (x[0] for x in _soup(g, 1, 400000, cuda, spread=60.0))
+    times = []
+    with torch.cuda.device(cuda):
+        for capacity in (1, 64):
+            eng = Engine(tri_capacity=len(x0), mesh_capacity=capacity, max_candidates_per_triangle=4,
+                         max_collisions_per_triangle=4)
+            sid = eng.add_mesh(len(x0))
+            eng.upload_soup(sid, x0, x1)
+            eng.set_active([sid])
+            eng.build([sid])
+            for _ in range(3):
+                eng.ccd()
+            torch.cuda.synchronize()
+            N.timing_begin()
+            for _ in range(9):
+                eng.ccd()
+            torch.cuda.synchronize()
+            times.append(N.timing_end()["k_engine_refit_front"][0])
+            eng.close()
+    assert times[0] < 1.5 * times[1], times
