@@ -290,7 +290,7 @@ template <class T> int refit(ccc_engine* e, const Tables& t, const int* flags, c
         e->at<TNode>(e->L.nodes), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop), e->at<int2>(e->L.front),
         (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_engine_refit_front", s, launch_chain(refit_top_grid(e), TOP_THREADS, sizeof(TopShared), s, k_engine_refit_top, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
+    CCC_LAUNCH("k_engine_refit_front", s, launch_chain(refit_top_grid(e), TOP_THREADS, sizeof(TopShared<TOP_CAP>), s, k_engine_refit_top, t.f, e->at<int>(e->L.nparent), e->at<int>(e->L.qcode), e->at<QNode>(e->L.qnodes), e->at<int2>(e->L.ntop),
         e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
         e->at<unsigned>(e->L.visits), e->at<int2>(e->L.front), (int)e->tri_cap, flags, e->hdr()));
     CCC_LAUNCH_CHECK();
@@ -507,7 +507,7 @@ template <class T> int build_trees(ccc_engine* e, int64_t ntri, int64_t nb, cuda
     CCC_LAUNCH("k_qtree_slots", s, launch_chain(item_grid(), ITEM_THREADS, 0, s, k_qtree_slots, t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<QNode>(e->L.qnodes),
         &e->hdr()->status));
     CCC_LAUNCH_CHECK();
-    CCC_LAUNCH("k_refit_plan", s, launch_chain(top_grid(e, 1), TOP_THREADS, sizeof(PlanShared), s, k_refit_plan, t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
+    CCC_LAUNCH("k_refit_plan", s, launch_chain(top_grid(e, 1), TOP_THREADS, PLAN_BYTES, s, k_refit_plan, t.f, e->at<TNode>(e->L.nodes), e->at<int>(e->L.qcode), e->at<int>(e->L.qleaf), e->at<int2>(e->L.nrange),
         e->at<int2>(e->L.ntop), e->at<int>(e->L.top_node), e->at<int>(e->L.top_index), e->at<int2>(e->L.top_child),
         &e->hdr()->status));
     CCC_LAUNCH_CHECK();
@@ -539,8 +539,8 @@ bool active_built(const ccc_engine* e) {
 // stream capture
 template <class T> bool prepare_kernels() {
     return cudaFuncSetAttribute(k_engine_refit_top, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(TopShared)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_refit_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PlanShared)) ==
+                                (int)sizeof(TopShared<TOP_CAP>)) == cudaSuccess &&
+           cudaFuncSetAttribute(k_refit_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLAN_BYTES) ==
                cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_REFERENCE, SRC_STAGED>() == cudaSuccess &&
            prepare_ccd_narrow<T, CCD_ROWS, CornerSink<T>, LIB_PORTABLE, SRC_STAGED>() == cudaSuccess &&

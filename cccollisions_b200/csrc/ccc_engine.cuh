@@ -985,22 +985,143 @@ template <class Fn> __device__ __forceinline__ int next_mesh(int m, int M, int s
     return M;
 }
 
+// ... and by a warp (in every warp of a team alike).
+template <class Fn> __device__ __forceinline__ int next_mesh_of_team(int m, int M, int step, Fn&& wanted) {
+    for (long long from = m; from < M; from += 32LL * step) {
+        const long long at = from + (long long)step * (threadIdx.x & 31);
+        const unsigned found = __ballot_sync(0xffffffffu, at < M && wanted((int)at));
+        if (found) return (int)(from + (long long)step * (__ffs(found) - 1));
+    }
+    return M;
+}
+
+// The threads that work on a mesh's top nodes together: a block, or one of its teams of TOP_TEAM
+// threads, each with its share of the block's shared memory.
+struct TopTeam {
+    int rank, size, barrier;
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(barrier), "r"(size) : "memory"); }
+    __device__ __forceinline__ bool any(bool x) const {      // (a barrier too)
+        int r;
+        asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.or.pred q, %2, %3, p;\nselp.s32 %0, 1, 0, q;\n}"
+                     : "=r"(r) : "r"((int)x), "r"(barrier), "r"(size) : "memory");
+        return r != 0;
+    }
+};
+static constexpr int TOP_TEAM = 128;
+static constexpr int TOP_TEAMS = TOP_THREADS / TOP_TEAM;
+static constexpr int TOP_TEAM_CAP = TOP_CAP / TOP_TEAMS;      // (960: meshes of some 27,000 triangles)
+static constexpr int TOP_NONE = 0xffff;
+static_assert(TOP_CAP < TOP_NONE, "top node indices are 16-bit");
+__device__ __forceinline__ TopTeam block_team() { return TopTeam{(int)threadIdx.x, TOP_THREADS, 0}; }
+__device__ __forceinline__ TopTeam own_team() {
+    return TopTeam{(int)threadIdx.x % TOP_TEAM, TOP_TEAM, 1 + (int)threadIdx.x / TOP_TEAM};
+}
+
 // The order of pass 2, laid down with the topology: the top nodes of a mesh by height above the
 // blocks (counting sort; a height is found in rounds, one more than the children's), each with
 // where its children's boxes are and its own slot code.  A child below comes from slots that
 // pass 1 writes: its own (a leaf, an even-depth node), or its two children's (an odd-depth
 // node, TOP_PAIR); a child above is ~ its place in the order.  ntop[sid] = (top nodes, levels),
 // level l's places from top_index[po + l].
+// A block a mesh, or, with more meshes than blocks, a team for each that fits (1,000 meshes of 600
+// triangles 77 -> 19 us).
 static constexpr int TOP_PAIR = 1 << 30;
-struct PlanShared {
-    int node[TOP_CAP];
-    int below[2][TOP_CAP];               // where the children's boxes are
-    unsigned short dep[2][TOP_CAP];      // the children that are top nodes (TOP_CAP: none)
-    unsigned short place[TOP_CAP];
-    unsigned char height[TOP_CAP];       // 0: not found yet
+template <int CAP> struct PlanShared {
+    int node[CAP];
+    int below[2][CAP];               // where the children's boxes are
+    unsigned short dep[2][CAP];      // the children that are top nodes, or TOP_NONE
+    unsigned short place[CAP];
+    unsigned char height[CAP];       // 0: not found yet
     int start[TOP_LEVELS + 1];
 };
-static_assert(TOP_CAP < 65536, "top node indices are 16-bit");
+template <int CAP>
+__device__ __forceinline__ void plan_mesh(const TopTeam& team, PlanShared<CAP>& S, const Forest& F, int m,
+                                          const TNode* __restrict__ nodes, const int* __restrict__ qcode,
+                                          const int* __restrict__ qleaf, const int2* __restrict__ nrange, int2* ntop,
+                                          int* top_node, int* top_index, int2* top_child, int* status) {
+    const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
+    const int sid = __ldg(F.sid + m);
+    const int nt = min(ntop[sid].x, CAP);
+    // where child c's box is: a slot code, ~ (index of a top node), or TOP_PAIR | the first of two
+    // slots; the last code of all for a malformed tree
+    auto where = [&](int c) {
+        if (c >= 0 && c < n - 1 && refit_crosses(__ldg(nrange + po + c))) {
+            const int f = top_index[po + c];
+            if (f >= 0 && f < nt) return ~f;
+        } else {
+            int code = c < 0 ? (~c < n ? __ldg(qleaf + po + ~c) : -1) : (c < n - 1 ? __ldg(qcode + po + c) : -1);
+            int pair = 0;
+            if (c >= 0 && code <= QCODE_ODD) {
+                code = QCODE_ODD - code;
+                pair = TOP_PAIR;
+            }
+            if (code >= 0 && (code >> 2) < n - 1 && !(pair && (code & 3) > 2)) return code | pair;
+        }
+        atomicOr(status, ST_MALFORMED_TREE);
+        return 0;
+    };
+    if (team.rank <= TOP_LEVELS) S.start[team.rank] = 0;
+    for (int f = team.rank; f < nt; f += team.size) {
+        const int i = top_node[po + f];
+        const int4 d = __ldg(&nodes[po + i].d);
+        const int a = where(d.x), b = where(d.y);
+        S.node[f] = i;
+        S.below[0][f] = a;
+        S.below[1][f] = b;
+        S.dep[0][f] = (unsigned short)(a < 0 ? ~a : TOP_NONE);
+        S.dep[1][f] = (unsigned short)(b < 0 ? ~b : TOP_NONE);
+        S.height[f] = 0;
+    }
+    team.sync();
+    int levels = 0;
+#pragma unroll 1
+    for (int round = 1; round <= TOP_LEVELS; ++round) {
+        bool left = false;
+        for (int f = team.rank; f < nt; f += team.size) {
+            if (S.height[f]) continue;
+            const int a = S.dep[0][f], b = S.dep[1][f];
+            const int ha = a != TOP_NONE ? S.height[a] : 0, hb = b != TOP_NONE ? S.height[b] : 0;
+            if ((a != TOP_NONE && (ha == 0 || ha >= round)) || (b != TOP_NONE && (hb == 0 || hb >= round))) {
+                left = true;
+                continue;
+            }
+            S.height[f] = (unsigned char)round;
+            atomicAdd(&S.start[round], 1);
+        }
+        levels = round;
+        if (!team.any(left)) break;
+        // (not reached by a tree: a cycle; its nodes join the last level)
+        if (round == TOP_LEVELS && left) {
+            atomicOr(status, ST_MALFORMED_TREE);
+            for (int f = team.rank; f < nt; f += team.size)
+                if (!S.height[f]) {
+                    S.height[f] = TOP_LEVELS;
+                    atomicAdd(&S.start[TOP_LEVELS], 1);
+                }
+        }
+    }
+    team.sync();
+    if (team.rank == 0)
+        for (int l = 1; l <= TOP_LEVELS; ++l) S.start[l] += S.start[l - 1];       // ends of the levels
+    team.sync();
+    if (team.rank <= levels) top_index[po + min(team.rank, n - 1)] = S.start[team.rank];
+    if (team.rank == 0) ntop[sid].y = levels;
+    team.sync();
+    for (int f = team.rank; f < nt; f += team.size)
+        S.place[f] = (unsigned short)atomicAdd(&S.start[S.height[f] - 1], 1);
+    team.sync();
+    for (int f = team.rank; f < nt; f += team.size) {
+        const int at = S.place[f], a = S.dep[0][f], b = S.dep[1][f];
+        top_child[po + at] = make_int2(a != TOP_NONE ? ~(int)S.place[a] : S.below[0][f],
+                                       b != TOP_NONE ? ~(int)S.place[b] : S.below[1][f]);
+        top_node[po + at] = __ldg(qcode + po + S.node[f]);
+    }
+    team.sync();
+}
+
+static constexpr size_t PLAN_BYTES = sizeof(PlanShared<TOP_CAP>) > TOP_TEAMS * sizeof(PlanShared<TOP_TEAM_CAP>)
+                                         ? sizeof(PlanShared<TOP_CAP>)
+                                         : TOP_TEAMS * sizeof(PlanShared<TOP_TEAM_CAP>);
 static __global__ void __launch_bounds__(TOP_THREADS)
 k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ qcode, const int* __restrict__ qleaf,
              const int2* __restrict__ nrange, int2* __restrict__ ntop, int* __restrict__ top_node,
@@ -1008,95 +1129,31 @@ k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ 
     chain_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ unsigned s_first[32];
-    PlanShared& S = *reinterpret_cast<PlanShared*>(smem);
-    const int M = forest_size(F);
+    const int M = forest_size(F), blocks = gridDim.x;
+    const int least = M > blocks ? TOP_TEAM_CAP : 0;    // a block takes the meshes with more top nodes
+    if (least) {
+        const int team = threadIdx.x / TOP_TEAM, step = blocks * TOP_TEAMS;
+        PlanShared<TOP_TEAM_CAP>& S = reinterpret_cast<PlanShared<TOP_TEAM_CAP>*>(smem)[team];
+        auto mine = [&](int m) {
+            const int nt = ntop[__ldg(F.sid + m)].x;
+            return nt > 0 && nt <= TOP_TEAM_CAP;
+        };
+        for (int m = next_mesh_of_team(team * blocks + blockIdx.x, M, step, mine); m < M;
+             m = next_mesh_of_team(m + step, M, step, mine))
+            plan_mesh(own_team(), S, F, m, nodes, qcode, qleaf, nrange, ntop, top_node, top_index, top_child, status);
+        __syncthreads();
+    }
+    PlanShared<TOP_CAP>& S = *reinterpret_cast<PlanShared<TOP_CAP>*>(smem);
     auto planned = [&](int m) {
         const int nt = ntop[__ldg(F.sid + m)].x;
-        return nt > 0 && nt <= TOP_CAP;
+        return nt > least && nt <= TOP_CAP;
     };
-    for (int m = blockIdx.x; m < M; m += gridDim.x) {
+    for (int m = blockIdx.x; m < M; m += blocks) {
         if (!planned(m)) {                              // (block-uniform)
-            m = next_mesh(m + gridDim.x, M, gridDim.x, s_first, planned);
+            m = next_mesh(m + blocks, M, blocks, s_first, planned);
             if (m >= M) break;
         }
-        const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
-        const int sid = __ldg(F.sid + m);
-        const int nt = ntop[sid].x;
-        // where child c's box is: a slot code, ~ (index of a top node), or TOP_PAIR | the first of two
-        // slots; the last code of all for a malformed tree
-        auto where = [&](int c) {
-            if (c >= 0 && c < n - 1 && refit_crosses(__ldg(nrange + po + c))) {
-                const int f = top_index[po + c];
-                if (f >= 0 && f < nt) return ~f;
-            } else {
-                int code = c < 0 ? (~c < n ? __ldg(qleaf + po + ~c) : -1) : (c < n - 1 ? __ldg(qcode + po + c) : -1);
-                int pair = 0;
-                if (c >= 0 && code <= QCODE_ODD) {
-                    code = QCODE_ODD - code;
-                    pair = TOP_PAIR;
-                }
-                if (code >= 0 && (code >> 2) < n - 1 && !(pair && (code & 3) > 2)) return code | pair;
-            }
-            atomicOr(status, ST_MALFORMED_TREE);
-            return 0;
-        };
-        if (threadIdx.x <= TOP_LEVELS) S.start[threadIdx.x] = 0;
-        for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
-            const int i = top_node[po + f];
-            const int4 d = __ldg(&nodes[po + i].d);
-            const int a = where(d.x), b = where(d.y);
-            S.node[f] = i;
-            S.below[0][f] = a;
-            S.below[1][f] = b;
-            S.dep[0][f] = (unsigned short)(a < 0 ? ~a : TOP_CAP);
-            S.dep[1][f] = (unsigned short)(b < 0 ? ~b : TOP_CAP);
-            S.height[f] = 0;
-        }
-        __syncthreads();
-        int levels = 0;
-#pragma unroll 1
-        for (int round = 1; round <= TOP_LEVELS; ++round) {
-            bool left = false;
-            for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
-                if (S.height[f]) continue;
-                const int a = S.dep[0][f], b = S.dep[1][f];
-                const int ha = a < TOP_CAP ? S.height[a] : 0, hb = b < TOP_CAP ? S.height[b] : 0;
-                if ((a < TOP_CAP && (ha == 0 || ha >= round)) || (b < TOP_CAP && (hb == 0 || hb >= round))) {
-                    left = true;
-                    continue;
-                }
-                S.height[f] = (unsigned char)round;
-                atomicAdd(&S.start[round], 1);
-            }
-            levels = round;
-            if (!__syncthreads_or(left)) break;
-            // (not reached by a tree: a cycle; its nodes join the last level)
-            if (round == TOP_LEVELS && left) {
-                atomicOr(status, ST_MALFORMED_TREE);
-                for (int f = threadIdx.x; f < nt; f += TOP_THREADS)
-                    if (!S.height[f]) {
-                        S.height[f] = TOP_LEVELS;
-                        atomicAdd(&S.start[TOP_LEVELS], 1);
-                    }
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int l = 1; l <= TOP_LEVELS; ++l) S.start[l] += S.start[l - 1];       // ends of the levels
-        __syncthreads();
-        if (threadIdx.x <= levels) top_index[po + min(threadIdx.x, n - 1)] = S.start[threadIdx.x];
-        if (threadIdx.x == 0) ntop[sid].y = levels;
-        __syncthreads();
-        for (int f = threadIdx.x; f < nt; f += TOP_THREADS)
-            S.place[f] = (unsigned short)atomicAdd(&S.start[S.height[f] - 1], 1);
-        __syncthreads();
-        for (int f = threadIdx.x; f < nt; f += TOP_THREADS) {
-            const int at = S.place[f], a = S.dep[0][f], b = S.dep[1][f];
-            top_child[po + at] = make_int2(a < TOP_CAP ? ~(int)S.place[a] : S.below[0][f],
-                                           b < TOP_CAP ? ~(int)S.place[b] : S.below[1][f]);
-            top_node[po + at] = __ldg(qcode + po + S.node[f]);
-        }
-        __syncthreads();
+        plan_mesh(block_team(), S, F, m, nodes, qcode, qleaf, nrange, ntop, top_node, top_index, top_child, status);
     }
 }
 
@@ -1108,10 +1165,133 @@ k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ 
 // L2 (20 levels above the blocks on 55,000 triangles): 5 small meshes 31 -> 8 us, 12 meshes 50
 // -> 16 us, 64 meshes 117 -> 88 us, ten served folds 40 -> 14 us; the plan is 27 us of a build of
 // the 12 meshes.  What is left is the gather's latency, some 400 cycles a level, and a launch.
-struct TopShared {
-    float lo[3][TOP_CAP], hi[3][TOP_CAP];
-    unsigned short dep[2][TOP_CAP];      // the children that are top nodes (TOP_CAP: none)
+// With more meshes than clusters, those that fit a team's share of the memory go to a team each,
+// since a cluster has some 14 us for a mesh, however small: 1,000 meshes of 600 triangles 387 -> 25
+// us, 200 of 2,000 88 -> 23, 60 of 6,000 25 -> 19.
+template <int CAP> struct TopShared {
+    float lo[3][CAP], hi[3][CAP];
+    unsigned short dep[2][CAP];      // the children that are top nodes, or TOP_NONE
 };
+
+// the boxes below node f, whose children are ch
+template <int CAP>
+__device__ __forceinline__ void top_gather(TopShared<CAP>& S, int f, int2 ch, int nt, const QNode* qn) {
+    float lo[3], hi[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        lo[x] = __int_as_float(0x7f800000);
+        hi[x] = __int_as_float(0xff800000);
+    }
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const int c = side ? ch.y : ch.x;
+        S.dep[side][f] = (unsigned short)(c < 0 ? min(~c, nt - 1) : TOP_NONE);
+        if (c < 0) continue;
+        const int code = c & ~TOP_PAIR;
+        float l[3], h[3];
+        read_qslot(qn, code, l, h);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            lo[x] = fminf(lo[x], l[x]);
+            hi[x] = fmaxf(hi[x], h[x]);
+        }
+        if (c & TOP_PAIR) {
+            read_qslot(qn, code + 1, l, h);
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                lo[x] = fminf(lo[x], l[x]);
+                hi[x] = fmaxf(hi[x], h[x]);
+            }
+        }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        S.lo[x][f] = lo[x];
+        S.hi[x][f] = hi[x];
+    }
+}
+
+// up the levels: the union of each node's boxes below and of its children above.  The first level
+// has no child above; the team takes the wide levels, a warp the rest, which has no use for the
+// team's barrier.
+template <int CAP>
+__device__ __forceinline__ void top_levels(const TopTeam& team, TopShared<CAP>& S, const int* end, int levels) {
+    auto unite = [&](int f) {
+        const int a = S.dep[0][f], b = S.dep[1][f];
+        const int ca = a != TOP_NONE ? a : f, cb = b != TOP_NONE ? b : f;
+        float lo[3], hi[3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            lo[x] = fminf(S.lo[x][f], fminf(S.lo[x][ca], S.lo[x][cb]));
+            hi[x] = fmaxf(S.hi[x][f], fmaxf(S.hi[x][ca], S.hi[x][cb]));
+        }
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            S.lo[x][f] = lo[x];
+            S.hi[x][f] = hi[x];
+        }
+    };
+    int l = 1;
+#pragma unroll 1
+    for (; l < levels && end[l + 1] - end[l] > 32; ++l) {
+        for (int f = end[l] + team.rank; f < end[l + 1]; f += team.size) unite(f);
+        team.sync();
+    }
+    if (team.rank < 32) {
+#pragma unroll 1
+        for (; l < levels; ++l) {
+            for (int f = end[l] + team.rank; f < end[l + 1]; f += 32) unite(f);
+            __syncwarp();
+        }
+    }
+}
+
+// node f's box into its slot, when it has one
+template <int CAP>
+__device__ __forceinline__ void top_store(const TopShared<CAP>& S, int f, int qc, int n, QNode* qn, WsHeader* hdr) {
+    if (qc < 0) return;
+    const float lo[3] = {S.lo[0][f], S.lo[1][f], S.lo[2][f]}, hi[3] = {S.hi[0][f], S.hi[1][f], S.hi[2][f]};
+    if ((qc >> 2) >= n - 1) atomicOr(&hdr->status, ST_MALFORMED_TREE);
+    else write_qslot(qn, qc, lo, hi);
+}
+
+// top nodes of mesh m, when it is to be refit in shared memory
+__device__ __forceinline__ int refit_top_nodes(const Forest& F, const int2* __restrict__ ntop, const int* __restrict__ mflags, int m) {
+    const int sid = __ldg(F.sid + m), nt = __ldg(&ntop[sid].x);
+    return nt <= TOP_CAP && !(mflags && (__ldg(mflags + sid) & MF_DONE)) ? nt : 0;
+}
+
+// the meshes with at most TOP_TEAM_CAP top nodes, a team each
+__device__ __forceinline__ void refit_top_by_teams(const Forest& F, int M, QNode* qnodes, const int2* __restrict__ ntop,
+                                                   const int* __restrict__ top_node, const int* __restrict__ top_index,
+                                                   const int2* __restrict__ top_child, const int* __restrict__ mflags,
+                                                   WsHeader* hdr, unsigned char* smem) {
+    __shared__ int s_ends[TOP_TEAMS][TOP_LEVELS + 1];
+    const int own = threadIdx.x / TOP_TEAM, step = gridDim.x * TOP_TEAMS;
+    const TopTeam team = own_team();
+    TopShared<TOP_TEAM_CAP>& S = reinterpret_cast<TopShared<TOP_TEAM_CAP>*>(smem)[own];
+    int* end = s_ends[own];
+    auto mine = [&](int m) {
+        const int nt = refit_top_nodes(F, ntop, mflags, m);
+        return nt > 0 && nt <= TOP_TEAM_CAP;
+    };
+    for (int m = next_mesh_of_team(own * gridDim.x + blockIdx.x, M, step, mine); m < M;
+         m = next_mesh_of_team(m + step, M, step, mine)) {
+        const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
+        const int2 plan = __ldg(ntop + __ldg(F.sid + m));
+        const int nt = plan.x, levels = min(plan.y, TOP_LEVELS);
+        QNode* qn = qnodes + po;
+        if (team.rank <= levels) end[team.rank] = min(__ldg(top_index + po + min(team.rank, n - 1)), nt);
+        for (int f = team.rank; f < nt; f += team.size) top_gather(S, f, __ldg(top_child + po + f), nt, qn);
+        team.sync();
+        top_levels(team, S, end, levels);
+        team.sync();
+        for (int f = team.rank; f < nt; f += team.size) top_store(S, f, __ldg(top_node + po + f), n, qn, hdr);
+        team.sync();
+    }
+}
+
+static_assert(TOP_TEAMS * sizeof(TopShared<TOP_TEAM_CAP>) <= sizeof(TopShared<TOP_CAP>), "the teams share a block's memory");
 static __global__ void __cluster_dims__(TOP_CLUSTER, 1, 1) __launch_bounds__(TOP_THREADS)
 k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restrict__ qcode, QNode* qnodes,
                    const int2* __restrict__ ntop, const int* __restrict__ top_node, const int* __restrict__ top_index,
@@ -1121,19 +1301,18 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_end[TOP_LEVELS + 1];
     __shared__ unsigned s_first[32];
+    const int M = forest_size(F), clusters = gridDim.x / TOP_CLUSTER;
+    const int least = M > clusters ? TOP_TEAM_CAP : 0;      // a cluster takes the meshes with more top nodes
+    if (least) refit_top_by_teams(F, M, qnodes, ntop, top_node, top_index, top_child, mflags, hdr, smem);
     const cg::cluster_group cluster = cg::this_cluster();
     // (a block's shared memory may be written by the others only once it has begun, which
-    // chain_begin, a wait for the kernel before, does not say)
+    // chain_begin, a wait for the kernel before, does not say, and once its teams are done)
     cluster.sync();
-    TopShared& S = *reinterpret_cast<TopShared*>(cluster.map_shared_rank(smem, 0));      // the first block's
+    TopShared<TOP_CAP>& S = *reinterpret_cast<TopShared<TOP_CAP>*>(cluster.map_shared_rank(smem, 0));   // the first block's
     const int rank = (int)cluster.block_rank();
     // (warp by warp over the blocks, so that a small mesh's nodes spread over them too)
     const int t0 = ((threadIdx.x >> 5) * TOP_CLUSTER + rank) * 32 + (threadIdx.x & 31);
-    const int M = forest_size(F), clusters = gridDim.x / TOP_CLUSTER;
-    auto refit = [&](int m) {
-        const int sid = __ldg(F.sid + m), nt = __ldg(&ntop[sid].x);
-        return nt > 0 && nt <= TOP_CAP && !(mflags && (__ldg(mflags + sid) & MF_DONE));
-    };
+    auto refit = [&](int m) { return refit_top_nodes(F, ntop, mflags, m) > least; };
     for (int m = blockIdx.x / TOP_CLUSTER; m < M; m += clusters) {
         if (!refit(m)) {                                // (cluster-uniform)
             m = next_mesh(m + clusters, M, clusters, s_first, refit);
@@ -1144,85 +1323,11 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
         const int nt = plan.x, levels = min(plan.y, TOP_LEVELS);
         QNode* qn = qnodes + po;
         if (rank == 0 && threadIdx.x <= levels) s_end[threadIdx.x] = min(__ldg(top_index + po + min(threadIdx.x, n - 1)), nt);
-        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) {
-            const int2 ch = __ldg(top_child + po + f);
-            float lo[3], hi[3];
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                lo[x] = __int_as_float(0x7f800000);
-                hi[x] = __int_as_float(0xff800000);
-            }
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                const int c = side ? ch.y : ch.x;
-                S.dep[side][f] = (unsigned short)(c < 0 ? min(~c, nt - 1) : TOP_CAP);
-                if (c < 0) continue;
-                const int code = c & ~TOP_PAIR;
-                float l[3], h[3];
-                read_qslot(qn, code, l, h);
-#pragma unroll
-                for (int x = 0; x < 3; ++x) {
-                    lo[x] = fminf(lo[x], l[x]);
-                    hi[x] = fmaxf(hi[x], h[x]);
-                }
-                if (c & TOP_PAIR) {
-                    read_qslot(qn, code + 1, l, h);
-#pragma unroll
-                    for (int x = 0; x < 3; ++x) {
-                        lo[x] = fminf(lo[x], l[x]);
-                        hi[x] = fmaxf(hi[x], h[x]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                S.lo[x][f] = lo[x];
-                S.hi[x][f] = hi[x];
-            }
-        }
+        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) top_gather(S, f, __ldg(top_child + po + f), nt, qn);
         cluster.sync();
-        if (rank == 0) {
-            TopShared& L = *reinterpret_cast<TopShared*>(smem);
-            // the union of node f's boxes below and of its children above
-            auto unite = [&](int f) {
-                const int a = L.dep[0][f], b = L.dep[1][f];
-                const int ca = a < TOP_CAP ? a : f, cb = b < TOP_CAP ? b : f;
-                float lo[3], hi[3];
-#pragma unroll
-                for (int x = 0; x < 3; ++x) {
-                    lo[x] = fminf(L.lo[x][f], fminf(L.lo[x][ca], L.lo[x][cb]));
-                    hi[x] = fmaxf(L.hi[x][f], fmaxf(L.hi[x][ca], L.hi[x][cb]));
-                }
-#pragma unroll
-                for (int x = 0; x < 3; ++x) {
-                    L.lo[x][f] = lo[x];
-                    L.hi[x][f] = hi[x];
-                }
-            };
-            // the first level has no child above; the block takes the wide levels, a warp the rest,
-            // which has no use for the block's barrier
-            int l = 1;
-#pragma unroll 1
-            for (; l < levels && s_end[l + 1] - s_end[l] > 32; ++l) {
-                for (int f = s_end[l] + threadIdx.x; f < s_end[l + 1]; f += TOP_THREADS) unite(f);
-                __syncthreads();
-            }
-            if (threadIdx.x < 32) {
-#pragma unroll 1
-                for (; l < levels; ++l) {
-                    for (int f = s_end[l] + threadIdx.x; f < s_end[l + 1]; f += 32) unite(f);
-                    __syncwarp();
-                }
-            }
-        }
+        if (rank == 0) top_levels(block_team(), *reinterpret_cast<TopShared<TOP_CAP>*>(smem), s_end, levels);
         cluster.sync();
-        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) {
-            const int qc = __ldg(top_node + po + f);
-            if (qc < 0) continue;
-            const float lo[3] = {S.lo[0][f], S.lo[1][f], S.lo[2][f]}, hi[3] = {S.hi[0][f], S.hi[1][f], S.hi[2][f]};
-            if ((qc >> 2) >= n - 1) atomicOr(&hdr->status, ST_MALFORMED_TREE);
-            else write_qslot(qn, qc, lo, hi);
-        }
+        for (int f = t0; f < nt; f += TOP_CLUSTER * TOP_THREADS) top_store(S, f, __ldg(top_node + po + f), n, qn, hdr);
         cluster.sync();      // (the next mesh overwrites the boxes; no block leaves before they are read)
     }
     // the climbs of the meshes with too many top nodes

@@ -34,6 +34,7 @@ def _ordered(rows, times):
     (12, 3000, {5: 300, 1999: 130, 2000: 5000, 2001: 127, 2999: 256}),
     (90, 700, {1: 258, 698: 2000}),
     (2, 45000, {44999: 2000}),                              # beyond a block's look at the next meshes
+    (12, 60, {7: 40000, 30: 600, 44: 28000}),               # too large for a team of threads, among many
 ])
 def test_rows_of_each_mesh(cuda, faces, count, larger):
     import cccollisions_b200 as C
@@ -41,7 +42,7 @@ def test_rows_of_each_mesh(cuda, faces, count, larger):
     small = _soup(g, count, faces, cuda)
     soups = [(small[0][i], small[1][i]) for i in range(count)]
     for i, f in larger.items():
-        x0, x1 = _soup(g, 1, f, cuda, spread=4.0)
+        x0, x1 = _soup(g, 1, f, cuda, spread=max(4.0, 0.5 * f ** (1 / 3)))
         soups[i] = (x0[0], x1[0])
     with torch.cuda.device(cuda):
         eng, sids = _engine(soups, max_candidates_per_triangle=32, max_collisions_per_triangle=64)
@@ -75,12 +76,12 @@ def test_rows_of_each_mesh(cuda, faces, count, larger):
     assert sum(expect.values()) == total and total > 0
 
 
-def _step_times(cuda):
-    """Kernel times of a step of 20,000 meshes of 12 triangles, none of which has a node above the
-    refit's blocks."""
+def _step_times(cuda, meshes=20000, faces=12):
+    """Kernel times of a step (20,000 meshes of 12 triangles: none has a node above the refit's
+    blocks)."""
     from cccollisions_b200 import _native as N
     g = torch.Generator(device=cuda).manual_seed(1)
-    x0, x1 = (x.cpu() for x in _soup(g, 20000, 12, cuda, spread=3.0))
+    x0, x1 = (x.cpu() for x in _soup(g, meshes, faces, cuda, spread=3.0))
     with torch.cuda.device(cuda):
         eng, _ = _engine(list(zip(x0, x1)), max_candidates_per_triangle=16, max_collisions_per_triangle=8)
         for _ in range(3):
@@ -96,10 +97,11 @@ def _step_times(cuda):
 
 
 @pytest.mark.gpu
-def test_small_meshes_cost_the_upper_pass_nothing(cuda):
+@pytest.mark.parametrize("meshes,faces", [(20000, 12), (1000, 600)])
+def test_small_meshes_cost_the_upper_pass_little(cuda, meshes, faces):
     """Going over them in turn took the upper pass 400 us, far longer than the pass that has all
     the work."""
-    times = _step_times(cuda)
+    times = _step_times(cuda, meshes, faces)
     assert times["k_engine_refit_front"] < times["k_engine_refit"]
 
 
