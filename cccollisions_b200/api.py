@@ -7,9 +7,11 @@ RuntimeError), allocates the outputs exactly as the reference does (-1 filled ro
 impulses), and calls the native library through its C ABI on the current CUDA stream.
 
 Capacity overflows print the reference's warnings (as ``warnings.warn``) and truncate like
-the reference; set ``cccollisions_b200.api.STRICT = True`` to raise instead.  Set
-``CHECK_STATUS = False`` to skip the status read-back (one small synchronising copy per
-call) when running inside CUDA graphs or tight loops.
+the reference; set ``cccollisions_b200.api.STRICT = True`` to raise instead.  A call returns
+when its outputs are complete: the queries read their status back (one small synchronising
+copy), the builds, which have none, wait for the stream.  Set ``CHECK_STATUS = False`` to skip
+both when running inside CUDA graphs or tight loops; outputs are then ordered by the calling
+stream only.
 """
 from __future__ import annotations
 
@@ -152,7 +154,7 @@ def bvh_motion(triangles, triangles_next):
 def _bvh(triangles, triangles_next):
     B, F = triangles.size(0), triangles.size(1)
     dev = triangles.device
-    # (the build writes every element, and nothing in it can fail on the device: no status)
+    # (the build writes every element)
     bboxes = torch.empty((B, 2 * F - 1, 6), dtype=triangles.dtype, device=dev)
     tree = torch.empty((B, 2 * F - 1, 4), dtype=torch.int64, device=dev)
     with _with_device(triangles):
@@ -160,6 +162,10 @@ def _bvh(triangles, triangles_next):
         rc = N.lib().ccc_bvh(_dtype_code(triangles), _ptr(triangles), _ptr(triangles_next), B, F, _ptr(bboxes),
                              _ptr(tree), _ptr(ws), ws.numel(), _stream(dev))
         N.check(rc, "bvh")
+        # Nothing in the build can fail on the device, so there is no status to read; the wait that
+        # came with it is part of the call: its tensors may be used on any stream afterwards.
+        if CHECK_STATUS:
+            torch.cuda.current_stream(dev).synchronize()
     return [bboxes, tree]
 
 
