@@ -94,7 +94,8 @@ def _status_words():
     try:
         return _thread.words
     except AttributeError:
-        _thread.words = torch.empty(2, dtype=torch.int32, pin_memory=True)
+        # (the device named: a default device that the caller has set is not one for page-locked memory)
+        _thread.words = torch.empty(2, dtype=torch.int32, device="cpu", pin_memory=True)
         return _thread.words
 
 
