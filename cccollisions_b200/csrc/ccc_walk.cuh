@@ -159,16 +159,20 @@ __device__ __forceinline__ void walk_forest(const Policy& pol, const QNode* __re
             S.stack[__popc(am & lt)] = (unsigned)lane << shift;       // the root
         }
         sp = __popc(am);
-        // (a query visits each node of its tree at most once)
-        long long rounds = 64 + (long long)sp * __reduce_max_sync(FULL, act ? (unsigned)Q.n : 0u);
+        // A query visits each node of its tree at most once, and a round that takes all the pending
+        // visits leaves only deeper ones, so that there are no more of those rounds than nodes: counted
+        // as 32 visits each, they bound a walk that goes in circles to some 2 n rounds, however few of
+        // the group's queries do.
+        long long left = 64 + (sp + 32LL) * __reduce_max_sync(FULL, act ? (unsigned)Q.n : 0u);
         __syncwarp();
         while (sp > 0) {
-            if (--rounds < 0 || sp > WALK_STACK - 3) {
-                if (lane == 0) atomicOr(&hdr->status, rounds < 0 ? ST_MALFORMED_TREE : ST_STACK_OVERFLOW);
+            if (left < 0 || sp > WALK_STACK - 3) {
+                if (lane == 0) atomicOr(&hdr->status, left < 0 ? ST_MALFORMED_TREE : ST_STACK_OVERFLOW);
                 sp = 0;
                 break;
             }
             const int k = min(min(sp, 32), max(1, (WALK_STACK - WALK_RESERVE - sp) / 3));
+            left -= k == sp ? 32 : k;
             const bool has = lane < k;
             const unsigned e = has ? S.stack[sp - k + lane] : 0u;
             sp -= k;
