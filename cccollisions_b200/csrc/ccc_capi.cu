@@ -458,9 +458,9 @@ int ccc_get_math_library(void) { return g_math_lib; }
 
 int ccc_debug_stage(int op, int lib, const double* in, int in_stride, double* out, int out_stride, int64_t n,
                     void* stream) {
-    if (op < 0 || op > 5 || (lib != LIB_REFERENCE && lib != LIB_PORTABLE) || n < 0 || n >= ((int64_t)1 << 31))
+    if (op < 0 || op > 6 || (lib != LIB_REFERENCE && lib != LIB_PORTABLE) || n < 0 || n >= ((int64_t)1 << 31))
         return CCC_ERR_INVALID_ARG;
-    const int need_in[6] = {24, 4, 26, 30, 4, 1}, need_out[6] = {4, 3, 1, 6, 3, 3};
+    const int need_in[7] = {24, 4, 26, 30, 4, 4, 25}, need_out[7] = {4, 3, 1, 6, 3, 4, 8};
     if (in_stride < need_in[op] || out_stride < need_out[op]) return CCC_ERR_INVALID_ARG;
     if (n == 0) return CCC_OK;
     if (!in || !out) return CCC_ERR_INVALID_ARG;
@@ -471,7 +471,7 @@ int ccc_debug_stage(int op, int lib, const double* in, int in_stride, double* ou
 }
 
 int ccc_debug_math(int op, const double* in, double* out, int64_t n, void* stream) {
-    if (op < 0 || op > 11 || n < 0 || (n > 0 && (!in || !out)) || n >= ((int64_t)1 << 31)) return CCC_ERR_INVALID_ARG;
+    if (op < 0 || op > 12 || n < 0 || (n > 0 && (!in || !out)) || n >= ((int64_t)1 << 31)) return CCC_ERR_INVALID_ARG;
     if (n == 0) return CCC_OK;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaSuccess;

@@ -56,7 +56,9 @@ CCC_CONTACT_TYPES(LoopSink)
 // them bit for bit with the CPU oracle and against CUDA's own elementary functions.
 // op 0 cbrt, 1 acos, 2 cos, 3 sin, 4 certified product (in: x0, x1, k, y; out: r0, r1),
 // 5 solve_cubic (in: a, b, c, d; out: three roots), 6 CUDA cbrt, 7 CUDA acos, 8 CUDA cos,
-// 9 CUDA sin.  in has 4 doubles per element, out 3.
+// 9 CUDA sin, 10 the solver prefix of a, b, c, d without its short cuts (out: f, g, h), 11 the
+// solver's divisions by 3 and by 27, 12 CUDA sincos (out: sine, cosine).  in has 4 doubles per
+// element, out 3.
 static __global__ void k_debug_math(int op, const double* __restrict__ in, double* __restrict__ out, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -79,18 +81,25 @@ static __global__ void k_debug_math(int op, const double* __restrict__ in, doubl
         case 7: o[0] = acos(a[0]); break;
         case 8: o[0] = cos(a[0]); break;
         case 9: o[0] = sin(a[0]); break;
-        case 10: case 11: {
-            double A = a[0], Bc = a[1], Cc = a[2], Dc = a[3];
-            double f = ((3.0 * Cc / A) - ((Bc * Bc) / (A * A))) / 3.0;
-            double b3 = 2 * ccc_cube_hi(Bc);
-            ccc_dd a2dd = ccc_sq_dd(A);
-            double a3 = ccc_certmul(a2dd.hi, a2dd.lo, 2, A).hi;
-            double g = (b3 / a3 - (Bc * Cc * 9) / a2dd.hi + 27.0 * Dc / A) / 27.0;
-            double h = addrn(mulrn(mulrn(g, g), 0.25), ccc_cube_hi(f) / 27.0);
-            if (op == 10) { o[0] = f; o[1] = g; o[2] = h; }
-            else { o[0] = b3; o[1] = a2dd.hi; o[2] = a3; }
+        case 10: {
+            // the solver prefix without its short cuts (certified products, divisions)
+            const double A = a[0], B = a[1], C = a[2], D = a[3];
+            auto cube = [](double x) {
+                const ccc_dd sq = ccc_certmul(x, 0.0, 1, x);
+                return ccc_certmul(sq.hi, sq.lo, 2, x).hi;
+            };
+            const double f = ((3.0 * C / A) - ((B * B) / (A * A))) / 3.0;
+            const double g = (2 * cube(B) / cube(A) - (B * C * 9) / ccc_certmul(A, 0.0, 1, A).hi + 27.0 * D / A) / 27.0;
+            o[0] = f;
+            o[1] = g;
+            o[2] = addrn(mulrn(mulrn(g, g), 0.25), cube(f) / 27.0);
             break;
         }
+        case 11:
+            o[0] = div_const<3>(a[0]);
+            o[1] = div_const<27>(a[0]);
+            break;
+        case 12: sincos(a[0], &o[0], &o[1]); break;
         default: break;
     }
 }
@@ -99,8 +108,40 @@ static __global__ void k_debug_math(int op, const double* __restrict__ in, doubl
 // doubles per element), for tests against the reference's own kernels and the oracle.
 // op 0: cubic coefficients -> 4 doubles; op 1: cubic solve (in: 4 coefficients) -> 3
 // roots; op 2: root filter (in: tet, type, root) -> 1.0 / 0.0; op 3: contact kinematics
-// (in: tet, type, root, 4 masses) -> normal (3), normal velocity, mass pair (2).
+// (in: tet, type, root, 4 masses) -> normal (3), normal velocity, mass pair (2); op 4: solver
+// prefix (in: 4 coefficients) -> class, g, h; op 5: early end of a cubic (in: 4 coefficients) ->
+// cubic_misses and the solver's roots in [0, 1], in double and in single precision; op 6: early
+// ends of a sub-test (in: tet, type) -> cubic_misses, roots_fail, the solver's roots in [0, 1]
+// and those of them that pass the filter, in double and in single precision.
 // lib selects the elementary functions (MathLib).
+template <class T> __device__ __forceinline__ int debug_roots(int lib, const T cf[4], T r[3]) {
+    if (lib == LIB_REFERENCE) solve_cubic<T, LIB_REFERENCE>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3], r);
+    else solve_cubic<T, LIB_PORTABLE>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3], r);
+    int n = 0;
+    for (int s = 0; s < 3; ++s) n += r[s] >= 0 && r[s] <= 1;
+    return n;
+}
+template <class T> __device__ __noinline__ void debug_cubic_end(int lib, const double* a, double* o) {
+    const T cf[4] = {(T)a[0], (T)a[1], (T)a[2], (T)a[3]};
+    T r[3];
+    o[0] = cubic_misses<T>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]);
+    o[1] = debug_roots(lib, cf, r);
+}
+template <class T> __device__ __noinline__ void debug_subtest_end(int lib, const MTet<double>& t, int k, double* o) {
+    MTet<T> m;
+    for (int p = 0; p < 4; ++p) {
+        m.v[p] = mk<T>((T)t.v[p].x, (T)t.v[p].y, (T)t.v[p].z);
+        m.dv[p] = mk<T>((T)t.dv[p].x, (T)t.dv[p].y, (T)t.dv[p].z);
+    }
+    T cf[4], r[3];
+    cubic_coeffs(m, cf);
+    o[0] = cubic_misses<T>((double)cf[0], (double)cf[1], (double)cf[2], (double)cf[3]);
+    o[1] = roots_fail(m, k, cf);
+    o[2] = debug_roots(lib, cf, r);
+    int pass = 0;
+    for (int s = 0; s < 3; ++s) pass += r[s] >= 0 && r[s] <= 1 && ccd_filter(m, k, r[s]);
+    o[3] = pass;
+}
 static __global__ void k_debug_stage(int op, int lib, const double* __restrict__ in, int in_stride,
                               double* __restrict__ out, int out_stride, int n) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -108,7 +149,7 @@ static __global__ void k_debug_stage(int op, int lib, const double* __restrict__
     const double* a = in + (long long)i * in_stride;
     double* o = out + (long long)i * out_stride;
     MTet<double> t;
-    if (op != 1) {
+    if (op != 1 && op != 4 && op != 5) {
         for (int p = 0; p < 4; ++p) {
             t.v[p] = mk<double>(a[3 * p], a[3 * p + 1], a[3 * p + 2]);
             t.dv[p] = mk<double>(a[12 + 3 * p], a[12 + 3 * p + 1], a[12 + 3 * p + 2]);
@@ -122,24 +163,18 @@ static __global__ void k_debug_stage(int op, int lib, const double* __restrict__
     } else if (op == 2) {
         o[0] = ccd_filter(t, (int)a[24], a[25]) ? 1.0 : 0.0;
     } else if (op == 4) {
-        // (f, g, h) of the solver prefix for coefficients (c3, c2, c1, c0)
-        double A = a[0], B = a[1], Cc = a[2], D = a[3];
-        double f = ((3.0 * Cc / A) - ((B * B) / (A * A))) / 3.0;
-        double b3 = 2 * ccc_cube_hi(B);
-        ccc_dd a2dd = ccc_sq_dd(A);
-        double a3 = ccc_certmul(a2dd.hi, a2dd.lo, 2, A).hi;
-        double g = (b3 / a3 - (B * Cc * 9) / a2dd.hi + 27.0 * D / A) / 27.0;
-        double g2 = lib == LIB_REFERENCE ? pow(g, 2.0) : mulrn(g, g);
-        o[0] = f;
+        double g, h;
+        const int cls = lib == LIB_REFERENCE ? cubic_prefix<LIB_REFERENCE>(a[0], a[1], a[2], a[3], g, h)
+                                             : cubic_prefix<LIB_PORTABLE>(a[0], a[1], a[2], a[3], g, h);
+        o[0] = cls;
         o[1] = g;
-        o[2] = addrn(mulrn(g2, 0.25), ccc_cube_hi(f) / 27.0);
+        o[2] = h;
     } else if (op == 5) {
-        // squares of a[0]: pow(x, 2), pow(x, 2.0), x * x
-        double x = a[0];
-        volatile int two = 2;
-        o[0] = pow(x, two);
-        o[1] = pow(x, (double)two);
-        o[2] = x * x;
+        debug_cubic_end<double>(lib, a, o);
+        debug_cubic_end<float>(lib, a, o + 2);
+    } else if (op == 6) {
+        debug_subtest_end<double>(lib, t, (int)a[24], o);
+        debug_subtest_end<float>(lib, t, (int)a[24], o + 4);
     } else if (op == 3) {
         double q[4] = {a[26], a[27], a[28], a[29]};
         Contact<double> ct = lib == LIB_REFERENCE ? contact<double, LIB_REFERENCE>(t, (int)a[24], a[25], q)

@@ -83,7 +83,12 @@ int ccc_get_math_library(void);
  * coefficients of (v0..v3, dv0..dv3) -> (c3, c2, c1, c0); op 1: cubic solve of
  * (c3, c2, c1, c0) -> three roots (-1 = none); op 2: root filter of (tet, type, root) ->
  * 1 / 0; op 3: contact kinematics of (tet, type, root, four masses) -> (normal, normal
- * velocity, mass pair).  lib: CCC_LIB_REFERENCE or CCC_LIB_PORTABLE. */
+ * velocity, mass pair); op 4: solver prefix of (c3, c2, c1, c0) -> (class, g, h); op 5: early end
+ * of the cubic (c3, c2, c1, c0) -> (1 when the narrow phase takes it to have no root in [0, 1],
+ * the solver's roots there), in double and again in single precision; op 6: early ends of the
+ * sub-test (tet, type) -> (as in op 5, 1 when none of its roots is taken to pass the filter, the
+ * solver's roots in [0, 1], those that pass), in double and again in single precision.
+ * lib: CCC_LIB_REFERENCE or CCC_LIB_PORTABLE. */
 int ccc_debug_stage(int op, int lib, const double* in, int in_stride, double* out, int out_stride, int64_t n,
                     void* stream);
 
@@ -91,8 +96,9 @@ int ccc_debug_stage(int op, int lib, const double* in, int in_stride, double* ou
  * arithmetic element-wise on the device so tests can compare it with the CPU oracle.
  * op: 0 cbrt, 1 acos, 2 cos, 3 sin (the library's own), 4 certified product
  * (in x0, x1, k, y -> out r0, r1), 5 cubic solve (in a, b, c, d -> out three roots,
- * -1 = none), 6..9 CUDA's cbrt, acos, cos, sin.  in: n x 4 doubles, out: n x 3 doubles
- * (device pointers). */
+ * -1 = none), 6..9 CUDA's cbrt, acos, cos, sin, 10 the solver prefix of a, b, c, d without its
+ * short cuts (out f, g, h), 11 the solver's x / 3 and x / 27, 12 CUDA's sincos.  in: n x 4
+ * doubles, out: n x 3 doubles (device pointers). */
 int ccc_debug_math(int op, const double* in, double* out, int64_t n, void* stream);
 
 /* Bytes of device scratch an operation needs for B meshes of F triangles with the given
