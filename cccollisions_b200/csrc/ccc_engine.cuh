@@ -795,12 +795,12 @@ __device__ __forceinline__ bool refit_chunk(const Forest& F, int M, int g, Refit
 
 // Where the meshes are that small that most chunks would hold a few triangles: the pieces of the
 // window of work items [g W, (g + 1) W), half as wide as a block.  The meshes that begin in it
-// take its one or two pieces: all but the last of them end in it, and go together with the last
-// one's first chunk when they fit.  A chunk further on in a mesh is its window's, but a last one
-// shorter than W, which the mesh's next or another may share a window with, is the window before's,
+// take its one or two pieces (`second`): all but the last of them end in it, and go together with
+// the last one's first chunk when they fit.  A chunk further on in a mesh is its window's, but a
+// last one shorter than W, which another mesh may share a window with, is the window before's,
 // where the mesh has nothing else.
 static constexpr int REFIT_WINDOW = REFIT_THREADS / 2;
-__device__ __forceinline__ int refit_window(const Forest& F, int M, int total, int g, RefitPiece piece[2]) {
+__device__ __forceinline__ bool refit_window(const Forest& F, int M, int total, int g, bool second, RefitPiece& piece) {
     const int begin = g * REFIT_WINDOW, stop = min(begin + REFIT_WINDOW, total);
     int m = find_mesh(F.voff, M, begin, 0);
     const int vo = __ldg(F.voff + m);
@@ -808,22 +808,19 @@ __device__ __forceinline__ int refit_window(const Forest& F, int M, int total, i
         const int end = __ldg(F.voff + m + 1), j = g - vo / REFIT_WINDOW;      // (1 or more)
         const int from = vo + (j + 1) / 2 * REFIT_THREADS;
         if (from < end && (j & 1) == (end - from < REFIT_WINDOW)) {
-            piece[0] = RefitPiece{from, min(from + REFIT_THREADS, end), m, false};
-            return 1;
+            piece = RefitPiece{from, min(from + REFIT_THREADS, end), m, false};
+            return !second;
         }
-        if (end >= stop) return 0;
+        if (end >= stop) return false;
         ++m;
     }
     const int last = find_mesh(F.voff, M, stop - 1, 0);
     const int from = __ldg(F.voff + m), at = __ldg(F.voff + last);
     const int to = min(at + REFIT_THREADS, __ldg(F.voff + last + 1));
-    if (to - from <= REFIT_THREADS) {
-        piece[0] = RefitPiece{from, to, m, m < last};
-        return 1;
-    }
-    piece[0] = RefitPiece{at, to, last, false};
-    piece[1] = RefitPiece{from, at, m, true};
-    return 2;
+    const bool together = to - from <= REFIT_THREADS;
+    if (second) piece = RefitPiece{from, at, m, true};
+    else piece = together ? RefitPiece{from, to, m, m < last} : RefitPiece{at, to, last, false};
+    return !(second && together);
 }
 
 // pass 1: REFIT_THREADS leaf positions of a mesh, from a multiple of REFIT_THREADS, or all of several
@@ -846,20 +843,14 @@ k_engine_refit_local(Forest F, const T* __restrict__ x0, const T* __restrict__ x
     __shared__ unsigned short s_done[REFIT_THREADS];    // round a local node was done in (0: not yet)
     const int M = forest_size(F);
     const int total = M > 0 ? __ldg(F.voff + M) : 0;
-    // (windows where the average mesh is smaller than a block: 20,000 meshes of 12 triangles 176 -> 48
-    // us, 5,000 of 200 triangles 130 -> 135 us)
-    const bool windows = total / REFIT_THREADS < M;
-    const int pieces = windows ? (total + REFIT_WINDOW - 1) / REFIT_WINDOW : total / REFIT_THREADS + M;
+    // (windows where the average mesh is smaller than one: 20,000 meshes of 12 triangles 176 -> 51
+    // us; 5,000 of 200 triangles would take 157 us so, 127 in chunks of their own)
+    const bool windows = total / REFIT_WINDOW < M;
+    const int pieces = windows ? 2 * ((total + REFIT_WINDOW - 1) / REFIT_WINDOW) : total / REFIT_THREADS + M;
     const int t = threadIdx.x;
-    RefitPiece piece[2];
-    int left = 0;
-    for (int g = blockIdx.x; g < pieces || left > 0;) {
-        if (left == 0) {
-            left = windows ? refit_window(F, M, total, g, piece) : (int)refit_chunk(F, M, g, piece[0]);
-            g += gridDim.x;
-            if (left == 0) continue;
-        }
-        const RefitPiece P = piece[--left];
+    for (int g = blockIdx.x; g < pieces; g += gridDim.x) {
+        RefitPiece P;
+        if (!(windows ? refit_window(F, M, total, g >> 1, g & 1, P) : refit_chunk(F, M, g, P))) continue;
         const int v = P.from + t;
         const int m = P.several && v < P.to ? find_mesh(F.voff, M, v, 0) : P.first;
         const int vo = __ldg(F.voff + m), po = __ldg(F.poff + m), n = __ldg(F.voff + m + 1) - vo;
@@ -1165,9 +1156,10 @@ k_refit_plan(Forest F, const TNode* __restrict__ nodes, const int* __restrict__ 
 // L2 (20 levels above the blocks on 55,000 triangles): 5 small meshes 31 -> 8 us, 12 meshes 50
 // -> 16 us, 64 meshes 117 -> 88 us, ten served folds 40 -> 14 us; the plan is 27 us of a build of
 // the 12 meshes.  What is left is the gather's latency, some 400 cycles a level, and a launch.
-// With more meshes than clusters, those that fit a team's share of the memory go to a team each,
+// With more than two meshes a cluster, those that fit a team's share of the memory go to a team each,
 // since a cluster has some 14 us for a mesh, however small: 1,000 meshes of 600 triangles 387 -> 25
-// us, 200 of 2,000 88 -> 23, 60 of 6,000 25 -> 19.
+// us, 200 of 2,000 88 -> 23.  (Two a cluster are as fast as the teams, which have the larger ones to
+// themselves: the 64 meshes, half of which fit, 45 -> 72 us.)
 template <int CAP> struct TopShared {
     float lo[3][CAP], hi[3][CAP];
     unsigned short dep[2][CAP];      // the children that are top nodes, or TOP_NONE
@@ -1302,7 +1294,7 @@ k_engine_refit_top(Forest F, const int* __restrict__ nparent, const int* __restr
     __shared__ int s_end[TOP_LEVELS + 1];
     __shared__ unsigned s_first[32];
     const int M = forest_size(F), clusters = gridDim.x / TOP_CLUSTER;
-    const int least = M > clusters ? TOP_TEAM_CAP : 0;      // a cluster takes the meshes with more top nodes
+    const int least = M > 2 * clusters ? TOP_TEAM_CAP : 0;      // a cluster takes the meshes with more top nodes
     if (least) refit_top_by_teams(F, M, qnodes, ntop, top_node, top_index, top_child, mflags, hdr, smem);
     const cg::cluster_group cluster = cg::this_cluster();
     // (a block's shared memory may be written by the others only once it has begun, which
