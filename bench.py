@@ -66,9 +66,10 @@ FP64_PEAK_NOMINAL_GFLOPS = 37000.0   # B200 FP64 datasheet figure (not measured 
 # sub-test, most of which end after the coefficients here
 FLOPS_PER_SUBTEST = 252
 # DRAM bytes (read + write) of one k_ccd_narrow launch per sub-test solved, from ncu's
-# dram__bytes_read.sum + dram__bytes_write.sum on the 32-mesh batched step; the 64-mesh
-# launch is too large for a full capture, so its traffic is this figure times its own count.
-NARROW_DRAM_BYTES_PER_SOLVED = (239520768 + 57656064) / 11536974
+# dram__bytes_read.sum + dram__bytes_write.sum on the 32-mesh batched step
+# (profiles/k_ccd_narrow_dram_batched32.md); the traffic reported for the 64-mesh launch is an
+# estimate, this figure times its own count.
+NARROW_DRAM_BYTES_PER_SOLVED = (160106752 + 16880384) / 11536974
 # the kernels of the narrow phase: staging (masks, solver choice), then the solves
 NARROW_PHASE = ("k_ccd_stage_mask", "k_ccd_stage_pending", "k_ccd_narrow")
 
@@ -405,8 +406,9 @@ def run_ours(args, rank, world, dev):
     dname, (dms, dcount) = max(kern.items(), key=lambda kv: kv[1][0])
     per_launch = dms / dcount
     # k_ccd_narrow reads a 16-byte record per pair with work and gathers both triangles at
-    # both ends of the step (2 x 2 x 72 bytes); it writes 32 bytes per row
-    narrow_bytes = cnt["live_pairs"] * (16 + 2 * 2 * 72) + int(sum(nrow)) * 32
+    # both ends of the step (2 x 2 x 72 bytes); it writes a 16-byte record per passing root, of
+    # which there are at most as many as rows (k_ccd_expand writes those)
+    narrow_bytes = cnt["live_pairs"] * (16 + 2 * 2 * 72) + int(sum(nrow)) * 16
     achieved = narrow_bytes / (per_launch / 1e3) / 1e9 if dname == "k_ccd_narrow" else None
     # the refit is two passes (block-local, then the levels above the blocks)
     r1 = kern.get("k_engine_refit", (float("nan"), 1))
@@ -433,7 +435,7 @@ def run_ours(args, rank, world, dev):
             "roofline": {"kernel": dname, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,
                          "traffic": (NARROW_DRAM_BYTES_PER_SOLVED * cnt["solved"]) if dname == "k_ccd_narrow"
-                         else None,
+                         else None,   # (an estimate from a smaller batch)
                          "alg_bytes_per_launch": narrow_bytes, "launch_ms": per_launch},
             "clocks": {"sm_mhz": clocks["sm_mhz"], "sm_max_mhz": clocks["sm_max_mhz"], "reasons": clocks["reasons"],
                        "samples": clocks["samples"]},

@@ -754,11 +754,11 @@ __device__ __forceinline__ float hmax4(float4 v) { return fmaxf(fmaxf(v.x, v.y),
 // Refit: every leaf's swept box (fp32, rounded outward) into its QNode slot, then bottom-up the
 // box of every even-depth node into its own, in two passes:
 //  * pass 1 (k_engine_refit_local): a block takes REFIT_THREADS consecutive leaf positions of a
-//    mesh and refits every node whose leaf range lies inside them, in shared memory, round by
-//    round;
+//    mesh, or several small meshes, and refits every node whose leaf range lies inside them, in
+//    shared memory, round by round;
 //  * pass 2 (k_engine_refit_top): the nodes above the blocks ("top" nodes, some nine a block), a
-//    cluster of TOP_CLUSTER blocks a mesh, again in shared memory, level by level in an order that
-//    the build lays down (k_refit_plan).
+//    cluster of TOP_CLUSTER blocks a mesh (a team of threads for each small one of many), again in
+//    shared memory, level by level in an order that the build lays down (k_refit_plan).
 // A mesh with more top nodes than pass 2 holds (TOP_CAP) is finished by climbs instead: in pass 1
 // an item whose parent is a top node hands that arrival over through the frontier list, and at
 // each node the second arrival (the one that finds the global counter odd, and so the node's
@@ -1793,13 +1793,17 @@ template <class T> struct LoopSink {
     VertTable vt;
     long long* acc;        // 8 words per vertex slot: dx xyz, dv xyz, count, unused
     int* contacts;         // per slot id
-    __device__ __forceinline__ void add(const MTet<T>& tet, long long gi, long long gj, int k, T root,
-                                        const Contact<T>& ct, const Forest& F, int M, int* status) const {
-        int m = forest_slot_mesh(F, M, gi);
-        // (one atomic for the lanes of a mesh, whose contacts all go to one word: k_ccd_contacts
-        // 118 -> 39 us an iteration of ten served folds)
+    // counts a contact for its mesh, which it returns (one atomic for the lanes of a mesh, whose
+    // contacts all go to one word: k_ccd_contacts 118 -> 39 us an iteration of ten served folds)
+    __device__ __forceinline__ int count(const Forest& F, int M, long long gi) const {
+        const int m = forest_slot_mesh(F, M, gi);
         const unsigned peers = __match_any_sync(__activemask(), m);
         if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(contacts + __ldg(F.sid + m), __popc(peers));
+        return m;
+    }
+    __device__ __forceinline__ void add(const MTet<T>& tet, long long gi, long long gj, int k, T root,
+                                        const Contact<T>& ct, const Forest& F, int M, int* status) const {
+        const int m = count(F, M, gi);
         loop_impulse(tet, gi, gj, k, root, ct, m, faces, vt, acc, status);
     }
     // The contacts of a warp's lanes (of those with `valid`), all lanes taking part: the seven
@@ -1817,11 +1821,7 @@ template <class T> struct LoopSink {
         ImpulseScale<T> sc;
         int vbase = 0, nv = 0;
         if (valid) {
-            const int m = forest_slot_mesh(F, M, gi);
-            // (one atomic for the lanes of a mesh, whose contacts all go to one word: k_ccd_contacts
-            // 118 -> 39 us an iteration of ten served folds)
-            const unsigned peers = __match_any_sync(__activemask(), m);
-            if (lane == __ffs(peers) - 1) atomicAdd(contacts + __ldg(F.sid + m), __popc(peers));
+            const int m = count(F, M, gi);
             sc = impulse_scale(ct, root);
             vbase = __ldg(vt.vpoff + m);
             nv = __ldg(vt.vvoff + m + 1) - __ldg(vt.vvoff + m);

@@ -34,7 +34,7 @@ __device__ __forceinline__ void chain_begin() { cudaGridDependencySynchronize();
 enum StatusBits {
     ST_CAND_OVERFLOW = 1,     // more candidate pairs than max_candidates_per_triangle * F
     ST_OUT_OVERFLOW = 2,      // more result rows than the output tensor holds
-    ST_STACK_OVERFLOW = 4,    // traversal deeper than the 64-entry stack
+    ST_STACK_OVERFLOW = 4,    // traversal deeper than its stack (one query a thread: 64 entries; walk: WALK_STACK)
     ST_MALFORMED_TREE = 8,    // child / parent index out of range or a cycle in the tree
 };
 
